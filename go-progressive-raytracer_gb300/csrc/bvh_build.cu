@@ -193,11 +193,10 @@ __global__ void k_collapse(TreeView T, const uint2* qin, const uint32_t* qin_n, 
       slot[pick] = T.left[c];
       slot[ns++] = T.right[c];
     }
-    float4* N = nodes + (size_t)item.y * 8;
+    NodeChild* N = reinterpret_cast<NodeChild*>(nodes + (size_t)item.y * 8);
     for (int i = 0; i < 4; i++) {
       if (i >= ns) {
-        N[2 * i] = make_float4(1e30f, 1e30f, 1e30f, __int_as_float(kEmptyChild));
-        N[2 * i + 1] = make_float4(-1e30f, -1e30f, -1e30f, __int_as_float(0));
+        N[i] = NodeChild{{1e30f, -1e30f}, {1e30f, -1e30f}, {1e30f, -1e30f}, kEmptyChild, 0};
         continue;
       }
       uint32_t c = slot[i];
@@ -220,8 +219,7 @@ __global__ void k_collapse(TreeView T, const uint2* qin, const uint32_t* qin_n, 
         ref = (int)child;
         meta = 0;
       }
-      N[2 * i] = make_float4(b.lo.x, b.lo.y, b.lo.z, __int_as_float(ref));
-      N[2 * i + 1] = make_float4(b.hi.x, b.hi.y, b.hi.z, __int_as_float(meta));
+      N[i] = NodeChild{{b.lo.x, b.hi.x}, {b.lo.y, b.hi.y}, {b.lo.z, b.hi.z}, ref, meta};
     }
   }
 }

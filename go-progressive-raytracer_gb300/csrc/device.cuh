@@ -438,17 +438,62 @@ struct TraceStats {
   uint32_t nodes, boxes, prims;
 };
 
+// What bounds the traversal and how it is laid out.  On a mesh the kernels
+// are bound by instruction issue at a fraction of the lanes (IPC 2.0-2.4,
+// 10-17 of 32 lanes per instruction with the boxes and leaves of a node in one
+// loop), on a handful of rays by the chain of loads of a node visit.  So a
+// visit is four 256-bit loads issued together and four box tests without a
+// branch (packed multiply-adds: two planes per instruction), and a leaf test
+// is a step of its own: a warp takes whichever step more of its lanes wait
+// for.  The leaves of a visited node come before any node below it, in slot
+// order, each checked against the hit so far when its turn comes: the
+// primitives are tested in the order, and culled by the comparisons, of a
+// loop that intersects each leaf as it meets it, so ties between equal
+// distances fall the same way.  Measured on GB300, before -> after: 2^24 rays
+// on 1.3 M triangles (closest hit) 23.0 -> 11.2 ms, 300,007 rays (any hit) on
+// 81,920 triangles 268 -> 186 us, the 1024^2 x 16 frame of the 1.3 M
+// triangles 28.7 -> 22.8 ms, a 128^2 x 1 pass of a sphere scene 907 -> 467 us.
 // State of one ray's traversal; `skip` is the primitive the ray leaves from:
 // a ray cannot re-enter the plane of the triangle or quad it starts on, and
 // for the sphere it starts on hits closer than 2e-4 x radius are rounding
 // noise of the FP32 origin.
+//
+// A ray is in one of two steps: it tests primitives [prim, end) of a leaf, or
+// (prim == end) it visits node `node`; node < 0 with no primitive left ends it.
+// The leaves a visited node's boxes let through are tested before any node
+// below it: `leaves` holds those of node `lnode` still to come (bit = child
+// slot), and `node` / `node_t` meanwhile the child to visit after them
+// (kPopNext: the top of the stack).
 struct Trav {
-  float3 o, d, inv, ood;
-  float tmin, best;
+  float3 o, d, inv, nood;  // nood = -(origin * inv)
+  float tmin, best;        // best: the hit distance so far (tmax before a hit)
   uint32_t skip;
   int node, sp;
-  Hit hit;
+  float node_t;  // entry distance of `node`
+  int lnode;
+  unsigned leaves;
+  int prim, end, type;
+  uint32_t hit;  // primitive hit so far (kNoHit, or the marker kOverflowHit)
+  float hu, hv;
+  __device__ __forceinline__ bool testing() const { return prim < end; }
+  __device__ __forceinline__ bool done() const { return prim >= end && node < 0; }
+  __device__ __forceinline__ Hit result() const { return Hit{hit < kOverflowHit ? best : -1.f, hit, hu, hv}; }
 };
+constexpr int kPopNext = -2;
+
+// One entry of a traversal stack: a node and the distance at which the ray
+// enters its box.
+struct TravEntry {
+  int node;
+  float t;
+};
+
+// 1 / d per axis, finite for directions along a plane.
+__device__ __forceinline__ float3 ray_inverse(float3 d) {
+  return f3(1.0f / (fabsf(d.x) > 1e-20f ? d.x : copysignf(1e-20f, d.x)),
+            1.0f / (fabsf(d.y) > 1e-20f ? d.y : copysignf(1e-20f, d.y)),
+            1.0f / (fabsf(d.z) > 1e-20f ? d.z : copysignf(1e-20f, d.z)));
+}
 
 // `root` is the BVH node the ray starts at (-1: nothing to intersect).  A
 // root carrying kRootStackCap starts the ray with only kTestStackCap free
@@ -456,140 +501,211 @@ struct Trav {
 // ends the traversal when popped), so that tests can drive the stack-overflow
 // path of one job on an ordinary scene.
 __device__ __forceinline__ void trav_init(Trav& s, float3 o, float3 d, float tmin, float tmax, uint32_t skip,
-                                          int root, int* stack) {
+                                          int root, TravEntry* stack) {
   s.o = o;
   s.d = d;
-  s.inv.x = 1.0f / (fabsf(d.x) > 1e-20f ? d.x : copysignf(1e-20f, d.x));
-  s.inv.y = 1.0f / (fabsf(d.y) > 1e-20f ? d.y : copysignf(1e-20f, d.y));
-  s.inv.z = 1.0f / (fabsf(d.z) > 1e-20f ? d.z : copysignf(1e-20f, d.z));
-  s.ood = o * s.inv;
+  s.inv = ray_inverse(d);
+  s.nood = -(o * s.inv);
   s.tmin = tmin;
   s.best = tmax;
   s.skip = skip;
   s.node = root;
   s.sp = 0;
+  s.leaves = 0;
+  s.prim = s.end = 0;
   if (root >= 0 && (root & kRootStackCap)) {
     s.node = root & ~kRootStackCap;
     s.sp = kTraceStack - kTestStackCap;
-    stack[s.sp - 1] = -1;
+    stack[s.sp - 1] = TravEntry{-1, -kInfF};
   }
-  s.hit.prim = kNoHit;
-  s.hit.t = -1.f;
-  s.hit.u = s.hit.v = 0.f;
+  s.hit = kNoHit;
+  s.hu = s.hv = 0.f;
 }
 
-// Visits node s.node: tests its children near-first, intersects the leaves
-// it hits, pushes the farther internal children and moves s.node to the
-// nearest one or to the top of the stack (-1 when the ray is finished).
-// Returns true when an any-hit query found a hit.  When the farther children
-// do not fit on the stack the ray ends at once with the marker hit
-// (prim = kOverflowHit): its result is not the closest hit, and the caller
-// reports the bound against the ray's job.
+// The two planes of each axis of a child box, the child's reference and meta
+// (layout.h), as four 64-bit words read in a single 256-bit load.
+struct ChildRec {
+  unsigned long long x, y, z, rm;
+  __device__ __forceinline__ int ref() const { return (int)(unsigned)rm; }
+  __device__ __forceinline__ int meta() const { return (int)(rm >> 32); }
+};
+__device__ __forceinline__ ChildRec ldg_child(const float4* p) {
+  ChildRec c;
+  asm("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];" : "=l"(c.x), "=l"(c.y), "=l"(c.z), "=l"(c.rm) : "l"(p));
+  return c;
+}
+// Both planes of one axis in one packed multiply-add: distances at which the
+// ray meets them, each rounded as fmaf(plane, inv, nood).
+__device__ __forceinline__ float2 slab(unsigned long long planes, float inv, float nood) {
+  unsigned long long k, c, r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(k) : "f"(inv));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(c) : "f"(nood));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(planes), "l"(k), "l"(c));
+  float2 t;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(t.x), "=f"(t.y) : "l"(r));
+  return t;
+}
+// Entry and exit distance of the ray in a child box, before the ray's own
+// far end.  Rounding is monotonic, so the nearer plane of each axis is the
+// smaller distance.
+__device__ __forceinline__ void child_span(float3 inv, float3 nood, float tmin, const ChildRec& c, float& tn,
+                                           float& tf) {
+  const float2 x = slab(c.x, inv.x, nood.x), y = slab(c.y, inv.y, nood.y), z = slab(c.z, inv.z, nood.z);
+  tn = fmaxf(fmaxf(fminf(x.x, x.y), fminf(y.x, y.y)), fmaxf(fminf(z.x, z.y), tmin));
+  tf = fminf(fminf(fmaxf(x.x, x.y), fmaxf(y.x, y.y)), fmaxf(z.x, z.y));
+}
+
+// Moves the ray to the nearest entry left on its stack, leaving out those
+// whose box starts behind the hit (nothing below them can be nearer).
+__device__ __forceinline__ void trav_pop(Trav& s, const TravEntry* stack) {
+  int node = -1;
+  while (s.sp > 0) {
+    const TravEntry e = stack[--s.sp];
+    if (!(e.t > s.best)) {
+      node = e.node;
+      break;
+    }
+  }
+  s.node = node;
+}
+
+// The ray's next leaf of node `lnode`, or, when none is left, its next node.
+// A leaf whose box starts behind a hit in a leaf before it is left out.
+__device__ __forceinline__ void trav_next_leaf(const DevScene& sc, Trav& s, const TravEntry* stack) {
+  while (s.leaves) {
+    const int i = __ffs(s.leaves) - 1;
+    s.leaves &= s.leaves - 1;
+    const ChildRec c = ldg_child(sc.nodes + (size_t)s.lnode * 8 + 2 * i);
+    float tn, tf;
+    child_span(s.inv, s.nood, s.tmin, c, tn, tf);
+    if (tn > s.best) continue;
+    s.prim = c.ref();
+    s.end = s.prim + (c.meta() & kLeafCountMask);
+    s.type = (c.meta() >> kLeafTypeShift) & 3;
+    return;
+  }
+  if (s.node == kPopNext || s.node_t > s.best) trav_pop(s, stack);
+}
+
+// The ray (o, d) against primitive p of type `type` (its global id in gid):
+// a hit with t in [tmin, best].
+__device__ __forceinline__ bool hit_prim(const DevScene& sc, int type, int p, float3 o, float3 d, float tmin, float best,
+                                         uint32_t skip, uint32_t& gid, float& t, float& u, float& v) {
+  u = v = 0.f;
+  if (type == kPrimTriangle) {
+    gid = (uint32_t)p;
+    if (gid == skip) return false;
+    const float4* T = sc.tris + (size_t)p * 3;
+    return hit_triangle(o, d, __ldg(T), __ldg(T + 1), __ldg(T + 2), tmin, best, t, u, v);
+  }
+  if (type == kPrimQuad) {
+    gid = sc.quad_base + (uint32_t)p;
+    if (gid == skip) return false;
+    const float4* Q = sc.quads + (size_t)p * 5;
+    float4 qq[5] = {__ldg(Q), __ldg(Q + 1), __ldg(Q + 2), __ldg(Q + 3), __ldg(Q + 4)};
+    return hit_quad(o, d, qq, tmin, best, t, u, v);
+  }
+  if (type == kPrimSphere) {
+    gid = sc.sphere_base + (uint32_t)p;
+    float4 S = __ldg(sc.spheres + (size_t)p * 2);
+    float lo = gid == skip ? fmaxf(tmin, 2e-4f * fabsf(S.w)) : tmin;
+    return hit_sphere(o, d, S, lo, best, t);
+  }
+  // a ray leaving a quadric may hit it again (the other side of a
+  // cylinder); hits closer than 2e-4 x radius are its own surface
+  gid = sc.quadric_base + (uint32_t)p;
+  const float4* Q = sc.quadrics + (size_t)p * 5;
+  float lo = tmin;
+  if (gid == skip) {
+    float4 g0 = __ldg(Q);
+    if (__float_as_int(__ldg(Q + 4).x) == kQuadricDisc) return false;  // planar
+    lo = fmaxf(tmin, 2e-4f * g0.w);
+  }
+  return hit_quadric(o, d, Q, lo, best, t, u);
+}
+
+// Tests the ray against primitive `prim` of its leaf and moves on: to the
+// leaf's next primitive, the node's next leaf or the ray's next node.
 template <bool kAnyHit, bool kCount>
-__device__ __forceinline__ bool trav_visit(const DevScene& sc, Trav& s, int* stack, TraceStats* st) {
+__device__ __forceinline__ void trav_prim(const DevScene& sc, Trav& s, const TravEntry* stack, TraceStats* st) {
+  uint32_t gid;
+  float t, u, v;
+  if (kCount) st->prims++;
+  if (hit_prim(sc, s.type, s.prim++, s.o, s.d, s.tmin, s.best, s.skip, gid, t, u, v)) {
+    s.best = t;
+    s.hu = u;
+    s.hv = v;
+    s.hit = gid;
+    if (kAnyHit) {
+      s.node = -1;
+      s.prim = s.end;
+      return;
+    }
+  }
+  if (s.prim == s.end) trav_next_leaf(sc, s, stack);
+}
+
+// Visits node s.node: tests its four children, pushes the farther internal
+// ones, and moves the ray to the first leaf it meets there, else to the
+// nearest internal child, else to the top of the stack.  When the farther
+// children do not fit on the stack the ray ends at once with the marker hit
+// (kOverflowHit): its result is not the closest hit, and the caller reports
+// the bound against the ray's job.
+template <bool kCount>
+__device__ __forceinline__ void trav_visit(const DevScene& sc, Trav& s, TravEntry* stack, TraceStats* st) {
   const float4* N = sc.nodes + (size_t)s.node * 8;
   if (kCount) st->nodes++;
-  int nint = 0;
-  int ich[4];
-  float itn[4];
+  ChildRec c[4];
+#pragma unroll
+  for (int i = 0; i < 4; i++) c[i] = ldg_child(N + 2 * i);
+  float tn[4];  // entry distances of the internal children hit, else infinite
+  int ref[4];
+  unsigned leaves = 0;
 #pragma unroll
   for (int i = 0; i < 4; i++) {
-    float4 a = __ldg(N + 2 * i);
-    int ref = __float_as_int(a.w);
-    if (ref == kEmptyChild) break;
-    float4 b = __ldg(N + 2 * i + 1);
-    int meta = __float_as_int(b.w);
-    if (kCount) st->boxes++;
-    float x0 = fmaf(s.inv.x < 0.f ? b.x : a.x, s.inv.x, -s.ood.x);
-    float x1 = fmaf(s.inv.x < 0.f ? a.x : b.x, s.inv.x, -s.ood.x);
-    float y0 = fmaf(s.inv.y < 0.f ? b.y : a.y, s.inv.y, -s.ood.y);
-    float y1 = fmaf(s.inv.y < 0.f ? a.y : b.y, s.inv.y, -s.ood.y);
-    float z0 = fmaf(s.inv.z < 0.f ? b.z : a.z, s.inv.z, -s.ood.z);
-    float z1 = fmaf(s.inv.z < 0.f ? a.z : b.z, s.inv.z, -s.ood.z);
-    float tn = fmaxf(fmaxf(x0, y0), fmaxf(z0, s.tmin));
-    float tf = fminf(fminf(x1, y1), fminf(z1, s.best));
-    if (tn > tf) continue;
-    if (meta == 0) {
-      int k = nint++;
-      while (k > 0 && itn[k - 1] > tn) {
-        itn[k] = itn[k - 1];
-        ich[k] = ich[k - 1];
-        k--;
-      }
-      itn[k] = tn;
-      ich[k] = ref;
-      continue;
-    }
-    int cnt = meta & kLeafCountMask;
-    int type = (meta >> kLeafTypeShift) & 3;
-    for (int k = 0; k < cnt; k++) {
-      int p = ref + k;
-      uint32_t gid = (type == kPrimTriangle ? 0u
-                      : type == kPrimQuad   ? sc.quad_base
-                      : type == kPrimSphere ? sc.sphere_base
-                                            : sc.quadric_base) +
-                     (uint32_t)p;
-      float t, u = 0.f, v = 0.f;
-      bool h;
-      if (kCount) st->prims++;
-      if (type == kPrimTriangle) {
-        if (gid == s.skip) continue;
-        const float4* T = sc.tris + (size_t)p * 3;
-        h = hit_triangle(s.o, s.d, __ldg(T), __ldg(T + 1), __ldg(T + 2), s.tmin, s.best, t, u, v);
-      } else if (type == kPrimQuad) {
-        if (gid == s.skip) continue;
-        const float4* Q = sc.quads + (size_t)p * 5;
-        float4 qq[5] = {__ldg(Q), __ldg(Q + 1), __ldg(Q + 2), __ldg(Q + 3), __ldg(Q + 4)};
-        h = hit_quad(s.o, s.d, qq, s.tmin, s.best, t, u, v);
-      } else if (type == kPrimSphere) {
-        float4 S = __ldg(sc.spheres + (size_t)p * 2);
-        float lo = gid == s.skip ? fmaxf(s.tmin, 2e-4f * fabsf(S.w)) : s.tmin;
-        h = hit_sphere(s.o, s.d, S, lo, s.best, t);
-      } else {
-        // a ray leaving a quadric may hit it again (the other side of a
-        // cylinder); hits closer than 2e-4 x radius are its own surface
-        const float4* Q = sc.quadrics + (size_t)p * 5;
-        float lo = s.tmin;
-        if (gid == s.skip) {
-          float4 g0 = __ldg(Q);
-          if (__float_as_int(__ldg(Q + 4).x) == kQuadricDisc) continue;  // planar
-          lo = fmaxf(s.tmin, 2e-4f * g0.w);
-        }
-        h = hit_quadric(s.o, s.d, Q, lo, s.best, t, u);
-      }
-      if (h) {
-        s.best = t;
-        s.hit.t = t;
-        s.hit.u = u;
-        s.hit.v = v;
-        s.hit.prim = gid;
-        if (kAnyHit) {
-          s.node = -1;
-          return true;
-        }
-      }
+    float tf;
+    child_span(s.inv, s.nood, s.tmin, c[i], tn[i], tf);
+    ref[i] = c[i].ref();
+    const bool used = ref[i] != kEmptyChild;
+    if (kCount) st->boxes += used;
+    const bool hit = used && !(tn[i] > fminf(tf, s.best));
+    const bool leaf = c[i].meta() != 0;
+    if (hit && leaf) leaves |= 1u << i;
+    if (!hit || leaf) {
+      tn[i] = kInfF;
+      ref[i] = -1;
     }
   }
-  // internal children still nearer than the (possibly shrunk) best distance
-  int keep = 0;
-  for (int k = 0; k < nint; k++)
-    if (itn[k] <= s.best) {
-      itn[keep] = itn[k];
-      ich[keep] = ich[k];
-      keep++;
-    }
-  if (keep > 0) {
-    if (s.sp + keep - 1 > kTraceStack) {
-      s.node = -1;
-      s.hit.prim = kOverflowHit;
-      return false;
-    }
-    for (int k = keep - 1; k >= 1; k--) stack[s.sp++] = ich[k];
-    s.node = ich[0];
-  } else {
-    s.node = s.sp > 0 ? stack[--s.sp] : -1;
+  // nearest first: an odd-even transposition network, stable as only a
+  // strictly greater neighbour changes places
+  auto order = [&](int i, int j) {
+    const bool swap = tn[i] > tn[j];
+    const float t0 = swap ? tn[j] : tn[i], t1 = swap ? tn[i] : tn[j];
+    const int r0 = swap ? ref[j] : ref[i], r1 = swap ? ref[i] : ref[j];
+    tn[i] = t0;
+    tn[j] = t1;
+    ref[i] = r0;
+    ref[j] = r1;
+  };
+  order(0, 1);
+  order(2, 3);
+  order(1, 2);
+  order(0, 1);
+  order(2, 3);
+  order(1, 2);
+  if (s.sp + (ref[1] >= 0) + (ref[2] >= 0) + (ref[3] >= 0) > kTraceStack) {
+    s.node = -1;
+    s.hit = kOverflowHit;
+    return;
   }
-  return false;
+  if (ref[3] >= 0) stack[s.sp++] = TravEntry{ref[3], tn[3]};
+  if (ref[2] >= 0) stack[s.sp++] = TravEntry{ref[2], tn[2]};
+  if (ref[1] >= 0) stack[s.sp++] = TravEntry{ref[1], tn[1]};
+  s.leaves = leaves;
+  s.lnode = s.node;
+  s.node = ref[0] >= 0 ? ref[0] : kPopNext;
+  s.node_t = tn[0];
+  if (leaves || ref[0] < 0) trav_next_leaf(sc, s, stack);
 }
 
 // Whole traversal of one ray from BVH node `root`.  A stack overflow returns
@@ -598,39 +714,120 @@ template <bool kAnyHit, bool kCount>
 __device__ __forceinline__ bool trace_from(const DevScene& sc, int root, float3 o, float3 d, float tmin, float tmax,
                                            uint32_t skip, Hit& hit, int* err, TraceStats* st = nullptr) {
   Trav s;
-  int stack[kTraceStack];
+  TravEntry stack[kTraceStack];
   trav_init(s, o, d, tmin, tmax, skip, root, stack);
   while (s.node >= 0) {
-    if (trav_visit<kAnyHit, kCount>(sc, s, stack, st)) break;
+    trav_visit<kCount>(sc, s, stack, st);
+    while (s.testing()) trav_prim<kAnyHit, kCount>(sc, s, stack, st);
   }
-  if (s.hit.prim == kOverflowHit) {
+  if (s.hit == kOverflowHit) {
     if (err) atomicOr(err, kErrStackOverflow);
-    s.hit.prim = kNoHit;
-    s.hit.t = -1.f;
+    s.hit = kNoHit;
   }
-  hit = s.hit;
-  return s.hit.prim != kNoHit;
+  hit = s.result();
+  return s.hit != kNoHit;
 }
 
-// Whole traversal of one ray of the scene (used inside the BDPT kernel).
+// A scene whose BVH is a single node holds only leaves (the host builder's
+// layout of at most 32 primitives, and anything smaller).
+__host__ __device__ __forceinline__ bool one_node(const DevScene& sc) { return sc.n_nodes == 1; }
+
+// Whole traversal of one ray of a one-node scene: its leaves in slot order,
+// each primitive by every lane of the warp at once, so that the loop, the
+// type and the record's address are the same for all lanes; a lane whose ray
+// misses the leaf's box sits it out.  The tests and their order are those of
+// trav_visit / trav_prim, whose step per primitive costs more here than the
+// lanes it fills (Cornell box, 18 quads, 400^2 x 64: 10.7 ms a frame stepped,
+// 7.8 ms in this loop).
 template <bool kAnyHit, bool kCount>
+__device__ __forceinline__ bool trace_one_node(const DevScene& sc, float3 o, float3 d, float tmin, float tmax,
+                                               uint32_t skip, Hit& hit, TraceStats* st = nullptr) {
+  const float3 inv = ray_inverse(d);
+  const float3 nood = -(o * inv);
+  float best = tmax, hu = 0.f, hv = 0.f;
+  uint32_t prim = kNoHit;
+  if (kCount) st->nodes++;
+  for (int i = 0; i < 4; i++) {
+    const ChildRec c = ldg_child(sc.nodes + 2 * i);
+    if (c.ref() == kEmptyChild) break;
+    if (kCount) st->boxes++;
+    float tn, tf;
+    child_span(inv, nood, tmin, c, tn, tf);
+    const bool in = !(tn > fminf(tf, best));
+    const int type = (c.meta() >> kLeafTypeShift) & 3, end = c.ref() + (c.meta() & kLeafCountMask);
+    auto leaf = [&](int kind) {
+      for (int p = c.ref(); p < end; p++) {
+        if (!in || (kAnyHit && prim != kNoHit)) continue;
+        uint32_t gid;
+        float t, u, v;
+        if (kCount) st->prims++;
+        if (hit_prim(sc, kind, p, o, d, tmin, best, skip, gid, t, u, v)) {
+          best = t;
+          hu = u;
+          hv = v;
+          prim = gid;
+        }
+      }
+    };
+    if (type == kPrimTriangle) leaf(kPrimTriangle);
+    else if (type == kPrimQuad) leaf(kPrimQuad);
+    else if (type == kPrimSphere) leaf(kPrimSphere);
+    else leaf(kPrimQuadric);
+  }
+  hit = Hit{prim != kNoHit ? best : -1.f, prim, hu, hv};
+  return prim != kNoHit;
+}
+
+// Whole traversal of one ray of the scene (the BDPT strategy kernels), in the
+// form for one_node(sc): a kernel holds one form, as both together spill.
+template <bool kAnyHit, bool kCount, bool kOneNode>
 __device__ __forceinline__ bool trace(const DevScene& sc, float3 o, float3 d, float tmin, float tmax, uint32_t skip,
                                       Hit& hit, int* err, TraceStats* st = nullptr) {
+  if (kOneNode) return trace_one_node<kAnyHit, kCount>(sc, o, d, tmin, tmax, skip, hit, st);
   return trace_from<kAnyHit, kCount>(sc, sc.root, o, d, tmin, tmax, skip, hit, err, st);
 }
 
+// A batch of rays of a one-node scene, one ray per thread (every ray costs
+// the same, so there is nothing to refill).
+template <bool kAnyHit, bool kCount, class Source>
+__device__ __forceinline__ void trace_batch_one_node(const DevScene& sc, Source& src, TraceStats* st,
+                                                     uint32_t* traced) {
+  const uint32_t n = src.count();
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    float3 o, d;
+    float tmin, tmax;
+    uint32_t skip;
+    int root;
+    src.load(i, o, d, tmin, tmax, skip, root);
+    Hit h;
+    trace_one_node<kAnyHit, kCount>(sc, o, d, tmin, tmax, skip, h, st);
+    src.store(i, h);
+    if (kCount) (*traced)++;
+  }
+}
+
 // Persistent traversal of a batch of rays: every warp loops until its work
-// is exhausted, one node visit per iteration, and lanes whose ray finished
-// take new rays once at least 16 lanes are idle (half the warp: fewer,
-// larger refills; on the sphere-scene batch extend + shadow ran 665 ms per
-// batch at 8, 632 at 16, 640 at 24), so warps stay full instead of waiting
-// for their slowest ray.  A warp draws rays from a chunk: with
-// `work` != null, chunks of 64 rays come from that counter (zeroed by the
-// previous kernel on the same stream); otherwise each warp owns a static
-// contiguous range of the batch.  Source provides count(),
+// is exhausted, one step per iteration (node visits or primitive tests,
+// whichever more lanes wait for), and lanes whose ray finished take new rays
+// once at least 16 lanes are idle (8, 12 and 20 measured within 2 %: 69.9,
+// 68.6 and 68.5 against 68.3 ms on the sphere batch, 22.7, 22.8 and 23.1
+// against 22.8 ms on 1.3 M triangles), so warps stay full instead of waiting
+// for their slowest ray.  Rays are dealt in chunks of up to 64.  Warp w of W
+// starts on chunk w; with `work` != null the chunks after the first W come
+// from that counter (zeroed by the previous kernel on the same stream),
+// otherwise warp w goes on with chunks w + W, w + 2 W, ... (calls on
+// different streams share no counter; one contiguous range per warp left the
+// warps of the cheap half of a batch idle).  A batch of fewer than 64 rays per
+// warp is dealt out in one smaller chunk per warp, so that it spreads over
+// the chip and draws nothing from the counter.  Source provides count(),
 // load(i, o, d, tmin, tmax, skip, root) and store(i, hit); store() sees the
 // marker hit of a ray that overflowed its stack and reports it.
 constexpr uint32_t kFetchChunk = 64;
+constexpr int kRefillIdle = 16;
+// 128-thread blocks per SM of the traversal kernels: 64 registers, 40 bytes
+// spilled; 7 blocks (72 registers) and 6 (80) measured 2 % and 6 % slower on
+// the sphere batch, 0 and 5 % on the 1.3 M triangles.
+constexpr int kTravBlocks = 8;
 
 template <bool kAnyHit, bool kCount, class Source>
 __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src, uint32_t* work, TraceStats* st,
@@ -638,29 +835,31 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
   const uint32_t n = src.count();
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
-  uint32_t cur, end;  // the warp's current chunk [cur, end), warp-uniform
-  if (work) {
-    cur = end = 0;
-  } else {
-    uint64_t w = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
-    uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    cur = (uint32_t)(n * w / nw);
-    end = (uint32_t)(n * (w + 1) / nw);
-  }
-  bool more = true;  // the warp may still draw rays
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t chunk = min(kFetchChunk, (n + nw - 1) / nw);
+  // the warp's current chunk [cur, end), warp-uniform
+  uint32_t cur = min((uint64_t)n, (uint64_t)w * chunk), end = min((uint64_t)n, (uint64_t)cur + chunk);
+  bool more = cur < end;  // the warp may still draw rays
+  uint32_t next = w;      // without `work`: the chunk it holds
   Trav s;
-  int stack[kTraceStack];
+  TravEntry stack[kTraceStack];
   int ray = -1;
   for (;;) {
-    bool idle = ray < 0;
-    unsigned idle_mask = __ballot_sync(0xffffffffu, idle);
-    if (more && idle_mask && (__popc(idle_mask) >= 16 || idle_mask == 0xffffffffu)) {
-      if (cur == end && work) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, kFetchChunk);
-        base = __shfl_sync(0xffffffffu, base, 0);
-        cur = min(base, n);
-        end = min(base + kFetchChunk, n);
+    const bool idle = ray < 0, testing = !idle && s.testing();
+    const unsigned idle_mask = __ballot_sync(0xffffffffu, idle), test_mask = __ballot_sync(0xffffffffu, testing);
+    if (more && __popc(idle_mask) >= kRefillIdle) {
+      if (cur == end) {
+        uint64_t at;
+        if (work) {
+          uint32_t base = 0;
+          if (n > (uint64_t)nw * chunk && lane == 0) base = atomicAdd(work, chunk);
+          at = (uint64_t)nw * chunk + __shfl_sync(0xffffffffu, base, 0);
+        } else {
+          next += nw;
+          at = (uint64_t)next * chunk;
+        }
+        cur = (uint32_t)min((uint64_t)n, at);
+        end = (uint32_t)min((uint64_t)n, at + chunk);
       }
       if (cur == end) {
         more = false;
@@ -680,14 +879,18 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
         }
         cur += take;
       }
+      continue;
     }
-    if (__ballot_sync(0xffffffffu, ray >= 0) == 0 && !more) break;
-    if (ray >= 0) {
-      if (s.node >= 0) trav_visit<kAnyHit, kCount>(sc, s, stack, st);
-      if (s.node < 0) {
-        src.store((uint32_t)ray, s.hit);
-        ray = -1;
-      }
+    if (idle_mask == 0xffffffffu) break;
+    // the step that more lanes wait for
+    if (2 * __popc(test_mask) > 32 - __popc(idle_mask)) {
+      if (testing) trav_prim<kAnyHit, kCount>(sc, s, stack, st);
+    } else if (!idle && !testing && s.node >= 0) {
+      trav_visit<kCount>(sc, s, stack, st);
+    }
+    if (!idle && s.done()) {
+      src.store((uint32_t)ray, s.result());
+      ray = -1;
     }
   }
 }

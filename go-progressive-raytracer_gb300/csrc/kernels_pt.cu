@@ -54,13 +54,14 @@ struct BatchSource {
   }
 };
 
-// Batches use static per-warp ranges: calls on different streams share no counter.
-template <bool kAny>
-__global__ void __launch_bounds__(128, 8) k_intersect(DevScene sc, BatchSource src) {
-  trace_persistent<kAny, false>(sc, src, nullptr, nullptr, nullptr);
+// Batches deal their rays out without a counter: calls on different streams share none.
+template <bool kAny, bool kOneNode>
+__global__ void __launch_bounds__(128, kTravBlocks) k_intersect(DevScene sc, BatchSource src) {
+  if (kOneNode) trace_batch_one_node<kAny, false>(sc, src, nullptr, nullptr);
+  else trace_persistent<kAny, false>(sc, src, nullptr, nullptr, nullptr);
 }
 
-int persistent_grid(int sm_count, int block) { return std::max(1, sm_count * (1024 / block)); }
+int persistent_grid(int sm_count, int block) { return std::max(1, sm_count * kTravBlocks * 128 / block); }
 
 void launch_intersect(const DevScene& sc, const gprt_ray* rays, uint32_t n, bool any_hit, gprt_hit* hits, int* err,
                       cudaStream_t st) {
@@ -70,8 +71,9 @@ void launch_intersect(const DevScene& sc, const gprt_ray* rays, uint32_t n, bool
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int grid = launch_grid((n + 31) / 32 * 32, 128, persistent_grid(sms, 128));
   BatchSource src{rays, hits, n, sc.root, err};
-  if (any_hit) k_intersect<true><<<grid, 128, 0, st>>>(sc, src);
-  else k_intersect<false><<<grid, 128, 0, st>>>(sc, src);
+  auto kernel = one_node(sc) ? (any_hit ? k_intersect<true, true> : k_intersect<false, true>)
+                             : (any_hit ? k_intersect<true, false> : k_intersect<false, false>);
+  kernel<<<grid, 128, 0, st>>>(sc, src);
 }
 
 // ----------------------------------------------------------------- raygen
@@ -160,8 +162,8 @@ struct ExtendSource {
 // The error sink of a wavefront's paths (per job, or per item of a multi-job step).
 static ErrSink err_sink(const DevPaths& P) { return ErrSink{P.counters + 3, P.item_err, P.item_start, P.n_items}; }
 
-template <bool kCount>
-__global__ void __launch_bounds__(128, 8)
+template <bool kCount, bool kOneNode>
+__global__ void __launch_bounds__(128, kTravBlocks)
     k_pt_extend(DevScene sc, ExtendSource src, uint32_t* counters, int cur, unsigned long long* stats) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     counters[cur ^ 1] = 0;  // next queue and shadow queue start empty
@@ -171,8 +173,12 @@ __global__ void __launch_bounds__(128, 8)
   }
   TraceStats ts{0, 0, 0};
   uint32_t rays = 0;
-  trace_persistent<false, kCount>(sc, src, counters + 4, &ts, &rays);
-  if (kCount) add_counts(stats, rays, ts);
+  if (kOneNode) trace_batch_one_node<false, kCount>(sc, src, &ts, &rays);
+  else trace_persistent<false, kCount>(sc, src, counters + 4, &ts, &rays);
+  if (kCount) {
+    __syncwarp();
+    add_counts(stats, rays, ts);
+  }
 }
 
 // One ray per thread (grid-stride), the variant GPRT_JOB_SIMPLE_EXTEND selects.
@@ -221,9 +227,9 @@ void launch_pt_extend(const DevScene& sc, const DevPaths& P, int cur, int bounce
     else k_pt_extend_simple<false><<<grid, b, 0, st>>>(sc, src, P.counters, cur, P.stats);
     return;
   }
-  int g = persistent_grid(sm_count_current(), 128);
-  if (P.stats) k_pt_extend<true><<<g, 128, 0, st>>>(sc, src, P.counters, cur, P.stats);
-  else k_pt_extend<false><<<g, 128, 0, st>>>(sc, src, P.counters, cur, P.stats);
+  auto kernel = one_node(sc) ? (P.stats ? k_pt_extend<true, true> : k_pt_extend<false, true>)
+                             : (P.stats ? k_pt_extend<true, false> : k_pt_extend<false, false>);
+  kernel<<<persistent_grid(sm_count_current(), 128), 128, 0, st>>>(sc, src, P.counters, cur, P.stats);
 }
 
 // ----------------------------------------------------------------- shade
@@ -321,13 +327,17 @@ struct ShadowSource {
   }
 };
 
-template <bool kCount>
-__global__ void __launch_bounds__(128, 8)
+template <bool kCount, bool kOneNode>
+__global__ void __launch_bounds__(128, kTravBlocks)
     k_pt_shadow(DevScene sc, ShadowSource src, uint32_t* counters, unsigned long long* stats) {
   TraceStats ts{0, 0, 0};
   uint32_t rays = 0;
-  trace_persistent<true, kCount>(sc, src, counters + 5, &ts, &rays);
-  if (kCount) add_counts(stats + 4, rays, ts);
+  if (kOneNode) trace_batch_one_node<true, kCount>(sc, src, &ts, &rays);
+  else trace_persistent<true, kCount>(sc, src, counters + 5, &ts, &rays);
+  if (kCount) {
+    __syncwarp();
+    add_counts(stats + 4, rays, ts);
+  }
 }
 
 // One shadow ray per thread (grid-stride), the variant GPRT_JOB_SIMPLE_SHADOW selects.
@@ -362,9 +372,9 @@ void launch_pt_shadow(const DevScene& sc, const DevPaths& P, int cur, int block,
     else k_pt_shadow_simple<false><<<grid, b, 0, st>>>(sc, src, P.counters, P.stats);
     return;
   }
-  int g = persistent_grid(sm_count_current(), 128);
-  if (P.stats) k_pt_shadow<true><<<g, 128, 0, st>>>(sc, src, P.counters, P.stats);
-  else k_pt_shadow<false><<<g, 128, 0, st>>>(sc, src, P.counters, P.stats);
+  auto kernel = one_node(sc) ? (P.stats ? k_pt_shadow<true, true> : k_pt_shadow<false, true>)
+                             : (P.stats ? k_pt_shadow<true, false> : k_pt_shadow<false, false>);
+  kernel<<<persistent_grid(sm_count_current(), 128), 128, 0, st>>>(sc, src, P.counters, P.stats);
 }
 
 // ----------------------------------------------------------------- accumulate

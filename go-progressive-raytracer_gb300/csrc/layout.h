@@ -3,10 +3,12 @@
 //
 // HBM layout (all arrays 16-byte aligned, read with 16-byte vector loads):
 //   nodes      8 x float4 (128 B, one cache line) per 4-wide BVH node; child i
-//              is the pair (lo.x, lo.y, lo.z, ref) (hi.x, hi.y, hi.z, meta):
+//              is the pair (lo.x, hi.x, lo.y, hi.y) (lo.z, hi.z, ref, meta)
+//              (NodeChild): the two planes of an axis side by side for one
+//              packed multiply-add, the 32 B of a child in one load;
 //              ref = node index (meta == 0), first primitive of a leaf
 //              (meta = count | type << 8), or kEmptyChild.  Used slots come
-//              first, so a traversal stops at the first empty one.
+//              first.
 //   tris       3 x float4 (48 B): (v0, material) (e1 = v1 - v0, group) (e2 = v2 - v0, -)
 //   tri_normals 1 x float4 per triangle: normalize(e1 x e2) computed in float64,
 //              or the mesh's custom normal (TriangleMeshOptions.Normals), normalised
@@ -98,6 +100,13 @@ struct DevLight {
   float radius;  // sphere light radius
 };
 static_assert(sizeof(DevLight) == 64, "DevLight is four 16-byte words");
+
+// One child slot of a node.
+struct alignas(16) NodeChild {
+  float x[2], y[2], z[2];  // lower and upper plane of each axis
+  int ref, meta;
+};
+static_assert(sizeof(NodeChild) == 32, "a child is half a 64-byte pair of sectors");
 
 // Camera (pkg/geometry/camera.go:35-67), derived in float64 on the host
 struct DevCamera {

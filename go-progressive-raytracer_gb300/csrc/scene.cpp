@@ -485,10 +485,9 @@ struct Emitter {
         meta[i] = 0;
       }
     }
-    float4* N = &out.nodes[(size_t)idx * 8];
-    for (int i = 0; i < 4; i++) {  // child i: (lo, ref) (hi, meta)
-      N[2 * i] = make_float4(lo[0][i], lo[1][i], lo[2][i], i2f((uint32_t)child[i]));
-      N[2 * i + 1] = make_float4(hi[0][i], hi[1][i], hi[2][i], i2f((uint32_t)meta[i]));
+    for (int i = 0; i < 4; i++) {
+      const NodeChild c = {{lo[0][i], hi[0][i]}, {lo[1][i], hi[1][i]}, {lo[2][i], hi[2][i]}, child[i], meta[i]};
+      std::memcpy(&out.nodes[(size_t)idx * 8 + 2 * i], &c, sizeof(c));
     }
     return idx;
   }
@@ -1127,10 +1126,10 @@ std::string validate_layout(const HostScene& s) {
   for (size_t k = 0; k < nn; k++) nseen[k].store(0, std::memory_order_relaxed);
   std::mutex mu;
   std::string first_err;
-  auto ri = [](float f) {
-    int x;
-    std::memcpy(&x, &f, 4);
-    return x;
+  auto child_of = [&](size_t n, int i) {
+    NodeChild c;
+    std::memcpy(&c, &s.nodes[n * 8 + 2 * i], sizeof(c));
+    return c;
   };
   parallel_for(nn, [&](size_t b0, size_t b1) {
     auto bad = [&](const char* m) {
@@ -1138,26 +1137,25 @@ std::string validate_layout(const HostScene& s) {
       if (first_err.empty()) first_err = m;
     };
     for (size_t n = b0; n < b1; n++) {
-      const float4* N = &s.nodes[n * 8];
       bool seen_empty = false;
       for (int i = 0; i < 4; i++) {
-        const float4 &A = N[2 * i], &B = N[2 * i + 1];
-        int ch = ri(A.w), mt = ri(B.w);
+        const NodeChild A = child_of(n, i);
+        int ch = A.ref, mt = A.meta;
         if (ch == kEmptyChild) {
           seen_empty = true;
           continue;
         }
         if (seen_empty) return bad("used child slot after an empty one");
-        float lo[3] = {A.x, A.y, A.z}, hi[3] = {B.x, B.y, B.z};
+        float lo[3] = {A.x[0], A.y[0], A.z[0]}, hi[3] = {A.x[1], A.y[1], A.z[1]};
         auto inside = [&](float x, int k) { return x >= lo[k] && x <= hi[k]; };
         if (mt == 0) {
           if (ch <= (int)n || (size_t)ch >= nn) return bad("bad child node index");
           nseen[ch].fetch_add(1, std::memory_order_relaxed);
-          const float4* C = &s.nodes[(size_t)ch * 8];
           for (int j = 0; j < 4; j++) {
-            const float4 &CA = C[2 * j], &CB = C[2 * j + 1];
-            if (ri(CA.w) == kEmptyChild) continue;
-            if (!(CA.x >= lo[0] && CB.x <= hi[0] && CA.y >= lo[1] && CB.y <= hi[1] && CA.z >= lo[2] && CB.z <= hi[2]))
+            const NodeChild C = child_of((size_t)ch, j);
+            if (C.ref == kEmptyChild) continue;
+            if (!(C.x[0] >= lo[0] && C.x[1] <= hi[0] && C.y[0] >= lo[1] && C.y[1] <= hi[1] && C.z[0] >= lo[2] &&
+                  C.z[1] <= hi[2]))
               return bad("child box not inside its parent slot");
           }
           continue;
@@ -1302,13 +1300,6 @@ void count_traversal(const HostScene& s, const gprt_ray* rays, uint32_t n, bool 
                      uint64_t& boxes, uint64_t& prims) {
   nodes = boxes = prims = 0;
   if (s.nodes.empty()) return;
-  auto rd = [](const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; };
-  auto ri = [&](const float4& v, int i) {
-    float f = rd(v, i);
-    int x;
-    std::memcpy(&x, &f, 4);
-    return x;
-  };
   for (uint32_t r = 0; r < n; r++) {
     const gprt_ray& ray = rays[r];
     float o[3] = {ray.ox, ray.oy, ray.oz}, d[3] = {ray.dx, ray.dy, ray.dz};
@@ -1323,18 +1314,20 @@ void count_traversal(const HostScene& s, const gprt_ray* rays, uint32_t n, bool 
     float best = ray.tmax;
     bool done = false;
     while (node >= 0 && !done) {
-      const float4* N = &s.nodes[(size_t)node * 8];
       nodes++;
       int ich[4];
       float itn[4];
       int nint = 0;
       for (int i = 0; i < 4 && !done; i++) {
-        int ch = ri(N[2 * i], 3), mt = ri(N[2 * i + 1], 3);
+        NodeChild c;
+        std::memcpy(&c, &s.nodes[(size_t)node * 8 + 2 * i], sizeof(c));
+        const int ch = c.ref, mt = c.meta;
         if (ch == kEmptyChild) break;
         boxes++;
         float t0[3], t1[3];
         for (int k = 0; k < 3; k++) {
-          float lo = rd(N[2 * i], k), hi = rd(N[2 * i + 1], k);
+          const float* plane = k == 0 ? c.x : k == 1 ? c.y : c.z;
+          float lo = plane[0], hi = plane[1];
           bool neg = inv[k] < 0;
           t0[k] = std::fma(neg ? hi : lo, inv[k], -ood[k]);
           t1[k] = std::fma(neg ? lo : hi, inv[k], -ood[k]);

@@ -197,16 +197,15 @@ __global__ void k_srv_accumulate(DevPaths P, const StepHdr* hdr, const uint32_t*
 __global__ void k_rebase_nodes(float4* nodes, uint32_t n, int node_off, int tri_off, int quad_off, int sph_off,
                                int qdr_off) {
   for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < n * 4u; c += gridDim.x * blockDim.x) {
-    float4* a = nodes + (size_t)(c >> 2) * 8 + 2 * (c & 3);
-    int ref = __float_as_int(a->w);
-    if (ref == kEmptyChild) continue;
-    int meta = __float_as_int(a[1].w);
+    NodeChild* a = reinterpret_cast<NodeChild*>(nodes) + c;
+    const int meta = a->meta;
+    if (a->ref == kEmptyChild) continue;
     int off = node_off;
     if (meta != 0) {
       int type = (meta >> kLeafTypeShift) & 3;
       off = type == kPrimTriangle ? tri_off : type == kPrimQuad ? quad_off : type == kPrimSphere ? sph_off : qdr_off;
     }
-    a->w = __int_as_float(ref + off);
+    a->ref += off;
   }
 }
 
