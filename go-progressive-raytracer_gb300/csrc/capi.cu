@@ -143,6 +143,15 @@ void run_chunk(gprt_job* j, const ChunkDesc& ch) {
     j->launches += 2;
     return;
   }
+  // a small chunk in one launch, unless the job asks for a variant of the
+  // wavefront's kernels or for their times and counters
+  const uint32_t wavefront = kVariantBits | GPRT_JOB_TIME_KERNELS | GPRT_JOB_COUNT_TRAVERSAL;
+  if (!(j->desc.flags & wavefront) && n <= pt_paths_max(sc, ctx->sm_count) && sc.max_depth > 0) {
+    launch_pt_paths(sc, j->film, j->paths, ch, ctx->sm_count, j->stream);
+    launch_accumulate(j->film, j->paths, ch, 256, j->stream);
+    j->launches += 2;
+    return;
+  }
   {
     TimedLaunch t(j, 3);
     launch_pt_raygen(sc, j->film, j->paths, ch, block, j->stream);
@@ -919,13 +928,17 @@ extern "C" int gprt_render_noalloc(gprt_scene* s, uint32_t spp, uint64_t seed, f
   const DevScene& sc = s->dev;
   const int block = 128;
   int grid = launch_grid((uint32_t)(npix * spp), block, std::max(1, ctx->sm_count * (2048 / block)));
-  launch_pt_raygen(sc, film, P, ch, block, st);
-  int cur = 0;
-  for (int b = 0; b < sc.max_depth; b++) {
-    launch_pt_extend(sc, P, cur, b, block, grid, st);
-    launch_pt_shade(sc, P, ch, cur, b, block, grid, st);
-    launch_pt_shadow(sc, P, cur, block, grid, st);
-    cur ^= 1;
+  if (npix * spp <= pt_paths_max(sc, ctx->sm_count) && sc.max_depth > 0) {
+    launch_pt_paths(sc, film, P, ch, ctx->sm_count, st);
+  } else {
+    launch_pt_raygen(sc, film, P, ch, block, st);
+    int cur = 0;
+    for (int b = 0; b < sc.max_depth; b++) {
+      launch_pt_extend(sc, P, cur, b, block, grid, st);
+      launch_pt_shade(sc, P, ch, cur, b, block, grid, st);
+      launch_pt_shadow(sc, P, cur, block, grid, st);
+      cur ^= 1;
+    }
   }
   k_noalloc_mean<<<launch_grid((uint32_t)npix, 256, 0), 256, 0, st>>>(P, (uint32_t)npix, spp, rgb_out, status_out);
   cudaError_t e = cudaGetLastError();

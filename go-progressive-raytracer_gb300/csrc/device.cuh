@@ -34,8 +34,25 @@ __device__ __forceinline__ float3 normalize(float3 a) {
   float l = length(a);
   return l == 0.f ? f3(0.f, 0.f, 0.f) : f3(a.x / l, a.y / l, a.z / l);
 }
+// normalize with the rounding of the squared length spelled out: z z + (x x +
+// y y) with y y rounded first, or (normalize_yx) x x rounded first.  Kernels
+// that inline the shading code differently then give the same directions.
+__device__ __forceinline__ float3 normalize_by(float3 a, float l2) {
+  float l = sqrtf(l2);
+  return l == 0.f ? f3(0.f, 0.f, 0.f) : f3(a.x / l, a.y / l, a.z / l);
+}
+__device__ __forceinline__ float3 normalize_xy(float3 a) {
+  return normalize_by(a, __fmaf_rn(a.z, a.z, __fmaf_rn(a.x, a.x, __fmul_rn(a.y, a.y))));
+}
+__device__ __forceinline__ float3 normalize_yx(float3 a) {
+  return normalize_by(a, __fmaf_rn(a.z, a.z, __fmaf_rn(a.y, a.y, __fmul_rn(a.x, a.x))));
+}
 // core.Vec3.Luminance (pkg/core/vec3.go:134-136)
 __device__ __forceinline__ float luminance(float3 c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z; }
+// with its roundings spelled out (as normalize_xy)
+__device__ __forceinline__ float luminance_xy(float3 c) {
+  return __fmaf_rn(0.0722f, c.z, __fmaf_rn(0.2126f, c.x, __fmul_rn(0.7152f, c.y)));
+}
 __device__ __forceinline__ bool is_zero(float3 c) { return c.x == 0.f && c.y == 0.f && c.z == 0.f; }
 
 constexpr float kPi = 3.14159265358979323846f;
@@ -626,8 +643,9 @@ __device__ __forceinline__ bool hit_prim(const DevScene& sc, int type, int p, fl
 
 // Tests the ray against primitive `prim` of its leaf and moves on: to the
 // leaf's next primitive, the node's next leaf or the ray's next node.
-template <bool kAnyHit, bool kCount>
-__device__ __forceinline__ void trav_prim(const DevScene& sc, Trav& s, const TravEntry* stack, TraceStats* st) {
+template <bool kCount>
+__device__ __forceinline__ void trav_prim(const DevScene& sc, Trav& s, bool any_hit, const TravEntry* stack,
+                                          TraceStats* st) {
   uint32_t gid;
   float t, u, v;
   if (kCount) st->prims++;
@@ -636,7 +654,7 @@ __device__ __forceinline__ void trav_prim(const DevScene& sc, Trav& s, const Tra
     s.hu = u;
     s.hv = v;
     s.hit = gid;
-    if (kAnyHit) {
+    if (any_hit) {
       s.node = -1;
       s.prim = s.end;
       return;
@@ -718,7 +736,7 @@ __device__ __forceinline__ bool trace_from(const DevScene& sc, int root, float3 
   trav_init(s, o, d, tmin, tmax, skip, root, stack);
   while (s.node >= 0) {
     trav_visit<kCount>(sc, s, stack, st);
-    while (s.testing()) trav_prim<kAnyHit, kCount>(sc, s, stack, st);
+    while (s.testing()) trav_prim<kCount>(sc, s, kAnyHit, stack, st);
   }
   if (s.hit == kOverflowHit) {
     if (err) atomicOr(err, kErrStackOverflow);
@@ -884,7 +902,7 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
     if (idle_mask == 0xffffffffu) break;
     // the step that more lanes wait for
     if (2 * __popc(test_mask) > 32 - __popc(idle_mask)) {
-      if (testing) trav_prim<kAnyHit, kCount>(sc, s, stack, st);
+      if (testing) trav_prim<kCount>(sc, s, kAnyHit, stack, st);
     } else if (!idle && !testing && s.node >= 0) {
       trav_visit<kCount>(sc, s, stack, st);
     }
@@ -1027,7 +1045,7 @@ __device__ __forceinline__ void surface_at(const DevScene& sc, float3 o, float3 
       float3 radial = s.p - (base + axis * hh);
       if (uv) s.uv = axial_uv(axis, radial, hh, g1.w);
       if (kind == kQuadricCone) radial = radial + axis * ((g0.w - __ldg(Q + 2).w) / g1.w);
-      outward = normalize(radial);
+      outward = normalize_yx(radial);
     }
   }
   s.front = dot(d, outward) < 0.f;
@@ -1086,14 +1104,14 @@ __device__ __forceinline__ bool scatter_basic(const DevScene& sc, const DevMater
     case kMatLambertian: {
       float2 u = rng.next2();
       float3 dir = sample_cosine_hemisphere(s.n, u);
-      float c = fmaxf(0.f, dot(normalize(dir), s.n));
+      float c = fmaxf(0.f, dot(normalize_xy(dir), s.n));
       out.dir = dir;
       out.att = albedo_at(sc, m, s) * (1.0f / kPi);
       out.pdf = c / kPi;
       return true;
     }
     case kMatMetal: {
-      float3 r = reflect(normalize(din), s.n);
+      float3 r = reflect(normalize_xy(din), s.n);
       if (m.fuzz > 0.f) {
         float a = rng.next(), b = rng.next(), c = rng.next();
         r = r + sample_in_unit_sphere(f3(a, b, c)) * m.fuzz;
@@ -1105,7 +1123,7 @@ __device__ __forceinline__ bool scatter_basic(const DevScene& sc, const DevMater
     }
     case kMatDielectric: {
       float ratio = s.front ? 1.0f / m.ior : m.ior;
-      float3 ud = normalize(din);
+      float3 ud = normalize_xy(din);
       float ct = fminf(-dot(ud, s.n), 1.0f);
       float st = sqrtf(1.0f - ct * ct);
       bool cannot = ratio * st > 1.0f;
@@ -1487,7 +1505,7 @@ __device__ __forceinline__ int pick_light(const DevScene& sc, float u) {
 __device__ __forceinline__ float3 background(const DevScene& sc, float3 d) {
   float3 e = f3(0.f, 0.f, 0.f);
   if (!sc.has_infinite) return e;
-  float3 dn = normalize(d);
+  float3 dn = normalize_xy(d);
   for (int i = 0; i < sc.n_lights; i++) {
     DevLight L = sc.lights[i];
     if (L.kind == kLightUniformInfinite) e += L.a;
@@ -1499,7 +1517,8 @@ __device__ __forceinline__ float3 background(const DevScene& sc, float3 d) {
 // powerHeuristic (path_tracing.go:225-235)
 __device__ __forceinline__ float power_heuristic(float f, float g) {
   if (f == 0.f) return 0.f;
-  return (f * f) / (f * f + g * g);
+  const float ff = __fmul_rn(f, f);  // roundings spelled out, as normalize_xy
+  return __fdiv_rn(ff, __fmaf_rn(g, g, ff));
 }
 
 // ----------------------------------------------------------------- camera

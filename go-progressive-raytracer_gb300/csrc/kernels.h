@@ -152,6 +152,12 @@ void launch_hit_order(const DevScene& sc, const DevPaths& P, int cur, uint32_t c
 void launch_pt_shade(const DevScene& sc, const DevPaths& P, const ChunkDesc& ch, int cur, int bounce, int block,
                      int grid, cudaStream_t st);
 void launch_pt_shadow(const DevScene& sc, const DevPaths& P, int cur, int block, int grid, cudaStream_t st);
+// The whole chunk in one launch (radiance of every path to P.Lout), for chunks
+// of at most pt_paths_max paths; no counters of its own, error bits as the
+// wavefront.
+uint32_t pt_paths_max(const DevScene& sc, int sms);
+void launch_pt_paths(const DevScene& sc, const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int sms,
+                     cudaStream_t st);
 void launch_accumulate(const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int block, cudaStream_t st);
 
 // bidirectional path tracing (pkg/integrator/bdpt.go): subpaths per sample,

@@ -377,6 +377,168 @@ void launch_pt_shadow(const DevScene& sc, const DevPaths& P, int cur, int block,
   kernel<<<persistent_grid(sm_count_current(), 128), 128, 0, st>>>(sc, src, P.counters, P.stats);
 }
 
+// ----------------------------------------------------------------- whole paths
+// Small wavefronts in one launch: a lane takes a path from its camera ray to
+// its end (trace the shadow ray of the last level and the path's ray, shade,
+// repeat), keeping the state in registers that the queues of the wavefront
+// pass through memory.  The wavefront's 3-4 launches per bounce cost 30-45 us
+// each on any number of paths (a launch, and one ray's chain of dependent
+// loads on an almost empty chip), and a scene of depth 50 pays that 50 times;
+// here the chain of a path's bounces is all that is left.  It loses on large
+// wavefronts, where lanes of a warp part ways and 16 warps per SM hide less
+// than the traversal kernels' 32.
+// Results are those of the wavefront, bit for bit: the same tests in the same
+// order, the shading with its roundings spelled out, and the radiance added
+// up as the kernels of the wavefront add it (each unoccluded shadow ray, and
+// what the path itself gathered when it ends).
+// 8 blocks of 2 warps per SM at 128 registers (10: 3-10 % slower up to one
+// path per lane; 1-warp blocks the same); a finished lane takes the warp's
+// next path at once (waiting for 8 or 16 idle lanes: 2 and 14 % slower at
+// 160,000 paths).
+constexpr int kPathsBlock = 64, kPathsBlocksPerSm = 8;
+
+// Paths of a wavefront at most that k_pt_paths renders: where both forms took
+// the same time on GB300 (1 sample per pixel, depth 8; wavefront / whole paths
+// in us).  One-node scenes, bound by issue: Cornell box 346 / 248 at 147,456
+// paths, 413 / 394 at 262,144; textured shapes 352 / 184 and 382 / 350 at
+// 331,776; quadrics 323 / 310 and 351 / 461 at 262,144.  Trees, whose
+// wavefront waits longer: sphere scene 582 / 491 at 262,144, 770 / 939 at
+// 589,824; sphere grid 437 / 293 at 147,456, 540 / 558 at 331,776; 20,480
+// triangles 1340 / 825 at 262,144, 1748 / 1522 at 589,824.
+uint32_t pt_paths_max(const DevScene& sc, int sms) { return (uint32_t)sms * (one_node(sc) ? 1024u : 2048u); }
+
+template <bool kOneNode>
+__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
+    k_pt_paths(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch) {
+  const uint32_t n = ch.npix * ch.layers;
+  const int lane = threadIdx.x & 31;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t chunk = min(32u, (n + nw - 1) / nw);
+  const ErrSink err{P.counters + 3, nullptr, nullptr, nullptr};
+  uint64_t at = (uint64_t)w * chunk;
+  uint32_t cur = (uint32_t)min((uint64_t)n, at), end = (uint32_t)min((uint64_t)n, at + chunk);
+  bool more = cur < end;
+  bool alive = false, shadow = false;  // the lane's path goes on; its last level left a shadow ray
+  uint32_t path = 0;
+  int bounce = 0;
+  uint4 ids = make_uint4(0, 0, 0, 0);
+  float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f), d4 = o4, w4 = o4, sh_o = o4, sh_d = o4;
+  float3 thr = f3(0.f, 0.f, 0.f), L = thr, sh_c = thr;
+  float3 Lo = thr;  // what the wavefront holds at the path's origin index
+  TravEntry stack[kTraceStack];
+  for (;;) {
+    // new paths for the idle lanes
+    unsigned idle = __ballot_sync(0xffffffffu, !alive && !shadow);
+    if (more && idle) {
+      if (cur == end) {
+        at += (uint64_t)nw * chunk;
+        cur = (uint32_t)min((uint64_t)n, at);
+        end = (uint32_t)min((uint64_t)n, at + chunk);
+      }
+      if (cur == end) more = false;
+      uint32_t take = min((uint32_t)__popc(idle), end - cur);
+      uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+      if (!alive && !shadow && rank < take) {
+        path = cur + rank;
+        uint32_t layer = path / ch.npix, i = path - layer * ch.npix;
+        uint32_t pix = ch.pix_list ? ch.pix_list[ch.pix0 + i] : ch.pix0 + i;
+        uint32_t sample = film.count[pix] + layer;
+        int x = (int)(pix % (uint32_t)film.width), y = (int)(pix / (uint32_t)film.width);
+        Rng rng;
+        rng.init(ch.seed, pix, sample);
+        float2 lens = rng.next2();
+        float2 jit = rng.next2();
+        float3 o, d;
+        camera_ray(sc.cam, x, y, lens, jit, o, d);
+        o4 = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
+        d4 = make_float4(d.x, d.y, d.z, __int_as_float(sc.root));
+        ids = make_uint4(pix, sample, rng.pos, 0u);
+        w4 = make_float4(1.f, 1.f, 1.f, __uint_as_float(path));
+        thr = f3(1.f, 1.f, 1.f);
+        L = Lo = f3(0.f, 0.f, 0.f);
+        bounce = 0;
+        alive = true;
+      }
+      cur += take;
+      if (take) idle = 0;
+    }
+    if (idle == 0xffffffffu && !more) break;
+    // the shadow ray of the last step, then the path's ray
+    Hit hit{-1.f, kNoHit, 0.f, 0.f};
+    if (kOneNode) {
+      if (shadow) {
+        Hit h;
+        if (!trace_one_node<true, false>(sc, f3(sh_o), f3(sh_d), 0.001f, sh_o.w, __float_as_uint(sh_d.w), h))
+          Lo = f3(Lo.x + sh_c.x, Lo.y + sh_c.y, Lo.z + sh_c.z);
+      }
+      if (alive) trace_one_node<false, false>(sc, f3(o4), f3(d4), 0.001f, kInfF, __float_as_uint(o4.w), hit);
+    } else {
+      Trav s;
+      bool any = shadow, busy = shadow || alive;
+      if (busy) {
+        if (any) trav_init(s, f3(sh_o), f3(sh_d), 0.001f, sh_o.w, __float_as_uint(sh_d.w), sc.root, stack);
+        else trav_init(s, f3(o4), f3(d4), 0.001f, kInfF, __float_as_uint(o4.w), sc.root, stack);
+      }
+      for (;;) {
+        const bool testing = busy && s.testing();
+        const unsigned busy_mask = __ballot_sync(0xffffffffu, busy), test_mask = __ballot_sync(0xffffffffu, testing);
+        if (!busy_mask) break;
+        if (2 * __popc(test_mask) > __popc(busy_mask)) {
+          if (testing) trav_prim<false>(sc, s, any, stack, nullptr);
+        } else if (busy && !testing && s.node >= 0) {
+          trav_visit<false>(sc, s, stack, nullptr);
+        }
+        if (busy && s.done()) {
+          if (any) {
+            if (s.hit == kOverflowHit) err.report(path, kErrStackOverflow);
+            else if (s.hit == kNoHit) Lo = f3(Lo.x + sh_c.x, Lo.y + sh_c.y, Lo.z + sh_c.z);
+            any = false;
+            busy = alive;
+            if (busy) trav_init(s, f3(o4), f3(d4), 0.001f, kInfF, __float_as_uint(o4.w), sc.root, stack);
+          } else {
+            if (s.hit == kOverflowHit) {
+              err.report(path, kErrStackOverflow);
+              s.hit = kNoHit;
+            }
+            hit = s.result();
+            busy = false;
+          }
+        }
+      }
+    }
+    if (shadow && !alive) P.Lout[path] = make_float4(Lo.x, Lo.y, Lo.z, 0.f);
+    shadow = false;
+    if (alive) {
+      ShadeOut out;
+      shade_step(sc, o4, d4, make_float4(hit.t, __uint_as_float(hit.prim), hit.u, hit.v), ids, w4, thr, L, ch.seed,
+                 bounce, out, [&](float3 p, float3 dir, float dist, uint32_t prim, float3 c) {
+                   shadow = true;
+                   sh_o = make_float4(p.x, p.y, p.z, dist - 0.001f);
+                   sh_d = make_float4(dir.x, dir.y, dir.z, __uint_as_float(prim));
+                   sh_c = c;
+                 });
+      o4 = out.o;
+      d4 = out.d;
+      w4 = out.w;
+      thr = out.thr;
+      L = out.L;
+      ids = out.ids;
+      bounce++;
+      if (!out.cont) {
+        alive = false;
+        Lo = f3(Lo.x + L.x, Lo.y + L.y, Lo.z + L.z);
+        if (!shadow) P.Lout[path] = make_float4(Lo.x, Lo.y, Lo.z, 0.f);
+      }
+    }
+  }
+}
+
+void launch_pt_paths(const DevScene& sc, const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int sms,
+                     cudaStream_t st) {
+  auto kernel = one_node(sc) ? k_pt_paths<true> : k_pt_paths<false>;
+  kernel<<<sms * kPathsBlocksPerSm, kPathsBlock, 0, st>>>(sc, film, P, ch);
+}
+
 // ----------------------------------------------------------------- accumulate
 // PixelStats.AddSample (pkg/renderer/stats.go:41-47), in sample order per pixel
 __global__ void k_accumulate(DevFilm film, DevPaths P, ChunkDesc ch) {

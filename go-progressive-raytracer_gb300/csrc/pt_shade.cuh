@@ -19,27 +19,19 @@ struct ShadeOut {
 
 // One level of rayColorRecursive (pkg/integrator/path_tracing.go:35-104) with
 // CalculateDirectLighting (:116-157), CalculateIndirectLighting (:160-189)
-// and ApplyRussianRoulette (:193-220), for slot i of queue Q at depth index
-// `bounce` (= MaxDepth - depth).  The Russian-roulette draw happens first at
-// every level, as in the reference.  The shadow ray of next-event estimation
-// goes to P's shadow queue at once (its contribution, when unoccluded, is
-// added to the path's radiance at its origin index), so its state is not
-// held to the end of the step.
-__device__ __forceinline__ void shade_path(const DevScene& sc, const DevPaths& P, const PathBuf& Q,
-                                           const float4* hits, uint32_t i, uint64_t seed, int bounce, ShadeOut& out) {
+// and ApplyRussianRoulette (:193-220), for a path at depth index `bounce`
+// (= MaxDepth - depth) whose ray (o4, d4) met h4, with radiance weight w4 (and
+// origin index), roulette throughput thr and radiance L so far.  The
+// Russian-roulette draw happens first at every level, as in the reference.
+// The shadow ray of next-event estimation goes to
+// `shadow(point, direction, light distance, primitive left, contribution)` as
+// soon as it is known, so its state is not held to the end of the step.
+template <class Shadow>
+__device__ __forceinline__ void shade_step(const DevScene& sc, float4 o4, float4 d4, float4 h4, uint4 ids, float4 w4,
+                                           float3 thr, float3 L, uint64_t seed, int bounce, ShadeOut& out,
+                                           Shadow shadow) {
   out.cont = false;
-  float4 o4 = Q.ray_o[i], d4 = Q.ray_d[i], h4 = hits[i];
-  uint4 ids = Q.ids[i];
   float3 d = f3(d4);
-  // at bounce 0 the path state raygen implies (not stored): weight 1, origin
-  // index = the slot, roulette throughput 1, radiance 0
-  float4 w4 = make_float4(1.f, 1.f, 1.f, __uint_as_float(i));
-  float3 thr = f3(1.f, 1.f, 1.f), L = f3(0.f, 0.f, 0.f);
-  if (bounce > 0) {
-    w4 = Q.weight[i];
-    thr = f3(Q.thr[i]);
-    L = f3(Q.L[i]);
-  }
   float3 W = f3(w4);
   out.o = o4;
   out.d = d4;
@@ -49,7 +41,7 @@ __device__ __forceinline__ void shade_path(const DevScene& sc, const DevPaths& P
   float u = rng.next();
   bool dead = false;
   if (bounce >= sc.rr_min_bounces) {
-    float surv = fminf(0.95f, fmaxf(0.5f, luminance(thr)));
+    float surv = fminf(0.95f, fmaxf(0.5f, luminance_xy(thr)));
     if (u > surv) dead = true;
     else W *= 1.0f / surv;
   }
@@ -86,18 +78,12 @@ __device__ __forceinline__ void shade_path(const DevScene& sc, const DevPaths& P
                 float w = power_heuristic(ls.pdf, mp);
                 float3 f = brdf(sc, m, d, ls.dir, s, true);
                 float3 c = W * (f * ls.emission) * (cosine * w / ls.pdf);
-                if (!is_zero(c)) {  // one warp-aggregated append among the lanes here
-                  uint32_t ss = warp_append(&P.counters[2], true);
-                  P.sh_o[ss] = make_float4(s.p.x, s.p.y, s.p.z, ls.dist - 0.001f);
-                  P.sh_d[ss] = make_float4(ls.dir.x, ls.dir.y, ls.dir.z, __uint_as_float(prim));
-                  P.sh_c[ss] = make_float4(c.x, c.y, c.z, w4.w);  // w4.w: the origin index
-                  if (P.sh_root) P.sh_root[ss] = __float_as_int(d4.w);
-                }
+                if (!is_zero(c)) shadow(s.p, ls.dir, ls.dist, prim, c);
               }
             }
           }
           // CalculateIndirectLighting
-          float3 sd = normalize(sc_.dir);
+          float3 sd = normalize_yx(sc_.dir);
           float cosine = dot(sd, s.n);
           if (cosine > 0.f) {
             float lp = total_light_pdf(sc, s.p, s.n, sd);
@@ -119,6 +105,33 @@ __device__ __forceinline__ void shade_path(const DevScene& sc, const DevPaths& P
   out.w = make_float4(W.x, W.y, W.z, w4.w);
   out.thr = thr;
   out.ids = make_uint4(ids.x, ids.y, rng.pos, ids.w);
+}
+
+// shade_step for slot i of queue Q.  The shadow ray goes to P's shadow queue
+// (its contribution, when unoccluded, is added to the path's radiance at its
+// origin index).
+__device__ __forceinline__ void shade_path(const DevScene& sc, const DevPaths& P, const PathBuf& Q,
+                                           const float4* hits, uint32_t i, uint64_t seed, int bounce, ShadeOut& out) {
+  float4 o4 = Q.ray_o[i], d4 = Q.ray_d[i], h4 = hits[i];
+  uint4 ids = Q.ids[i];
+  // at bounce 0 the path state raygen implies (not stored): weight 1, origin
+  // index = the slot, roulette throughput 1, radiance 0
+  float4 w4 = make_float4(1.f, 1.f, 1.f, __uint_as_float(i));
+  float3 thr = f3(1.f, 1.f, 1.f), L = f3(0.f, 0.f, 0.f);
+  if (bounce > 0) {
+    w4 = Q.weight[i];
+    thr = f3(Q.thr[i]);
+    L = f3(Q.L[i]);
+  }
+  shade_step(sc, o4, d4, h4, ids, w4, thr, L, seed, bounce, out,
+             [&](float3 p, float3 dir, float dist, uint32_t prim, float3 c) {
+               // one warp-aggregated append among the lanes here
+               uint32_t ss = warp_append(&P.counters[2], true);
+               P.sh_o[ss] = make_float4(p.x, p.y, p.z, dist - 0.001f);
+               P.sh_d[ss] = make_float4(dir.x, dir.y, dir.z, __uint_as_float(prim));
+               P.sh_c[ss] = make_float4(c.x, c.y, c.z, w4.w);  // w4.w: the origin index
+               if (P.sh_root) P.sh_root[ss] = __float_as_int(d4.w);
+             });
 }
 
 // Brings the shading inputs of slot i of queue Q (ray, hit, ids and, after
