@@ -460,16 +460,18 @@ struct TraceStats {
 // 10-17 of 32 lanes per instruction with the boxes and leaves of a node in one
 // loop), on a handful of rays by the chain of loads of a node visit.  So a
 // visit is four 256-bit loads issued together and four box tests without a
-// branch (packed multiply-adds: two planes per instruction), and a leaf test
-// is a step of its own: a warp takes whichever step more of its lanes wait
-// for.  The leaves of a visited node come before any node below it, in slot
-// order, each checked against the hit so far when its turn comes: the
-// primitives are tested in the order, and culled by the comparisons, of a
-// loop that intersects each leaf as it meets it, so ties between equal
-// distances fall the same way.  Measured on GB300, before -> after: 2^24 rays
-// on 1.3 M triangles (closest hit) 23.0 -> 11.2 ms, 300,007 rays (any hit) on
-// 81,920 triangles 268 -> 186 us, the 1024^2 x 16 frame of the 1.3 M
-// triangles 28.7 -> 22.8 ms, a 128^2 x 1 pass of a sphere scene 907 -> 467 us.
+// branch (packed multiply-adds: two planes per instruction; three-input
+// minima and maxima, as the ALU is now the busiest pipe, at 65-75 %), and a
+// primitive test is a step of its own, taken when enough lanes wait for it.
+// The leaves of a visited node come before any node below it, in slot order,
+// each checked against the hit so far when its turn comes: the primitives are
+// tested in the order, and culled by the comparisons, of a loop that
+// intersects each leaf as it meets it, so ties between equal distances fall
+// the same way.  Measured on GB300, before -> after: 2^24 rays on 1.3 M
+// triangles (closest hit) 23.0 -> 10.1 ms, 300,007 rays (any hit) on 81,920
+// triangles 268 -> 167 us, the 1024^2 x 16 frame of the 1.3 M triangles
+// 28.7 -> 21.0 ms.
+
 // State of one ray's traversal; `skip` is the primitive the ray leaves from:
 // a ray cannot re-enter the plane of the triangle or quad it starts on, and
 // for the sphere it starts on hits closer than 2e-4 x radius are rounding
@@ -562,14 +564,24 @@ __device__ __forceinline__ float2 slab(unsigned long long planes, float inv, flo
   asm("mov.b64 {%0, %1}, %2;" : "=f"(t.x), "=f"(t.y) : "l"(r));
   return t;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 // Entry and exit distance of the ray in a child box, before the ray's own
 // far end.  Rounding is monotonic, so the nearer plane of each axis is the
 // smaller distance.
 __device__ __forceinline__ void child_span(float3 inv, float3 nood, float tmin, const ChildRec& c, float& tn,
                                            float& tf) {
   const float2 x = slab(c.x, inv.x, nood.x), y = slab(c.y, inv.y, nood.y), z = slab(c.z, inv.z, nood.z);
-  tn = fmaxf(fmaxf(fminf(x.x, x.y), fminf(y.x, y.y)), fmaxf(fminf(z.x, z.y), tmin));
-  tf = fminf(fminf(fmaxf(x.x, x.y), fmaxf(y.x, y.y)), fmaxf(z.x, z.y));
+  tn = max3(fminf(x.x, x.y), fminf(y.x, y.y), fmaxf(fminf(z.x, z.y), tmin));
+  tf = min3(fmaxf(x.x, x.y), fmaxf(y.x, y.y), fmaxf(z.x, z.y));
 }
 
 // Moves the ray to the nearest entry left on its stack, leaving out those
@@ -641,6 +653,16 @@ __device__ __forceinline__ bool hit_prim(const DevScene& sc, int type, int p, fl
   return hit_quadric(o, d, Q, lo, best, t, u);
 }
 
+// The first leaf of the node just visited, whose box was tested there.
+__device__ __forceinline__ void trav_first_leaf(const DevScene& sc, Trav& s) {
+  const int i = __ffs(s.leaves) - 1;
+  s.leaves &= s.leaves - 1;
+  const int2 rm = __ldg(reinterpret_cast<const int2*>(sc.nodes + (size_t)s.lnode * 8 + 2 * i + 1) + 1);
+  s.prim = rm.x;
+  s.end = rm.x + (rm.y & kLeafCountMask);
+  s.type = (rm.y >> kLeafTypeShift) & 3;
+}
+
 // Tests the ray against primitive `prim` of its leaf and moves on: to the
 // leaf's next primitive, the node's next leaf or the ray's next node.
 template <bool kCount>
@@ -689,10 +711,7 @@ __device__ __forceinline__ void trav_visit(const DevScene& sc, Trav& s, TravEntr
     const bool hit = used && !(tn[i] > fminf(tf, s.best));
     const bool leaf = c[i].meta() != 0;
     if (hit && leaf) leaves |= 1u << i;
-    if (!hit || leaf) {
-      tn[i] = kInfF;
-      ref[i] = -1;
-    }
+    if (!hit || leaf) tn[i] = kInfF;
   }
   // nearest first: an odd-even transposition network, stable as only a
   // strictly greater neighbour changes places
@@ -711,19 +730,21 @@ __device__ __forceinline__ void trav_visit(const DevScene& sc, Trav& s, TravEntr
   order(0, 1);
   order(2, 3);
   order(1, 2);
-  if (s.sp + (ref[1] >= 0) + (ref[2] >= 0) + (ref[3] >= 0) > kTraceStack) {
+  const bool p1 = tn[1] < kInfF, p2 = tn[2] < kInfF, p3 = tn[3] < kInfF;
+  if (s.sp + p1 + p2 + p3 > kTraceStack) {
     s.node = -1;
     s.hit = kOverflowHit;
     return;
   }
-  if (ref[3] >= 0) stack[s.sp++] = TravEntry{ref[3], tn[3]};
-  if (ref[2] >= 0) stack[s.sp++] = TravEntry{ref[2], tn[2]};
-  if (ref[1] >= 0) stack[s.sp++] = TravEntry{ref[1], tn[1]};
-  s.leaves = leaves;
+  if (p3) stack[s.sp++] = TravEntry{ref[3], tn[3]};
+  if (p2) stack[s.sp++] = TravEntry{ref[2], tn[2]};
+  if (p1) stack[s.sp++] = TravEntry{ref[1], tn[1]};
   s.lnode = s.node;
-  s.node = ref[0] >= 0 ? ref[0] : kPopNext;
+  s.node = tn[0] < kInfF ? ref[0] : kPopNext;
   s.node_t = tn[0];
-  if (leaves || ref[0] < 0) trav_next_leaf(sc, s, stack);
+  s.leaves = leaves;
+  if (leaves) trav_first_leaf(sc, s);
+  else if (s.node == kPopNext) trav_pop(s, stack);
 }
 
 // Whole traversal of one ray from BVH node `root`.  A stack overflow returns
@@ -824,9 +845,17 @@ __device__ __forceinline__ void trace_batch_one_node(const DevScene& sc, Source&
   }
 }
 
+// The step of a warp whose lanes `busy` are on a ray and `testing` wait for a
+// primitive test: a test costs about a third of a node visit, so it is taken
+// once more than a third of the lanes wait for it (1/2, 1/4, 1/6 and 2/3:
+// 21.3, 21.1, 21.5 and 22.5 against 21.0 ms for the frame of 1.3 M triangles;
+// 64.3, 64.5, 64.9 and 65.3 against 64.3 ms for 32 sphere scenes).
+__device__ __forceinline__ bool trav_test_now(unsigned testing, unsigned busy) {
+  return 3 * __popc(testing) > __popc(busy);
+}
+
 // Persistent traversal of a batch of rays: every warp loops until its work
-// is exhausted, one step per iteration (node visits or primitive tests,
-// whichever more lanes wait for), and lanes whose ray finished take new rays
+// is exhausted, one step per iteration (trav_test_now), and lanes whose ray finished take new rays
 // once at least 16 lanes are idle (8, 12 and 20 measured within 2 %: 69.9,
 // 68.6 and 68.5 against 68.3 ms on the sphere batch, 22.7, 22.8 and 23.1
 // against 22.8 ms on 1.3 M triangles), so warps stay full instead of waiting
@@ -900,8 +929,7 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
       continue;
     }
     if (idle_mask == 0xffffffffu) break;
-    // the step that more lanes wait for
-    if (2 * __popc(test_mask) > 32 - __popc(idle_mask)) {
+    if (trav_test_now(test_mask, ~idle_mask)) {
       if (testing) trav_prim<kCount>(sc, s, kAnyHit, stack, st);
     } else if (!idle && !testing && s.node >= 0) {
       trav_visit<kCount>(sc, s, stack, st);

@@ -483,7 +483,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
         const bool testing = busy && s.testing();
         const unsigned busy_mask = __ballot_sync(0xffffffffu, busy), test_mask = __ballot_sync(0xffffffffu, testing);
         if (!busy_mask) break;
-        if (2 * __popc(test_mask) > __popc(busy_mask)) {
+        if (trav_test_now(test_mask, busy_mask)) {
           if (testing) trav_prim<false>(sc, s, any, stack, nullptr);
         } else if (busy && !testing && s.node >= 0) {
           trav_visit<false>(sc, s, stack, nullptr);
