@@ -247,6 +247,27 @@ int upload_geometry(gprt_ctx* ctx, gprt_scene* s) {
   return rc;
 }
 
+// Sets dev.one when the scene's BVH is one node of at most kOneNodePrims
+// primitives (its records copied from the host arrays in leaf order).
+void fill_one_node(gprt_scene* s) {
+  const HostScene& h = s->host;
+  DevScene& d = s->dev;
+  d.one = nullptr;
+  if (d.n_nodes != 1 || d.n_prims > (uint32_t)kOneNodePrims) return;
+  OneNode& g = s->one;
+  std::memcpy(g.child, h.nodes.data(), sizeof(g.child));
+  const std::vector<float4>* rec[4] = {&h.tris, &h.quads, &h.spheres, &h.quadrics};
+  const uint32_t base[4] = {0, d.quad_base, d.sphere_base, d.quadric_base};
+  int n = 0;
+  for (int t = 0; t < 4; t++) {
+    g.base[t] = base[t];
+    g.off[t] = n;
+    std::copy(rec[t]->begin(), rec[t]->end(), g.rec + n);
+    n += (int)rec[t]->size();
+  }
+  d.one = &g;
+}
+
 // Uploads materials, lights and textures, sets the scalar fields of s->dev
 // and waits for the copies; frees the scene's buffers on failure.
 int upload_rest(gprt_ctx* ctx, gprt_scene* s) {
@@ -283,6 +304,7 @@ int upload_rest(gprt_ctx* ctx, gprt_scene* s) {
     free_all(s->buffers);
     return fail(ctx, GPRT_E_INVALID, "the scene has too many primitives for 32-bit primitive ids");
   }
+  fill_one_node(s);
   d.has_infinite = h.has_infinite;
   d.has_specular = 0;
   for (const DevMaterial& m : h.materials) d.has_specular |= m.kind == kMatMetal || m.kind == kMatDielectric;

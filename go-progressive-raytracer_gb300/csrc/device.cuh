@@ -324,9 +324,10 @@ __device__ __forceinline__ float axial_height(float3 o, float3 d, float t, float
 // FP32 roots accurate when the ray starts far away; the candidate order and
 // the height / nappe checks are the reference's.  `part` tells the surface
 // code which piece was hit: 0 body (or disc), 1 base cap, 2 top cap.
-__device__ __forceinline__ bool hit_quadric(float3 o, float3 d, const float4* Q, float tmin, float tmax, float& t,
-                                            float& part) {
-  float4 g0 = __ldg(Q), g1 = __ldg(Q + 1), g4 = __ldg(Q + 4);
+template <class Load>
+__device__ __forceinline__ bool hit_quadric(float3 o, float3 d, const float4* Q, Load ld, float tmin, float tmax,
+                                            float& t, float& part) {
+  float4 g0 = ld(Q), g1 = ld(Q + 1), g4 = ld(Q + 4);
   int kind = __float_as_int(g4.x);
   float3 p0 = f3(g0), axis = f3(g1);
   if (kind == kQuadricDisc) {
@@ -334,7 +335,7 @@ __device__ __forceinline__ bool hit_quadric(float3 o, float3 d, const float4* Q,
     part = 0.f;
     return true;
   }
-  float4 g2 = __ldg(Q + 2);
+  float4 g2 = ld(Q + 2);
   float height = g1.w, best = tmax;
   bool any = false;
   if (kind == kQuadricCylinder) {
@@ -389,7 +390,7 @@ __device__ __forceinline__ bool hit_quadric(float3 o, float3 d, const float4* Q,
       }
     }
   } else {
-    float4 g3 = __ldg(Q + 3);
+    float4 g3 = ld(Q + 3);
     float3 apex = f3(g3);
     float kk = __fadd_rn(1.f, g3.w);  // 1 + tan^2
     float3 CO = sub_rn(o, apex);
@@ -577,11 +578,18 @@ __device__ __forceinline__ float min3(float a, float b, float c) {
 // Entry and exit distance of the ray in a child box, before the ray's own
 // far end.  Rounding is monotonic, so the nearer plane of each axis is the
 // smaller distance.
-__device__ __forceinline__ void child_span(float3 inv, float3 nood, float tmin, const ChildRec& c, float& tn,
-                                           float& tf) {
-  const float2 x = slab(c.x, inv.x, nood.x), y = slab(c.y, inv.y, nood.y), z = slab(c.z, inv.z, nood.z);
+__device__ __forceinline__ void span_of(float2 x, float2 y, float2 z, float tmin, float& tn, float& tf) {
   tn = max3(fminf(x.x, x.y), fminf(y.x, y.y), fmaxf(fminf(z.x, z.y), tmin));
   tf = min3(fmaxf(x.x, x.y), fmaxf(y.x, y.y), fmaxf(z.x, z.y));
+}
+__device__ __forceinline__ void child_span(float3 inv, float3 nood, float tmin, const ChildRec& c, float& tn,
+                                           float& tf) {
+  span_of(slab(c.x, inv.x, nood.x), slab(c.y, inv.y, nood.y), slab(c.z, inv.z, nood.z), tmin, tn, tf);
+}
+__device__ __forceinline__ void child_span(float3 inv, float3 nood, float tmin, const NodeChild& c, float& tn,
+                                           float& tf) {
+  auto axis = [](const float* p, float k, float c0) { return make_float2(__fmaf_rn(p[0], k, c0), __fmaf_rn(p[1], k, c0)); };
+  span_of(axis(c.x, inv.x, nood.x), axis(c.y, inv.y, nood.y), axis(c.z, inv.z, nood.z), tmin, tn, tf);
 }
 
 // Moves the ray to the nearest entry left on its stack, leaving out those
@@ -616,41 +624,55 @@ __device__ __forceinline__ void trav_next_leaf(const DevScene& sc, Trav& s, cons
   if (s.node == kPopNext || s.node_t > s.best) trav_pop(s, stack);
 }
 
-// The ray (o, d) against primitive p of type `type` (its global id in gid):
-// a hit with t in [tmin, best].
-__device__ __forceinline__ bool hit_prim(const DevScene& sc, int type, int p, float3 o, float3 d, float tmin, float best,
-                                         uint32_t skip, uint32_t& gid, float& t, float& u, float& v) {
+// The ray (o, d) against the record R (read through `ld`) of a primitive of
+// type `type` with global id gid: a hit with t in [tmin, best].
+template <class Load>
+__device__ __forceinline__ bool hit_record(int type, const float4* R, Load ld, float3 o, float3 d, float tmin, float best,
+                                           uint32_t skip, uint32_t gid, float& t, float& u, float& v) {
   u = v = 0.f;
   if (type == kPrimTriangle) {
-    gid = (uint32_t)p;
     if (gid == skip) return false;
-    const float4* T = sc.tris + (size_t)p * 3;
-    return hit_triangle(o, d, __ldg(T), __ldg(T + 1), __ldg(T + 2), tmin, best, t, u, v);
+    return hit_triangle(o, d, ld(R), ld(R + 1), ld(R + 2), tmin, best, t, u, v);
   }
   if (type == kPrimQuad) {
-    gid = sc.quad_base + (uint32_t)p;
     if (gid == skip) return false;
-    const float4* Q = sc.quads + (size_t)p * 5;
-    float4 qq[5] = {__ldg(Q), __ldg(Q + 1), __ldg(Q + 2), __ldg(Q + 3), __ldg(Q + 4)};
+    float4 qq[5] = {ld(R), ld(R + 1), ld(R + 2), ld(R + 3), ld(R + 4)};
     return hit_quad(o, d, qq, tmin, best, t, u, v);
   }
   if (type == kPrimSphere) {
-    gid = sc.sphere_base + (uint32_t)p;
-    float4 S = __ldg(sc.spheres + (size_t)p * 2);
+    float4 S = ld(R);
     float lo = gid == skip ? fmaxf(tmin, 2e-4f * fabsf(S.w)) : tmin;
     return hit_sphere(o, d, S, lo, best, t);
   }
   // a ray leaving a quadric may hit it again (the other side of a
   // cylinder); hits closer than 2e-4 x radius are its own surface
-  gid = sc.quadric_base + (uint32_t)p;
-  const float4* Q = sc.quadrics + (size_t)p * 5;
   float lo = tmin;
   if (gid == skip) {
-    float4 g0 = __ldg(Q);
-    if (__float_as_int(__ldg(Q + 4).x) == kQuadricDisc) return false;  // planar
+    float4 g0 = ld(R);
+    if (__float_as_int(ld(R + 4).x) == kQuadricDisc) return false;  // planar
     lo = fmaxf(tmin, 2e-4f * g0.w);
   }
-  return hit_quadric(o, d, Q, lo, best, t, u);
+  return hit_quadric(o, d, R, ld, lo, best, t, u);
+}
+
+// The ray against primitive p of type `type` of the scene.
+__device__ __forceinline__ bool hit_prim(const DevScene& sc, int type, int p, float3 o, float3 d, float tmin, float best,
+                                         uint32_t skip, uint32_t& gid, float& t, float& u, float& v) {
+  auto ld = [](const float4* x) { return __ldg(x); };
+  if (type == kPrimTriangle) {
+    gid = (uint32_t)p;
+    return hit_record(kPrimTriangle, sc.tris + (size_t)p * 3, ld, o, d, tmin, best, skip, gid, t, u, v);
+  }
+  if (type == kPrimQuad) {
+    gid = sc.quad_base + (uint32_t)p;
+    return hit_record(kPrimQuad, sc.quads + (size_t)p * 5, ld, o, d, tmin, best, skip, gid, t, u, v);
+  }
+  if (type == kPrimSphere) {
+    gid = sc.sphere_base + (uint32_t)p;
+    return hit_record(kPrimSphere, sc.spheres + (size_t)p * 2, ld, o, d, tmin, best, skip, gid, t, u, v);
+  }
+  gid = sc.quadric_base + (uint32_t)p;
+  return hit_record(kPrimQuadric, sc.quadrics + (size_t)p * 5, ld, o, d, tmin, best, skip, gid, t, u, v);
 }
 
 // The first leaf of the node just visited, whose box was tested there.
@@ -767,51 +789,69 @@ __device__ __forceinline__ bool trace_from(const DevScene& sc, int root, float3 
   return s.hit != kNoHit;
 }
 
-// A scene whose BVH is a single node holds only leaves (the host builder's
-// layout of at most 32 primitives, and anything smaller).
-__host__ __device__ __forceinline__ bool one_node(const DevScene& sc) { return sc.n_nodes == 1; }
+__host__ __device__ __forceinline__ bool one_node(const DevScene& sc) { return sc.one != nullptr; }
+
+// What a kernel takes beside the scene: the one node, or nothing.
+struct NoGeom {};
+template <bool kOneNode>
+struct GeomOf {
+  using type = NoGeom;
+};
+template <>
+struct GeomOf<true> {
+  using type = OneNode;
+};
+template <bool kOneNode>
+using Geom = typename GeomOf<kOneNode>::type;
 
 // Whole traversal of one ray of a one-node scene: its leaves in slot order,
 // each primitive by every lane of the warp at once, so that the loop, the
 // type and the record's address are the same for all lanes; a lane whose ray
-// misses the leaf's box sits it out.  The tests and their order are those of
-// trav_visit / trav_prim, whose step per primitive costs more here than the
-// lanes it fills (Cornell box, 18 quads, 400^2 x 64: 10.7 ms a frame stepped,
-// 7.8 ms in this loop).
-template <bool kAnyHit, bool kCount>
-__device__ __forceinline__ bool trace_one_node(const DevScene& sc, float3 o, float3 d, float tmin, float tmax,
-                                               uint32_t skip, Hit& hit, TraceStats* st = nullptr) {
+// misses the leaf's box (or without a ray: !live) sits it out.  The tests and
+// their order are those of trav_visit / trav_prim, whose step per primitive
+// costs more here than the lanes it fills (Cornell box, 18 quads, 400^2 x 64:
+// 10.7 ms a frame stepped, 7.8 ms in this loop).  The records come from the
+// launch's constant bank: as 128-bit global loads they kept the load pipe at
+// 65-71 % (every one returns 512 bytes a warp, though all lanes read the same
+// 16); now it is at 2-6 % and issue bounds the loop (IPC 2.6-2.9).  Cornell
+// box 7.83 -> 7.58 ms, Cornell boxes BDPT 512^2 x 64 90.8 -> 85.9 ms,
+// textured shapes 517x290 x 3 605 -> 559 us.
+template <bool kCount>
+__device__ __forceinline__ bool trace_one_node(const OneNode& g, bool live, bool any_hit, float3 o, float3 d, float tmin,
+                                               float tmax, uint32_t skip, Hit& hit, TraceStats* st = nullptr) {
   const float3 inv = ray_inverse(d);
   const float3 nood = -(o * inv);
+  auto ld = [](const float4* x) { return *x; };
   float best = tmax, hu = 0.f, hv = 0.f;
   uint32_t prim = kNoHit;
-  if (kCount) st->nodes++;
+  if (kCount && live) st->nodes++;
   for (int i = 0; i < 4; i++) {
-    const ChildRec c = ldg_child(sc.nodes + 2 * i);
-    if (c.ref() == kEmptyChild) break;
-    if (kCount) st->boxes++;
+    const int ref = g.child[i].ref, meta = g.child[i].meta;
+    if (ref == kEmptyChild) break;
+    if (kCount && live) st->boxes++;
     float tn, tf;
-    child_span(inv, nood, tmin, c, tn, tf);
-    const bool in = !(tn > fminf(tf, best));
-    const int type = (c.meta() >> kLeafTypeShift) & 3, end = c.ref() + (c.meta() & kLeafCountMask);
-    auto leaf = [&](int kind) {
-      for (int p = c.ref(); p < end; p++) {
-        if (!in || (kAnyHit && prim != kNoHit)) continue;
-        uint32_t gid;
+    child_span(inv, nood, tmin, g.child[i], tn, tf);
+    bool in = live && !(tn > fminf(tf, best)) && !(any_hit && prim != kNoHit);
+    auto leaf = [&](int type, int stride) {
+      const float4* R = g.rec + g.off[type] + ref * stride;
+      uint32_t gid = g.base[type] + (uint32_t)ref;
+      for (int k = meta & kLeafCountMask; k > 0; k--, R += stride, gid++) {
         float t, u, v;
-        if (kCount) st->prims++;
-        if (hit_prim(sc, kind, p, o, d, tmin, best, skip, gid, t, u, v)) {
+        if (kCount && in) st->prims++;
+        if (in && hit_record(type, R, ld, o, d, tmin, best, skip, gid, t, u, v)) {
           best = t;
           hu = u;
           hv = v;
           prim = gid;
+          in = !any_hit;
         }
       }
     };
-    if (type == kPrimTriangle) leaf(kPrimTriangle);
-    else if (type == kPrimQuad) leaf(kPrimQuad);
-    else if (type == kPrimSphere) leaf(kPrimSphere);
-    else leaf(kPrimQuadric);
+    const int type = (meta >> kLeafTypeShift) & 3;
+    if (type == kPrimTriangle) leaf(kPrimTriangle, 3);
+    else if (type == kPrimQuad) leaf(kPrimQuad, 5);
+    else if (type == kPrimSphere) leaf(kPrimSphere, 2);
+    else leaf(kPrimQuadric, 5);
   }
   hit = Hit{prim != kNoHit ? best : -1.f, prim, hu, hv};
   return prim != kNoHit;
@@ -819,29 +859,32 @@ __device__ __forceinline__ bool trace_one_node(const DevScene& sc, float3 o, flo
 
 // Whole traversal of one ray of the scene (the BDPT strategy kernels), in the
 // form for one_node(sc): a kernel holds one form, as both together spill.
-template <bool kAnyHit, bool kCount, bool kOneNode>
-__device__ __forceinline__ bool trace(const DevScene& sc, float3 o, float3 d, float tmin, float tmax, uint32_t skip,
-                                      Hit& hit, int* err, TraceStats* st = nullptr) {
-  if (kOneNode) return trace_one_node<kAnyHit, kCount>(sc, o, d, tmin, tmax, skip, hit, st);
-  return trace_from<kAnyHit, kCount>(sc, sc.root, o, d, tmin, tmax, skip, hit, err, st);
+template <bool kAnyHit, bool kOneNode>
+__device__ __forceinline__ bool trace(const DevScene& sc, const Geom<kOneNode>& g, float3 o, float3 d, float tmin,
+                                      float tmax, uint32_t skip, Hit& hit, int* err) {
+  if constexpr (kOneNode) return trace_one_node<false>(g, true, kAnyHit, o, d, tmin, tmax, skip, hit);
+  else return trace_from<kAnyHit, false>(sc, sc.root, o, d, tmin, tmax, skip, hit, err);
 }
 
 // A batch of rays of a one-node scene, one ray per thread (every ray costs
 // the same, so there is nothing to refill).
 template <bool kAnyHit, bool kCount, class Source>
-__device__ __forceinline__ void trace_batch_one_node(const DevScene& sc, Source& src, TraceStats* st,
-                                                     uint32_t* traced) {
+__device__ __forceinline__ void trace_batch_one_node(const OneNode& g, Source& src, TraceStats* st, uint32_t* traced) {
   const uint32_t n = src.count();
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    float3 o, d;
-    float tmin, tmax;
-    uint32_t skip;
+  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
+    const uint32_t i = base + threadIdx.x;
+    const bool live = i < n;
+    float3 o = f3(0.f, 0.f, 0.f), d = f3(0.f, 0.f, 1.f);
+    float tmin = 0.f, tmax = 0.f;
+    uint32_t skip = kNoHit;
     int root;
-    src.load(i, o, d, tmin, tmax, skip, root);
+    if (live) src.load(i, o, d, tmin, tmax, skip, root);
     Hit h;
-    trace_one_node<kAnyHit, kCount>(sc, o, d, tmin, tmax, skip, h, st);
-    src.store(i, h);
-    if (kCount) (*traced)++;
+    trace_one_node<kCount>(g, live, kAnyHit, o, d, tmin, tmax, skip, h, st);
+    if (live) {
+      src.store(i, h);
+      if (kCount) (*traced)++;
+    }
   }
 }
 
@@ -1493,7 +1536,7 @@ __device__ __forceinline__ float light_pdf(const DevScene& sc, const DevLight& L
   if (L.kind == kLightDisc || L.kind == kLightDiscSpot) {  // disc_light.go:78-100
     const float4* Q = sc.quadrics + (size_t)L.prim * 5;
     float t, part;
-    if (!hit_quadric(p, dir, Q, 0.001f, kInfF, t, part)) return 0.f;
+    if (!hit_quadric(p, dir, Q, [](const float4* x) { return __ldg(x); }, 0.001f, kInfF, t, part)) return 0.f;
     float ct = fabsf(dot(f3(__ldg(Q + 1)), -dir));
     if (ct < 1e-6f) return 0.f;
     return (1.0f / L.area) * t * t / ct;

@@ -39,6 +39,7 @@ struct gprt_scene {
   gprt_ctx* ctx = nullptr;
   HostScene host;
   DevScene dev{};
+  OneNode one{};  // what dev.one points to
   std::vector<void*> buffers;
   size_t bytes = 0;
   int* d_err = nullptr;

@@ -333,9 +333,10 @@ __device__ __forceinline__ float light_origin_pdf(const DevScene& sc, const BVer
 
 // Any-hit test of a connection / shadow ray (one call site for all strategies).
 template <bool kOneNode>
-__device__ __forceinline__ bool occluded(const DevScene& sc, float3 o, float3 d, float tmax, uint32_t skip, int* err) {
+__device__ __forceinline__ bool occluded(const DevScene& sc, const Geom<kOneNode>& geo, float3 o, float3 d, float tmax,
+                                         uint32_t skip, int* err) {
   Hit hh;
-  return trace<true, false, kOneNode>(sc, o, d, 0.001f, tmax, skip, hh, err);
+  return trace<true, kOneNode>(sc, geo, o, d, 0.001f, tmax, skip, hh, err);
 }
 
 // ---------------------------------------------------------------- vertex store
@@ -626,8 +627,8 @@ __device__ __forceinline__ uint32_t draws_before(int s, int t, uint2 m) {
 // evaluateBDPTStrategy (bdpt.go:294-561) for strategy (s, t) of sample i;
 // returns the weighted contribution to the sample (t = 1 splats instead).
 template <int CLS, bool kOneNode>
-__device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const DevFilm& film, const DevBdpt& B, uint32_t i,
-                                             int s, int t, Rng& rs, int* err) {
+__device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<kOneNode>& geo, const DevFilm& film,
+                                                const DevBdpt& B, uint32_t i, int s, int t, Rng& rs, int* err) {
   const float3 zero = f3(0.f, 0.f, 0.f);
   SubpathRef C{&B, i, 0}, Lp{&B, i, B.maxv};
   float3 Lc = zero;
@@ -740,7 +741,7 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const DevFil
     rskip = cv.prim;
     Lc = c;
   }
-  if (test && occluded<kOneNode>(sc, ro, rd, rt, rskip, err)) return zero;
+  if (test && occluded<kOneNode>(sc, geo, ro, rd, rt, rskip, err)) return zero;
   if (splat) {
     // MapRayToPixel, then the light pdf of the camera vertex (bdpt.go:440-470)
     float3 dir = sampled.wi;
@@ -837,9 +838,10 @@ struct BdptSource {
 };
 
 template <bool kOneNode>
-__global__ void __launch_bounds__(128, kTravBlocks) k_bdpt_trace(DevScene sc, BdptSource src, uint32_t* counters, int cur) {
+__global__ void __launch_bounds__(128, kTravBlocks) 
+    k_bdpt_trace(DevScene sc, BdptSource src, uint32_t* counters, int cur, const __grid_constant__ Geom<kOneNode> geo) {
   if (blockIdx.x == 0 && threadIdx.x == 0) counters[cur ^ 1] = 0;  // the next queue starts empty
-  if (kOneNode) trace_batch_one_node<false, false>(sc, src, nullptr, nullptr);
+  if constexpr (kOneNode) trace_batch_one_node<false, false>(geo, src, nullptr, nullptr);
   else trace_persistent<false, false>(sc, src, counters + 4, nullptr, nullptr);
 }
 
@@ -1215,7 +1217,8 @@ __global__ void __launch_bounds__(1024) k_bdpt_prefix(DevPaths PS) {
 // measured fastest on the Cornell-boxes frame (558 ms vs 624 ms at 96
 // registers and 5 blocks).
 template <int MAXV, int CLS, bool kOneNode>
-__global__ void __launch_bounds__(128, 8) k_bdpt_strategies(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch) {
+__global__ void __launch_bounds__(128, 8) 
+    k_bdpt_strategies(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> geo) {
   constexpr int K = (MAXV + 1) * MAXV;
   const DevBdpt& B = PS.bd;
   const uint32_t n = ch.npix * ch.layers;
@@ -1237,7 +1240,7 @@ __global__ void __launch_bounds__(128, 8) k_bdpt_strategies(DevScene sc, DevFilm
     uint4 m = B.meta[i];
     Rng rs;
     rs.init(ch.seed, m.z, m.w, m.y + draws_before(s, t, B.masks[i]));
-    float3 c = eval_strategy<CLS, kOneNode>(sc, film, B, i, s, t, rs, err);
+    float3 c = eval_strategy<CLS, kOneNode>(sc, geo, film, B, i, s, t, rs, err);
     B.contrib[(size_t)k * n + i] = make_float4(c.x, c.y, c.z, 0.f);
   }
 }
@@ -1264,6 +1267,8 @@ __global__ void k_bdpt_sum(DevPaths PS, ChunkDesc ch) {
 template <int MAXV, bool kOneNode>
 void launch_bdpt_maxv(const DevScene& sc, const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int sms,
                       cudaStream_t st) {
+  Geom<kOneNode> geo{};
+  if constexpr (kOneNode) geo = *sc.one;
   const uint32_t n = ch.npix * ch.layers;
   const int gs = launch_grid(n, 128, std::max(1, sms * 8));  // grid-stride kernels over the queue
   const int gt = std::max(1, sms * kTravBlocks);                       // persistent traversal
@@ -1276,16 +1281,16 @@ void launch_bdpt_maxv(const DevScene& sc, const DevFilm& film, const DevPaths& P
   for (int it = 0; it < 2 * sc.max_depth; it++) {
     BdptSource src{P.bd.q[cur].o, P.bd.q[cur].d, P.bd.hit, P.counters + cur, sc.root,
                    reinterpret_cast<int*>(P.counters + 3)};
-    k_bdpt_trace<kOneNode><<<gt, 128, 0, st>>>(sc, src, P.counters, cur);
+    k_bdpt_trace<kOneNode><<<gt, 128, 0, st>>>(sc, src, P.counters, cur, geo);
     k_bdpt_extend<MAXV><<<gs, 128, 0, st>>>(sc, P, ch, cur);
     cur ^= 1;
   }
   k_bdpt_list<MAXV><<<gl, 1024, 0, st>>>(P, ch);
   k_bdpt_prefix<MAXV><<<1, 1024, 0, st>>>(P);
-  k_bdpt_strategies<MAXV, 0, false><<<g2, 128, 0, st>>>(sc, film, P, ch);
-  k_bdpt_strategies<MAXV, 1, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch);
-  k_bdpt_strategies<MAXV, 2, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch);
-  k_bdpt_strategies<MAXV, 3, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch);
+  k_bdpt_strategies<MAXV, 0, false><<<g2, 128, 0, st>>>(sc, film, P, ch, NoGeom{});
+  k_bdpt_strategies<MAXV, 1, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+  k_bdpt_strategies<MAXV, 2, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+  k_bdpt_strategies<MAXV, 3, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
   k_bdpt_sum<MAXV><<<g3, 256, 0, st>>>(P, ch);
 }
 

@@ -56,8 +56,8 @@ struct BatchSource {
 
 // Batches deal their rays out without a counter: calls on different streams share none.
 template <bool kAny, bool kOneNode>
-__global__ void __launch_bounds__(128, kTravBlocks) k_intersect(DevScene sc, BatchSource src) {
-  if (kOneNode) trace_batch_one_node<kAny, false>(sc, src, nullptr, nullptr);
+__global__ void __launch_bounds__(128, kTravBlocks) k_intersect(DevScene sc, BatchSource src, const __grid_constant__ Geom<kOneNode> g) {
+  if constexpr (kOneNode) trace_batch_one_node<kAny, false>(g, src, nullptr, nullptr);
   else trace_persistent<kAny, false>(sc, src, nullptr, nullptr, nullptr);
 }
 
@@ -71,9 +71,8 @@ void launch_intersect(const DevScene& sc, const gprt_ray* rays, uint32_t n, bool
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int grid = launch_grid((n + 31) / 32 * 32, 128, persistent_grid(sms, 128));
   BatchSource src{rays, hits, n, sc.root, err};
-  auto kernel = one_node(sc) ? (any_hit ? k_intersect<true, true> : k_intersect<false, true>)
-                             : (any_hit ? k_intersect<true, false> : k_intersect<false, false>);
-  kernel<<<grid, 128, 0, st>>>(sc, src);
+  if (one_node(sc)) (any_hit ? k_intersect<true, true> : k_intersect<false, true>)<<<grid, 128, 0, st>>>(sc, src, *sc.one);
+  else (any_hit ? k_intersect<true, false> : k_intersect<false, false>)<<<grid, 128, 0, st>>>(sc, src, NoGeom{});
 }
 
 // ----------------------------------------------------------------- raygen
@@ -164,7 +163,8 @@ static ErrSink err_sink(const DevPaths& P) { return ErrSink{P.counters + 3, P.it
 
 template <bool kCount, bool kOneNode>
 __global__ void __launch_bounds__(128, kTravBlocks)
-    k_pt_extend(DevScene sc, ExtendSource src, uint32_t* counters, int cur, unsigned long long* stats) {
+    k_pt_extend(DevScene sc, ExtendSource src, uint32_t* counters, int cur, unsigned long long* stats,
+                const __grid_constant__ Geom<kOneNode> g) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     counters[cur ^ 1] = 0;  // next queue and shadow queue start empty
     counters[2] = 0;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(128, kTravBlocks)
   }
   TraceStats ts{0, 0, 0};
   uint32_t rays = 0;
-  if (kOneNode) trace_batch_one_node<false, kCount>(sc, src, &ts, &rays);
+  if constexpr (kOneNode) trace_batch_one_node<false, kCount>(g, src, &ts, &rays);
   else trace_persistent<false, kCount>(sc, src, counters + 4, &ts, &rays);
   if (kCount) {
     __syncwarp();
@@ -227,9 +227,13 @@ void launch_pt_extend(const DevScene& sc, const DevPaths& P, int cur, int bounce
     else k_pt_extend_simple<false><<<grid, b, 0, st>>>(sc, src, P.counters, cur, P.stats);
     return;
   }
-  auto kernel = one_node(sc) ? (P.stats ? k_pt_extend<true, true> : k_pt_extend<false, true>)
-                             : (P.stats ? k_pt_extend<true, false> : k_pt_extend<false, false>);
-  kernel<<<persistent_grid(sm_count_current(), 128), 128, 0, st>>>(sc, src, P.counters, cur, P.stats);
+  const int g = persistent_grid(sm_count_current(), 128);
+  if (one_node(sc))
+    (P.stats ? k_pt_extend<true, true> : k_pt_extend<false, true>)<<<g, 128, 0, st>>>(sc, src, P.counters, cur, P.stats,
+                                                                                      *sc.one);
+  else
+    (P.stats ? k_pt_extend<true, false> : k_pt_extend<false, false>)<<<g, 128, 0, st>>>(sc, src, P.counters, cur,
+                                                                                        P.stats, NoGeom{});
 }
 
 // ----------------------------------------------------------------- shade
@@ -329,10 +333,11 @@ struct ShadowSource {
 
 template <bool kCount, bool kOneNode>
 __global__ void __launch_bounds__(128, kTravBlocks)
-    k_pt_shadow(DevScene sc, ShadowSource src, uint32_t* counters, unsigned long long* stats) {
+    k_pt_shadow(DevScene sc, ShadowSource src, uint32_t* counters, unsigned long long* stats,
+                const __grid_constant__ Geom<kOneNode> g) {
   TraceStats ts{0, 0, 0};
   uint32_t rays = 0;
-  if (kOneNode) trace_batch_one_node<true, kCount>(sc, src, &ts, &rays);
+  if constexpr (kOneNode) trace_batch_one_node<true, kCount>(g, src, &ts, &rays);
   else trace_persistent<true, kCount>(sc, src, counters + 5, &ts, &rays);
   if (kCount) {
     __syncwarp();
@@ -372,9 +377,13 @@ void launch_pt_shadow(const DevScene& sc, const DevPaths& P, int cur, int block,
     else k_pt_shadow_simple<false><<<grid, b, 0, st>>>(sc, src, P.counters, P.stats);
     return;
   }
-  auto kernel = one_node(sc) ? (P.stats ? k_pt_shadow<true, true> : k_pt_shadow<false, true>)
-                             : (P.stats ? k_pt_shadow<true, false> : k_pt_shadow<false, false>);
-  kernel<<<persistent_grid(sm_count_current(), 128), 128, 0, st>>>(sc, src, P.counters, P.stats);
+  const int g = persistent_grid(sm_count_current(), 128);
+  if (one_node(sc))
+    (P.stats ? k_pt_shadow<true, true> : k_pt_shadow<false, true>)<<<g, 128, 0, st>>>(sc, src, P.counters, P.stats,
+                                                                                      *sc.one);
+  else
+    (P.stats ? k_pt_shadow<true, false> : k_pt_shadow<false, false>)<<<g, 128, 0, st>>>(sc, src, P.counters, P.stats,
+                                                                                        NoGeom{});
 }
 
 // ----------------------------------------------------------------- whole paths
@@ -409,7 +418,7 @@ uint32_t pt_paths_max(const DevScene& sc, int sms) { return (uint32_t)sms * (one
 
 template <bool kOneNode>
 __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
-    k_pt_paths(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch) {
+    k_pt_paths(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> g) {
   const uint32_t n = ch.npix * ch.layers;
   const int lane = threadIdx.x & 31;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
@@ -465,13 +474,20 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
     if (idle == 0xffffffffu && !more) break;
     // the shadow ray of the last step, then the path's ray
     Hit hit{-1.f, kNoHit, 0.f, 0.f};
-    if (kOneNode) {
-      if (shadow) {
+    if constexpr (kOneNode) {
+      // one copy of the loop for both rays: the kernel's code does not fit the
+      // instruction caches
+#pragma unroll 1
+      for (int ray = 0; ray < 2; ray++) {
+        const bool any = ray == 0, live = any ? shadow : alive;
+        if (!__any_sync(0xffffffffu, live)) continue;
+        const float4 ro = any ? sh_o : o4, rd = any ? sh_d : d4;
         Hit h;
-        if (!trace_one_node<true, false>(sc, f3(sh_o), f3(sh_d), 0.001f, sh_o.w, __float_as_uint(sh_d.w), h))
-          Lo = f3(Lo.x + sh_c.x, Lo.y + sh_c.y, Lo.z + sh_c.z);
+        trace_one_node<false>(g, live, any, f3(ro), f3(rd), 0.001f, any ? sh_o.w : kInfF,
+                              __float_as_uint(any ? sh_d.w : o4.w), h);
+        if (!any) hit = h;
+        else if (live && h.prim == kNoHit) Lo = f3(Lo.x + sh_c.x, Lo.y + sh_c.y, Lo.z + sh_c.z);
       }
-      if (alive) trace_one_node<false, false>(sc, f3(o4), f3(d4), 0.001f, kInfF, __float_as_uint(o4.w), hit);
     } else {
       Trav s;
       bool any = shadow, busy = shadow || alive;
@@ -535,8 +551,9 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
 
 void launch_pt_paths(const DevScene& sc, const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int sms,
                      cudaStream_t st) {
-  auto kernel = one_node(sc) ? k_pt_paths<true> : k_pt_paths<false>;
-  kernel<<<sms * kPathsBlocksPerSm, kPathsBlock, 0, st>>>(sc, film, P, ch);
+  const int grid = sms * kPathsBlocksPerSm;
+  if (one_node(sc)) k_pt_paths<true><<<grid, kPathsBlock, 0, st>>>(sc, film, P, ch, *sc.one);
+  else k_pt_paths<false><<<grid, kPathsBlock, 0, st>>>(sc, film, P, ch, NoGeom{});
 }
 
 // ----------------------------------------------------------------- accumulate

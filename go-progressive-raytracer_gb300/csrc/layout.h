@@ -117,7 +117,20 @@ struct DevCamera {
   int width, height, has_lens;
 };
 
+// A scene whose BVH is a single node (all of whose children are leaves: the
+// host builder's layout of at most 32 primitives, and anything smaller), as
+// its kernels take it: by value, in the launch's constant bank.  `rec` holds
+// the triangle, quad, sphere and quadric records from off[type] on.
+constexpr int kOneNodePrims = 32;
+struct OneNode {
+  NodeChild child[4];
+  uint32_t base[4];  // global id of the first primitive of each type
+  int off[4];
+  float4 rec[kOneNodePrims * 5];
+};
+
 struct DevScene {
+  const OneNode* one;  // host memory, for the launchers; null unless the scene is one node
   const float4* nodes;
   const float4* tris;
   const float4* tri_normals;
