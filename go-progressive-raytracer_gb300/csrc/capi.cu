@@ -933,13 +933,13 @@ extern "C" int gprt_render_noalloc(gprt_scene* s, uint32_t spp, uint64_t seed, f
   P.stats = nullptr;
   // queue counters and the error word start at zero
   CK(ctx, cudaMemsetAsync(P.counters, 0, 8 * sizeof(uint32_t), st));
-  // a film view whose sample counts are zero: the ids array of the second
+  // a film view whose sample counts are zero: the state array of the second
   // queue holds them until the first bounce (raygen reads them before any
   // path is moved there)
   DevFilm film{};
   film.width = (int)s->host.sampling.width;
   film.height = (int)s->host.sampling.height;
-  film.count = reinterpret_cast<uint32_t*>(P.q[1].ids);
+  film.count = reinterpret_cast<uint32_t*>(P.q[1].st);
   k_noalloc_zero<<<launch_grid((uint32_t)npix, 256, 0), 256, 0, st>>>(film.count, (uint32_t)npix);
   ChunkDesc ch{};
   ch.pix0 = 0;

@@ -58,6 +58,25 @@ __device__ __forceinline__ bool is_zero(float3 c) { return c.x == 0.f && c.y == 
 constexpr float kPi = 3.14159265358979323846f;
 #define kInfF (__int_as_float(0x7f800000))
 
+// 32-byte records (32-byte aligned) in one 256-bit access
+__device__ __forceinline__ void load32(const float4* p, float4& a, float4& b) {
+  asm("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p)
+      : "memory");
+}
+__device__ __forceinline__ void store32(float4* p, float4 a, float4 b) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w),
+               "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+               : "memory");
+}
+__device__ __forceinline__ float4 as_float4(uint4 v) {
+  return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+__device__ __forceinline__ uint4 as_uint4(float4 v) {
+  return make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z), __float_as_uint(v.w));
+}
+
 // ----------------------------------------------------------------- sampler
 // Counter-based sampler: every value is a pure function of (job seed, pixel,
 // sample index, dimension), so a sample renders identically alone, batched
@@ -994,6 +1013,24 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* counter, bool want) {
   if (lane == leader) base = atomicAdd(counter, (uint32_t)__popc(mask));
   base = __shfl_sync(mask, base, leader);
   return base + (uint32_t)__popc(mask & ((1u << lane) - 1u));
+}
+
+// The same in two parts: the lanes that call warp_reserve together take
+// consecutive places (one atomic), and each reads its own where it needs it,
+// so that what lies between hides the atomic's way to L2 and back.
+struct Reserve {
+  unsigned mask;  // the lanes that reserved together
+  uint32_t base;  // the first place, in their lowest lane
+};
+__device__ __forceinline__ Reserve warp_reserve(uint32_t* counter) {
+  Reserve r;
+  r.mask = __activemask();
+  r.base = 0;
+  if ((threadIdx.x & 31) == (unsigned)(__ffs(r.mask) - 1)) r.base = atomicAdd(counter, (uint32_t)__popc(r.mask));
+  return r;
+}
+__device__ __forceinline__ uint32_t reserved_slot(const Reserve& r) {
+  return __shfl_sync(r.mask, r.base, __ffs(r.mask) - 1) + (uint32_t)__popc(r.mask & ((1u << (threadIdx.x & 31)) - 1u));
 }
 
 // Largest k < n with start[k] <= x (start[0] = 0, start ascending).

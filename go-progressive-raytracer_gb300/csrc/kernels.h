@@ -18,15 +18,17 @@ struct DevFilm {
 };
 
 // Live paths of one bounce, compacted: slot i of the queue holds the whole
-// state of one path (structure of arrays), so every kernel of a bounce reads
-// and writes contiguous slots.
+// state of one path, so every kernel of a bounce reads and writes contiguous
+// slots.  A path is read and written in 32-byte records, one 256-bit access
+// each: a record fills a sector, so the shading kernel's gathers in slot order
+// fetch nothing for other slots.  The radiance gathered so far is not part of
+// the state: what a path meets either emits and ends it, or scatters and emits
+// nothing, so a continuing path has gathered none (shade_step).
 struct PathBuf {
-  float4* ray_o;   // origin.xyz, primitive the ray leaves (uint bits)
-  float4* ray_d;   // direction.xyz, BVH root node of the path's scene (int bits)
-  float4* weight;  // radiance weight rgb, origin index of the path (uint bits)
-  float4* thr;     // Russian-roulette throughput rgb
-  float4* L;       // radiance gathered so far rgb
-  uint4* ids;      // pixel, sample index, sampler position, work item
+  float4* ray;  // 2 per path: origin.xyz, primitive the ray leaves (uint bits); direction.xyz, BVH root node (int bits)
+  float4* st;   // 2 per path: radiance weight rgb, origin index of the path (uint bits); pixel, sample index,
+                // sampler position, work item (uint bits)
+  float4* thr;  // Russian-roulette throughput rgb; stored only where roulette can still end the path
 };
 
 // Wavefront path state (capacity = paths per chunk).  Paths are generated in
@@ -121,7 +123,7 @@ constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 // Device bytes of the path state of `cap` paths (one region: counters, two
 // queues, hits, origin radiance, shadow rays, slot order; sh_root when multi-scene).
 constexpr size_t path_region_bytes(uint32_t cap, bool multi) {
-  return 256 + 2 * (5 * align256((size_t)cap * sizeof(float4)) + align256((size_t)cap * sizeof(uint4))) +
+  return 256 + 2 * (2 * align256((size_t)cap * 2 * sizeof(float4)) + align256((size_t)cap * sizeof(float4))) +
          5 * align256((size_t)cap * sizeof(float4)) + align256((size_t)cap * sizeof(uint32_t)) +
          (multi ? align256((size_t)cap * sizeof(int)) : 0);
 }

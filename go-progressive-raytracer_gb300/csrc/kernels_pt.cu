@@ -93,11 +93,10 @@ __global__ void k_pt_raygen(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch)
     float3 o, d;
     camera_ray(sc.cam, x, y, lens, jit, o, d);
     const PathBuf& Q = P.q[0];
-    Q.ray_o[p] = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
-    Q.ray_d[p] = make_float4(d.x, d.y, d.z, __int_as_float(sc.root));
-    // weight 1 with origin index p, roulette throughput 1 and radiance 0 are
-    // implied at bounce 0 (not stored)
-    Q.ids[p] = make_uint4(pix, sample, rng.pos, 0u);
+    store32(Q.ray + 2 * (size_t)p, make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit)),
+            make_float4(d.x, d.y, d.z, __int_as_float(sc.root)));
+    store32(Q.st + 2 * (size_t)p, make_float4(1.f, 1.f, 1.f, __uint_as_float(p)),
+            as_float4(make_uint4(pix, sample, rng.pos, 0u)));  // throughput 1 is implied at bounce 0
     P.Lout[p] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -130,15 +129,15 @@ __device__ __forceinline__ void add_counts(unsigned long long* dst, uint32_t ray
 // The rays of the current queue; built on the host and passed as a kernel
 // argument, so its pointers stay in the constant bank.
 struct ExtendSource {
-  const float4* ray_o;
-  const float4* ray_d;
+  const float4* ray;
   float4* hit;
   const uint32_t* n;
-  const float4* weight;  // origin index of each path (.w), read when reporting a bound; null at bounce 0 (slot = origin)
+  const float4* st;  // origin index of each path (first .w), read when reporting a bound
   ErrSink err;
   __device__ uint32_t count() const { return *n; }
   __device__ void load(uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& skip, int& rt) const {
-    float4 a = ray_o[i], b = ray_d[i];
+    float4 a, b;
+    load32(ray + 2 * (size_t)i, a, b);
     rt = __float_as_int(b.w);
     o = f3(a);
     d = f3(b);
@@ -151,7 +150,7 @@ struct ExtendSource {
   __device__ void store(uint32_t i, const Hit& h) const {
     bool any = h.prim != kNoHit;
     if (h.prim == kOverflowHit) {
-      err.report(weight ? __float_as_uint(weight[i].w) : i, kErrStackOverflow);
+      err.report(__float_as_uint(st[2 * (size_t)i].w), kErrStackOverflow);
       any = false;
     }
     hit[i] = make_float4(any ? h.t : -1.f, __uint_as_float(any ? h.prim : kNoHit), h.u, h.v);
@@ -219,8 +218,7 @@ static int sm_count_current() {
 }
 
 void launch_pt_extend(const DevScene& sc, const DevPaths& P, int cur, int bounce, int block, int grid, cudaStream_t st) {
-  ExtendSource src{P.q[cur].ray_o, P.q[cur].ray_d, P.hit, P.counters + cur, bounce > 0 ? P.q[cur].weight : nullptr,
-                   err_sink(P)};
+  ExtendSource src{P.q[cur].ray, P.hit, P.counters + cur, P.q[cur].st, err_sink(P)};
   if (P.variant & GPRT_JOB_SIMPLE_EXTEND) {
     int b = std::min(block, 256);
     if (P.stats) k_pt_extend_simple<true><<<grid, b, 0, st>>>(sc, src, P.counters, cur, P.stats);
@@ -271,9 +269,13 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
     ShadeOut o;
     o.cont = false;
     bool live = i < n;
-    if (live) shade_path(sc, P, P.q[cur], P.hit, slot, ch.seed, bounce, o);
+    if (live) {
+      float4 w4, ids;
+      load32(P.q[cur].st + 2 * (size_t)slot, w4, ids);
+      shade_path(sc, P, cur, slot, w4, as_uint4(ids), ch.seed, bounce, o);
+    }
     push_shade_out(P, cur, live, o);
-    if (inext < n) prefetch_slot(P.q[cur], P.hit, snext, bounce > 0);
+    if (inext < n) prefetch_slot(P.q[cur], P.hit, snext);
     slot = snext;
   }
 }
@@ -432,7 +434,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
   int bounce = 0;
   uint4 ids = make_uint4(0, 0, 0, 0);
   float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f), d4 = o4, w4 = o4, sh_o = o4, sh_d = o4;
-  float3 thr = f3(0.f, 0.f, 0.f), L = thr, sh_c = thr;
+  float3 thr = f3(0.f, 0.f, 0.f), sh_c = thr;
   float3 Lo = thr;  // what the wavefront holds at the path's origin index
   TravEntry stack[kTraceStack];
   for (;;) {
@@ -464,7 +466,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
         ids = make_uint4(pix, sample, rng.pos, 0u);
         w4 = make_float4(1.f, 1.f, 1.f, __uint_as_float(path));
         thr = f3(1.f, 1.f, 1.f);
-        L = Lo = f3(0.f, 0.f, 0.f);
+        Lo = f3(0.f, 0.f, 0.f);
         bounce = 0;
         alive = true;
       }
@@ -526,8 +528,8 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
     shadow = false;
     if (alive) {
       ShadeOut out;
-      shade_step(sc, o4, d4, make_float4(hit.t, __uint_as_float(hit.prim), hit.u, hit.v), ids, w4, thr, L, ch.seed,
-                 bounce, out, [&](float3 p, float3 dir, float dist, uint32_t prim, float3 c) {
+      shade_step(sc, o4, d4, make_float4(hit.t, __uint_as_float(hit.prim), hit.u, hit.v), ids, w4, thr, ch.seed,
+                 bounce, out, []() {}, [&](float3 p, float3 dir, float dist, uint32_t prim, float3 c) {
                    shadow = true;
                    sh_o = make_float4(p.x, p.y, p.z, dist - 0.001f);
                    sh_d = make_float4(dir.x, dir.y, dir.z, __uint_as_float(prim));
@@ -537,12 +539,11 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
       d4 = out.d;
       w4 = out.w;
       thr = out.thr;
-      L = out.L;
       ids = out.ids;
       bounce++;
+      if (!out.cont || !is_zero(out.L)) Lo = f3(Lo.x + out.L.x, Lo.y + out.L.y, Lo.z + out.L.z);
       if (!out.cont) {
         alive = false;
-        Lo = f3(Lo.x + L.x, Lo.y + L.y, Lo.z + L.z);
         if (!shadow) P.Lout[path] = make_float4(Lo.x, Lo.y, Lo.z, 0.f);
       }
     }
@@ -587,7 +588,7 @@ void launch_accumulate(const DevFilm& film, const DevPaths& P, const ChunkDesc& 
 namespace gprt {
 
 void carve_paths(unsigned char* base, uint32_t cap, bool multi, DevPaths& P) {
-  size_t f4 = align256((size_t)cap * sizeof(float4)), u4 = align256((size_t)cap * sizeof(uint4));
+  size_t f4 = align256((size_t)cap * sizeof(float4)), f8 = align256((size_t)cap * 2 * sizeof(float4));
   unsigned char* p = base;
   auto take = [&](size_t n) {
     unsigned char* r = p;
@@ -597,12 +598,9 @@ void carve_paths(unsigned char* base, uint32_t cap, bool multi, DevPaths& P) {
   P.counters = reinterpret_cast<uint32_t*>(take(256));
   for (int k = 0; k < 2; k++) {
     PathBuf& Q = P.q[k];
-    Q.ray_o = reinterpret_cast<float4*>(take(f4));
-    Q.ray_d = reinterpret_cast<float4*>(take(f4));
-    Q.weight = reinterpret_cast<float4*>(take(f4));
+    Q.ray = reinterpret_cast<float4*>(take(f8));
+    Q.st = reinterpret_cast<float4*>(take(f8));
     Q.thr = reinterpret_cast<float4*>(take(f4));
-    Q.L = reinterpret_cast<float4*>(take(f4));
-    Q.ids = reinterpret_cast<uint4*>(take(u4));
   }
   P.hit = reinterpret_cast<float4*>(take(f4));
   P.Lout = reinterpret_cast<float4*>(take(f4));

@@ -92,11 +92,10 @@ __global__ void k_srv_raygen(DevPaths P, const StepHdr* hdr, const uint32_t* pat
     float3 o, d;
     camera_ray(it.cam, x, y, lens, jit, o, d);
     const PathBuf& Q = P.q[0];
-    Q.ray_o[p] = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
-    Q.ray_d[p] = make_float4(d.x, d.y, d.z, __int_as_float(it.root));
-    // weight 1 with origin index p, roulette throughput 1 and radiance 0 are
-    // implied at bounce 0 (not stored)
-    Q.ids[p] = make_uint4(pix, sample, rng.pos, k);
+    store32(Q.ray + 2 * (size_t)p, make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit)),
+            make_float4(d.x, d.y, d.z, __int_as_float(it.root)));
+    store32(Q.st + 2 * (size_t)p, make_float4(1.f, 1.f, 1.f, __uint_as_float(p)),
+            as_float4(make_uint4(pix, sample, rng.pos, k)));  // throughput 1 is implied at bounce 0
     P.Lout[p] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -130,8 +129,9 @@ __device__ __forceinline__ void srv_shade(const DevScene& pool, const DevPaths& 
     o.cont = false;
     bool live = i < n;
     if (live) {
-      i = slot;
-      const DevItem& it = items[Q.ids[i].w];
+      float4 w4, id4;
+      load32(Q.st + 2 * (size_t)slot, w4, id4);
+      const DevItem& it = items[__float_as_uint(id4.w)];
       DevScene v = pool;
       v.materials = pool.materials + it.mat_off;
       v.lights = pool.lights + it.light_off;
@@ -146,10 +146,10 @@ __device__ __forceinline__ void srv_shade(const DevScene& pool, const DevPaths& 
       v.max_depth = it.max_depth;
       v.rr_min_bounces = it.rr_min_bounces;
       v.root = it.root;
-      shade_path(v, P, Q, P.hit, i, it.seed, bounce, o);
+      shade_path(v, P, cur, slot, w4, as_uint4(id4), it.seed, bounce, o);
     }
     push_shade_out(P, cur, live, o);
-    if (inext < n) prefetch_slot(Q, P.hit, snext, bounce > 0);
+    if (inext < n) prefetch_slot(Q, P.hit, snext);
     slot = snext;
   }
 }
