@@ -232,6 +232,43 @@ int check_device_errors(gprt_job* j) {
   return GPRT_OK;
 }
 
+// A device buffer of `bytes` for one call: the context's staging buffer, or
+// the call's own (in `own`) when it is larger than the context keeps.
+unsigned char* stage_device(gprt_ctx* ctx, size_t bytes, std::vector<void*>& own) {
+  unsigned char* d = nullptr;
+  if (bytes > kDevStage) return dev_alloc(ctx, own, &d, bytes) ? nullptr : d;
+  if (bytes > ctx->dev_stage_bytes) {
+    if (ctx->dev_stage) cudaFree(ctx->dev_stage);
+    ctx->dev_stage = nullptr;
+    ctx->dev_stage_bytes = 0;
+    std::vector<void*> kept;
+    if (dev_alloc(ctx, kept, &d, bytes)) return nullptr;
+    ctx->dev_stage = d;
+    ctx->dev_stage_bytes = bytes;
+  }
+  return ctx->dev_stage;
+}
+
+// What launch(device pointer) writes of the film, `bytes` of it, to host memory.
+template <class Launch>
+int read_via_device(gprt_job* j, size_t bytes, void* out, const char* what, Launch launch) {
+  gprt_ctx* ctx = j->scene->ctx;
+  std::vector<void*> own;
+  const bool direct = bytes <= kHostStage;
+  unsigned char* d = direct ? ctx->host_stage : stage_device(ctx, bytes, own);
+  if (!d) return GPRT_E_OOM;
+  launch(d);
+  j->launches++;
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, j->stream);
+  cudaError_t w = cudaStreamSynchronize(j->stream);
+  if (e == cudaSuccess) e = w;
+  free_all(own);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, what);
+  if (direct) std::memcpy(out, d, bytes);
+  return GPRT_OK;
+}
+
 // Uploads the primitive and node arrays of s->host (host-built BVH, and the
 // server's private copies).
 int upload_geometry(gprt_ctx* ctx, gprt_scene* s) {
@@ -340,11 +377,12 @@ int gprt_ctx_create(int device, gprt_ctx** out) {
   if (cudaSetDevice(device) != cudaSuccess) return GPRT_E_DEVICE;
   cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
   if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) return GPRT_E_DEVICE;
-  if (cudaMallocHost(reinterpret_cast<void**>(&c->h_words), 64) != cudaSuccess) {
+  if (cudaMallocHost(reinterpret_cast<void**>(&c->h_words), 256 + kHostStage) != cudaSuccess) {
     cudaGetLastError();
     cudaStreamDestroy(c->stream);
     return GPRT_E_OOM;
   }
+  c->host_stage = reinterpret_cast<unsigned char*>(c->h_words) + 256;
   *out = c.release();
   return GPRT_OK;
 }
@@ -368,6 +406,7 @@ int gprt_ctx_destroy(gprt_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
     cudaFreeHost(ctx->h_words);
+    if (ctx->dev_stage) cudaFree(ctx->dev_stage);
   }
   delete ctx;
   return GPRT_OK;
@@ -516,27 +555,36 @@ int gprt_intersect_host(gprt_scene* s, const gprt_ray* rays, uint32_t n, uint32_
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   cudaSetDevice(ctx->device);
   if (n == 0) return GPRT_OK;
-  std::vector<void*> tmp;
-  gprt_ray* dr = nullptr;
-  gprt_hit* dh = nullptr;
-  if (dev_alloc(ctx, tmp, &dr, n) || dev_alloc(ctx, tmp, &dh, n)) {
-    free_all(tmp);
-    return GPRT_E_OOM;
-  }
-  cudaError_t e = cudaMemsetAsync(s->d_err, 0, sizeof(int), ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(dr, rays, (size_t)n * sizeof(gprt_ray), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) {
-    launch_intersect(s->dev, dr, n, flags == GPRT_ANY, dh, s->d_err, ctx->stream);
+  const size_t in = (size_t)n * sizeof(gprt_ray), out = (size_t)n * sizeof(gprt_hit);
+  // the kernel sets the error word in pinned memory (only a ray that
+  // overflowed its stack writes it)
+  ctx->h_words[0] = 0;
+  int* err = reinterpret_cast<int*>(ctx->h_words);
+  cudaError_t e = cudaSuccess;
+  std::vector<void*> own;
+  if (in + out <= kHostStage) {
+    gprt_ray* r = reinterpret_cast<gprt_ray*>(ctx->host_stage);
+    gprt_hit* h = reinterpret_cast<gprt_hit*>(ctx->host_stage + in);
+    std::memcpy(r, rays, in);
+    launch_intersect(s->dev, r, n, flags == GPRT_ANY, h, err, ctx->stream);
     e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) std::memcpy(hits, h, out);
+  } else {
+    unsigned char* d = stage_device(ctx, in + out, own);
+    if (!d) return GPRT_E_OOM;
+    gprt_ray* r = reinterpret_cast<gprt_ray*>(d);
+    gprt_hit* h = reinterpret_cast<gprt_hit*>(d + in);
+    e = cudaMemcpyAsync(r, rays, in, cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) {
+      launch_intersect(s->dev, r, n, flags == GPRT_ANY, h, err, ctx->stream);
+      e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(hits, h, out, cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    free_all(own);
   }
-  if (e == cudaSuccess) e = cudaMemcpyAsync(hits, dh, (size_t)n * sizeof(gprt_hit), cudaMemcpyDeviceToHost, ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  free_all(tmp);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "intersect_host");
-  if (cudaMemcpyAsync(ctx->h_words, s->d_err, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess ||
-      cudaStreamSynchronize(ctx->stream) != cudaSuccess)
-    return cuda_fail(ctx, cudaGetLastError(), "intersect_host error word");
   if (ctx->h_words[0]) return fail(ctx, GPRT_E_BOUND, "device bound exceeded: traversal stack");
   return GPRT_OK;
 }
@@ -749,27 +797,14 @@ int gprt_job_read_film(gprt_job* j, float* rgb_sum, float* lum_sum, float* lum2_
   return GPRT_OK;
 }
 
-static int read_via_device(gprt_job* j, size_t bytes, int kind, void* out) {
-  gprt_ctx* ctx = j->scene->ctx;
-  std::vector<void*> tmp;
-  uint8_t* d = nullptr;
-  if (dev_alloc(ctx, tmp, &d, bytes)) return GPRT_E_OOM;
-  if (kind == 0) launch_resolve_rgba8(j->film, d, j->stream);
-  else launch_image_mean(j->film, reinterpret_cast<float*>(d), j->stream);
-  j->launches++;
-  cudaError_t e = cudaMemcpyAsync(out, d, bytes, cudaMemcpyDeviceToHost, j->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(j->stream);
-  free_all(tmp);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "image read-back");
-  return GPRT_OK;
-}
-
 int gprt_job_read_image(gprt_job* j, float* rgb_mean) {
   if (!j || !rgb_mean) return GPRT_E_INVALID;
   std::lock_guard<std::recursive_mutex> lk(j->scene->ctx->mu);
   cudaSetDevice(j->scene->ctx->device);
   size_t npix = (size_t)j->film.width * j->film.height;
-  return read_via_device(j, npix * 3 * sizeof(float), 1, rgb_mean);
+  return read_via_device(j, npix * 3 * sizeof(float), rgb_mean, "image read-back", [&](unsigned char* d) {
+    launch_image_mean(j->film, reinterpret_cast<float*>(d), j->stream);
+  });
 }
 
 int gprt_job_read_rgba8(gprt_job* j, uint8_t* rgba) {
@@ -777,7 +812,8 @@ int gprt_job_read_rgba8(gprt_job* j, uint8_t* rgba) {
   std::lock_guard<std::recursive_mutex> lk(j->scene->ctx->mu);
   cudaSetDevice(j->scene->ctx->device);
   size_t npix = (size_t)j->film.width * j->film.height;
-  return read_via_device(j, npix * 4, 0, rgba);
+  return read_via_device(j, npix * 4, rgba, "image read-back",
+                         [&](unsigned char* d) { launch_resolve_rgba8(j->film, d, j->stream); });
 }
 
 int gprt_job_read_tile(gprt_job* j, uint32_t x0, uint32_t y0, uint32_t x1, uint32_t y1, uint8_t* rgba) {
@@ -787,17 +823,8 @@ int gprt_job_read_tile(gprt_job* j, uint32_t x0, uint32_t y0, uint32_t x1, uint3
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   cudaSetDevice(ctx->device);
   // resolved on the device: only the tile's bytes cross to the host
-  size_t bytes = (size_t)(x1 - x0) * (y1 - y0) * 4;
-  std::vector<void*> tmp;
-  uint8_t* d = nullptr;
-  if (dev_alloc(ctx, tmp, &d, bytes)) return GPRT_E_OOM;
-  launch_resolve_tile(j->film, x0, y0, x1, y1, d, j->stream);
-  j->launches++;
-  cudaError_t e = cudaMemcpyAsync(rgba, d, bytes, cudaMemcpyDeviceToHost, j->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(j->stream);
-  free_all(tmp);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "tile read-back");
-  return GPRT_OK;
+  return read_via_device(j, (size_t)(x1 - x0) * (y1 - y0) * 4, rgba, "tile read-back",
+                         [&](unsigned char* d) { launch_resolve_tile(j->film, x0, y0, x1, y1, d, j->stream); });
 }
 
 int gprt_job_get_stats(gprt_job* j, gprt_render_stats* stats) {
