@@ -25,6 +25,16 @@ __device__ __forceinline__ float3& operator+=(float3& a, float3 b) { a = a + b; 
 __device__ __forceinline__ float3& operator*=(float3& a, float3 b) { a = a * b; return a; }
 __device__ __forceinline__ float3& operator*=(float3& a, float s) { a = a * s; return a; }
 __device__ __forceinline__ float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
+// dot with its roundings spelled out (as normalize_xy and normalize_yx)
+__device__ __forceinline__ float dot_xy(float3 a, float3 b) {
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
+}
+__device__ __forceinline__ float dot_yx_z(float3 a, float3 b) {  // z z rounded as well
+  return __fadd_rn(__fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)), __fmul_rn(a.z, b.z));
+}
+__device__ __forceinline__ float dot_yx(float3 a, float3 b) {
+  return __fmaf_rn(a.z, b.z, __fmaf_rn(a.y, b.y, __fmul_rn(a.x, b.x)));
+}
 __device__ __forceinline__ float3 cross(float3 a, float3 b) {
   return f3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
 }
@@ -1087,7 +1097,9 @@ __device__ __forceinline__ float2 cap_uv(float3 n, float3 c, float r, float3 p) 
   return make_float2((dot(l, tangent) / r + 1.f) * 0.5f, (dot(l, bitangent) / r + 1.f) * 0.5f);
 }
 
-__device__ __forceinline__ void surface_at(const DevScene& sc, float3 o, float3 d, const Hit& h, Surface& s) {
+// `yx`: the rounding of a cylinder or cone body's normal (normalize_yx, the
+// path tracer's; else normalize_xy, the BDPT subpaths').
+__device__ __forceinline__ void surface_at(const DevScene& sc, float3 o, float3 d, const Hit& h, Surface& s, bool yx) {
   s.p = o + d * h.t;  // Ray.At (pkg/core/vec3.go:216-218)
   float3 outward;
   uint32_t p = h.prim;
@@ -1153,7 +1165,7 @@ __device__ __forceinline__ void surface_at(const DevScene& sc, float3 o, float3 
       float3 radial = s.p - (base + axis * hh);
       if (uv) s.uv = axial_uv(axis, radial, hh, g1.w);
       if (kind == kQuadricCone) radial = radial + axis * ((g0.w - __ldg(Q + 2).w) / g1.w);
-      outward = normalize_yx(radial);
+      outward = yx ? normalize_yx(radial) : normalize_xy(radial);
     }
   }
   s.front = dot(d, outward) < 0.f;
@@ -1631,15 +1643,16 @@ __device__ __forceinline__ float power_heuristic(float f, float g) {
 
 // ----------------------------------------------------------------- camera
 // Camera.GetRay (pkg/geometry/camera.go:173-190)
+// `yx` as in surface_at.
 __device__ __forceinline__ void camera_ray(const DevCamera& c, int i, int j, float2 lens, float2 jit, float3& o,
-                                           float3& d) {
+                                           float3& d, bool yx) {
   float3 ps = c.pixel00 + c.du * ((float)i + (jit.x - 0.5f)) + c.dv * ((float)j + (jit.y - 0.5f));
   o = c.center;
   if (c.has_lens) {
     float2 p = sample_unit_disk(lens);
     o = c.center + c.disk_u * p.x + c.disk_v * p.y;
   }
-  d = normalize(ps - o);
+  d = yx ? normalize_yx(ps - o) : normalize_xy(ps - o);
 }
 
 }  // namespace gprt

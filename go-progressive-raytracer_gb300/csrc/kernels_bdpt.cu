@@ -20,6 +20,8 @@
 //                      vertex store (fields indexed [vertex][sample]) and the
 //                      continuing subpaths compacted into the other queue; a
 //                      camera subpath that ends starts its light subpath;
+//   k_bdpt_subpaths    (small chunks, instead of the three above) both subpaths
+//                      of every sample in one launch;
 //   k_bdpt_list        lists, per strategy (s,t) and window of 16,384
 //                      samples, the samples that have it;
 //   k_bdpt_prefix      each strategy class's prefix sums of the list counts
@@ -128,7 +130,7 @@ __device__ __forceinline__ void sample_emission(const DevScene& sc, const DevLig
     dir = sample_cosine_hemisphere(N, sd);
     n = N;
     area_pdf = 1.0f / L.area;
-    dir_pdf = dot(dir, N) / kPi;
+    dir_pdf = dot_xy(dir, N) / kPi;
     Le = L.a;
     return;
   }
@@ -142,7 +144,7 @@ __device__ __forceinline__ void sample_emission(const DevScene& sc, const DevLig
     p = f3(S) + ld * S.w;
     n = ld;
     dir = sample_cosine_hemisphere(n, sd);
-    dir_pdf = dot(dir, n) / kPi;
+    dir_pdf = dot_xy(dir, n) / kPi;
     area_pdf = 1.0f / (4.f * kPi * S.w * S.w);
     Le = L.a;
     return;
@@ -159,7 +161,7 @@ __device__ __forceinline__ void sample_emission(const DevScene& sc, const DevLig
     }
     if (L.kind == kLightDisc) {  // SampleEmissionDirection (light_sampling.go:58-80)
       dir = sample_cosine_hemisphere(n, sd);
-      dir_pdf = dot(dir, n) / kPi;
+      dir_pdf = dot_xy(dir, n) / kPi;
       Le = L.a;
       return;
     }
@@ -693,7 +695,7 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
     LightSample ls = light_sample(sc, L, cv.p, cv.n, rs.next2());
     ls.pdf *= L.prob;
     if (is_zero(ls.emission) || ls.pdf <= 0.f) return zero;
-    float ct = fabsf(dot(ls.dir, cv.n));
+    float ct = fabsf(dot_yx(ls.dir, cv.n));
     if (ct <= 0.f) return zero;
     float3 f = vertex_brdf(sc, cv, ls.dir, true);
     float3 lb = ls.emission * (1.f / ls.pdf);
@@ -762,45 +764,77 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
   return Lc * w;
 }
 
-// generateCameraPath (bdpt.go:106-135): the camera vertex and ray of every
-// sample of the chunk, queue 0 slot p = sample p.
+// Samples of a chunk per SM at most whose subpaths run in one launch and whose
+// strategies share one: above it the wavefront is as fast (1 sample per pixel,
+// depth 8, wavefront / one launch each in us: Cornell boxes 644 / 471 at
+// 65,536 samples, 993 / 970 at 147,456; spot scene 525 / 499 at 93,440, 692 /
+// 983 at 210,432; sphere scene 470 / 328 at 65,536, 564 / 617 at 147,456;
+// 20,480 triangles 877 / 505 at 65,536, 1343 / 1382 at 262,144).
+constexpr uint32_t kSmallBdptPerSm = 640;
+constexpr int kSubpathsBlock = 64, kSubpathsBlocksPerSm = 8;
+
+// A subpath between bounces (one slot of BdQueue).
+struct BdState {
+  float4 o, d, beta, last;
+  uint4 ids;
+  uint2 st;
+};
+
+// generateCameraPath (bdpt.go:106-135): the camera vertex and ray of sample p
+// of the chunk.
+__device__ __forceinline__ BdState camera_start(const DevScene& sc, const DevFilm& film, const DevBdpt& B,
+                                                const ChunkDesc& ch, uint32_t p) {
+  uint32_t layer = p / ch.npix, i = p - layer * ch.npix;
+  uint32_t pix = ch.pix_list ? ch.pix_list[ch.pix0 + i] : ch.pix0 + i;
+  uint32_t sample = film.count[pix] + layer;
+  int x = (int)(pix % (uint32_t)film.width), y = (int)(pix / (uint32_t)film.width);
+  Rng rng;
+  rng.init(ch.seed, pix, sample);
+  float2 lens = rng.next2();
+  float2 jit = rng.next2();
+  float3 o, d;
+  camera_ray(sc.cam, x, y, lens, jit, o, d, false);
+  BVert c;
+  c.p = o;
+  c.n = -d;
+  c.wi = f3(0.f, 0.f, 0.f);
+  c.beta = f3(1.f, 1.f, 1.f);
+  c.Le = f3(0.f, 0.f, 0.f);
+  c.uv = make_float2(0.f, 0.f);
+  c.fwd = 0.f;
+  c.rev = 0.f;
+  c.mat = -1;
+  c.light = -1;
+  c.prim = kNoHit;
+  c.flags = kFlagCamera;
+  put_vert(B, 0, p, c, 0.f);
+  BdState S;
+  S.o = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
+  S.d = make_float4(d.x, d.y, d.z, camera_dir_pdf(sc.cam, o, d));
+  S.beta = make_float4(1.f, 1.f, 1.f, 0.f);
+  S.last = make_float4(c.n.x, c.n.y, c.n.z, 0.f);
+  S.ids = make_uint4(p, rng.pos, pix, sample);
+  S.st = make_uint2(1u | kStCamera | kStOkBefore | kStOkLast, 0u);
+  return S;
+}
+
+__device__ __forceinline__ void put_state(const BdQueue& Q, uint32_t i, const BdState& S) {
+  Q.o[i] = S.o;
+  Q.d[i] = S.d;
+  Q.beta[i] = S.beta;
+  Q.last[i] = S.last;
+  Q.ids[i] = S.ids;
+  Q.st[i] = S.st;
+}
+
+// The camera vertex and ray of every sample of the chunk, queue 0 slot p =
+// sample p.
 template <int MAXV>
 __global__ void k_bdpt_camgen(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch) {
   const DevBdpt& B = PS.bd;
   const uint32_t n = ch.npix * ch.layers;
-  const BdQueue& Q = B.q[0];
-  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-    uint32_t layer = p / ch.npix, i = p - layer * ch.npix;
-    uint32_t pix = ch.pix_list ? ch.pix_list[ch.pix0 + i] : ch.pix0 + i;
-    uint32_t sample = film.count[pix] + layer;
-    int x = (int)(pix % (uint32_t)film.width), y = (int)(pix / (uint32_t)film.width);
-    Rng rng;
-    rng.init(ch.seed, pix, sample);
-    float2 lens = rng.next2();
-    float2 jit = rng.next2();
-    float3 o, d;
-    camera_ray(sc.cam, x, y, lens, jit, o, d);
-    BVert c;
-    c.p = o;
-    c.n = -d;
-    c.wi = f3(0.f, 0.f, 0.f);
-    c.beta = f3(1.f, 1.f, 1.f);
-    c.Le = f3(0.f, 0.f, 0.f);
-    c.uv = make_float2(0.f, 0.f);
-    c.fwd = 0.f;
-    c.rev = 0.f;
-    c.mat = -1;
-    c.light = -1;
-    c.prim = kNoHit;
-    c.flags = kFlagCamera;
-    put_vert(B, 0, p, c, 0.f);
-    Q.o[p] = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
-    Q.d[p] = make_float4(d.x, d.y, d.z, camera_dir_pdf(sc.cam, o, d));
-    Q.beta[p] = make_float4(1.f, 1.f, 1.f, 0.f);
-    Q.last[p] = make_float4(c.n.x, c.n.y, c.n.z, 0.f);
-    Q.ids[p] = make_uint4(p, rng.pos, pix, sample);
-    Q.st[p] = make_uint2(1u | kStCamera | kStOkBefore | kStOkLast, 0u);
-  }
+  for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x)
+    put_state(B.q[0], p, camera_start(sc, film, B, ch, p));
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     PS.counters[0] = n;
     PS.counters[1] = 0;
@@ -845,218 +879,292 @@ __global__ void __launch_bounds__(128, kTravBlocks)
   else trace_persistent<false, false>(sc, src, counters + 4, nullptr, nullptr);
 }
 
-// One bounce of extendPath (bdpt.go:206-291) for every subpath of queue
-// `cur`: the vertex hit (or the camera subpath's background vertex,
+// One bounce of extendPath (bdpt.go:206-291) for one subpath whose ray met h4:
+// the vertex hit (or the camera subpath's background vertex,
 // createBackgroundVertex bdpt.go:585-601), its scatter, the reverse pdf of
-// the vertex before it; continuing subpaths move to queue cur ^ 1.  A camera
-// subpath that ends starts the sample's light subpath (generateLightPath,
-// bdpt.go:139-202); a light subpath that ends gets the infinite-light pdf
-// fix-ups and completes its sample.
+// the vertex before it.  Returns whether the sample goes on, with S its next
+// ray: a camera subpath that ends starts the sample's light subpath
+// (generateLightPath, bdpt.go:139-202); a light subpath that ends gets the
+// infinite-light pdf fix-ups and completes its sample.
+template <int MAXV>
+__device__ __forceinline__ bool extend_subpath(const DevScene& sc, const DevBdpt& B, uint64_t seed, BdState& S, float4 h4) {
+  const float4 o4 = S.o, d4 = S.d, b4 = S.beta, l4 = S.last;
+  const uint4 ids = S.ids;
+  const uint2 st2 = S.st;
+  const uint32_t p = ids.x;
+  Rng rng;
+  rng.init(seed, ids.z, ids.w, ids.y);
+  const uint32_t bits = st2.x;
+  bool camera = bits & kStCamera;
+  int len = (int)(bits & 0xFF), b = (int)((bits >> 8) & 0xFF);
+  int nc = (int)st2.y;
+  const int vb = camera ? 0 : MAXV;  // vertex base of the subpath
+  const int max_bounces = camera ? sc.max_depth : sc.max_depth - 1;
+  float3 o = f3(o4), d = f3(d4), beta = f3(b4);
+  float pdf_fwd = d4.w, acc = b4.w;
+  bool ok_before = bits & kStOkBefore, ok_last = bits & kStOkLast;
+  bool surf_last = bits & kStSurfLast, inf_last = bits & kStInfLast;
+  float3 last_n = f3(l4);
+  float last_fwd = l4.w;
+  bool ended = true;
+  uint32_t prim = __float_as_uint(h4.y);
+  float rev_last = 0.f;  // the reverse pdf of the last vertex (0 unless the new vertex scatters)
+  BVert v;
+  bool has_v = false, v_ok = false;
+  if (prim == kNoHit) {
+    if (camera) {  // createBackgroundVertex (bdpt.go:585-601)
+      float3 bg = background(sc, d);
+      v.p = o + d * 1000.f;
+      v.n = -d;
+      v.wi = -d;
+      v.fwd = pdf_fwd;
+      v.rev = 0.f;
+      v.beta = beta;
+      v.Le = bg;
+      v.uv = make_float2(0.f, 0.f);
+      v.mat = -1;
+      v.light = -1;
+      v.prim = kNoHit;
+      v.flags = kFlagInfinite | (is_zero(bg) ? 0 : kFlagLight);
+      has_v = true;
+    }
+  } else {
+    Hit h{h4.x, prim, h4.z, h4.w};
+    Surface s;
+    surface_at(sc, o, d, h, s, false);
+    DevMaterial m = load_material(sc, s.mat);
+    v.p = s.p;
+    v.n = s.n;
+    v.wi = -d;
+    v.beta = beta;
+    v.Le = emitted(m, s.front, d);
+    v.mat = s.mat;
+    v.uv = s.uv;
+    v.light = -1;
+    v.prim = prim;
+    v.flags = (s.front ? kFlagFront : 0) | (is_zero(v.Le) ? 0 : kFlagLight);
+    v.rev = 0.f;
+    v.fwd = to_area_at(o, v.p, v.n, v.mat >= 0, false, pdf_fwd);
+    has_v = true;
+    Scatter scn;
+    if (scatter(sc, m, d, s, rng, scn)) {
+      float npdf = scn.pdf;
+      if (scn.pdf <= 0.f) v.flags |= kFlagSpecular;
+      float ct = fabsf(dot_yx_z(scn.dir, s.n));
+      float3 nbeta = scn.pdf <= 0.f ? beta * scn.att : beta * scn.att * (ct / scn.pdf);
+      bool rdelta;
+      float pdf_rev = mat_pdf(sc, m, scn.dir, -d, s.n, rdelta);
+      if (rdelta) {
+        v.flags |= kFlagSpecular;
+        pdf_rev = 0.f;
+        npdf = 0.f;
+      }
+      rev_last = to_area_at(v.p, o, last_n, surf_last, inf_last, pdf_rev);
+      if (b + 1 < max_bounces && len + 1 < MAXV) {
+        ended = false;
+        S.o = make_float4(s.p.x, s.p.y, s.p.z, __uint_as_float(prim));
+        S.d = make_float4(scn.dir.x, scn.dir.y, scn.dir.z, npdf);
+        beta = nbeta;
+      }
+    }
+  }
+  // the last vertex is final now: its reverse pdf and MIS prefix
+  float pre_last = next_prefix(camera, len - 1, rev_last, last_fwd, ok_last, ok_before, acc);
+  patch_vert(B, vb + len - 1, p, rev_last, pre_last);
+  if (has_v) {
+    v_ok = vertex_ok(sc, v, camera);
+    // a vertex that ends its subpath is stored with its final prefix
+    float pre_v = ended ? next_prefix(camera, len, 0.f, v.fwd, v_ok, ok_last, pre_last) : 0.f;
+    put_vert(B, vb + len, p, v, pre_v);
+    len++;
+  }
+  if (!ended) {
+    S.beta = make_float4(beta.x, beta.y, beta.z, pre_last);
+    S.last = make_float4(v.n.x, v.n.y, v.n.z, v.fwd);
+    S.ids = make_uint4(p, rng.pos, ids.z, ids.w);
+    S.st = make_uint2((uint32_t)len | ((uint32_t)(b + 1) << 8) | (camera ? kStCamera : 0u) |
+                         (ok_last ? kStOkBefore : 0u) | (v_ok ? kStOkLast : 0u) | (v.mat >= 0 ? kStSurfLast : 0u),
+                     (uint32_t)nc);
+    return true;
+  } else if (camera) {
+    nc = len;
+    if (sc.n_lights > 0) {
+      // generateLightPath (bdpt.go:139-202), in the same sampler stream
+      int li = pick_light(sc, rng.next());
+      DevLight L = sc.lights[li];
+      float2 sp = rng.next2();
+      float2 sd = rng.next2();
+      float3 ep, en, ed, Le;
+      float apdf, dpdf;
+      sample_emission(sc, L, sp, sd, ep, en, ed, Le, apdf, dpdf);
+      float ct = fabsf(dot_yx(ed, en));
+      BVert lv;
+      lv.p = ep;
+      lv.n = en;
+      lv.wi = f3(0.f, 0.f, 0.f);
+      lv.uv = make_float2(0.f, 0.f);
+      lv.light = li;
+      lv.mat = -1;
+      lv.prim = L.kind == kLightQuad     ? sc.quad_base + (uint32_t)L.prim
+                : L.kind == kLightSphere ? (L.prim >= 0 ? sc.sphere_base + (uint32_t)L.prim : kNoHit)
+                : (L.kind == kLightDisc || L.kind == kLightDiscSpot) ? sc.quadric_base + (uint32_t)L.prim
+                                                                     : kNoHit;
+      lv.fwd = apdf * L.prob;
+      lv.rev = 0.f;
+      bool inf = L.kind == kLightUniformInfinite || L.kind == kLightGradientInfinite;
+      lv.flags = kFlagLight | (inf ? kFlagInfinite : 0);
+      lv.beta = Le;
+      lv.Le = Le;
+      bool lok = vertex_ok(sc, lv, false);
+      bool lsurf = light_is_area(sc, li);
+      if (inf) {
+        B.lorig[3 * (size_t)p] = make_float4(ep.x, ep.y, ep.z, apdf);
+        B.lorig[3 * (size_t)p + 1] = make_float4(en.x, en.y, en.z, L.prob);
+        B.lorig[3 * (size_t)p + 2] = make_float4(ed.x, ed.y, ed.z, 0.f);
+      }
+      if (0 < sc.max_depth - 1 && 1 < MAXV) {
+        put_vert(B, MAXV, p, lv, 0.f);
+        float3 lb = Le * (ct / (L.prob * apdf * dpdf));
+        S.o = make_float4(ep.x, ep.y, ep.z, __uint_as_float(lv.prim));
+        S.d = make_float4(ed.x, ed.y, ed.z, dpdf);
+        S.beta = make_float4(lb.x, lb.y, lb.z, 0.f);
+        S.last = make_float4(en.x, en.y, en.z, lv.fwd);
+        S.ids = make_uint4(p, rng.pos, ids.z, ids.w);
+        S.st = make_uint2(1u | kStOkBefore | (lok ? kStOkLast : 0u) | (lsurf ? kStSurfLast : 0u) |
+                             (inf ? kStInfLast : 0u),
+                         (uint32_t)nc);
+        return true;
+      } else {  // a light subpath of the light vertex alone
+        put_vert(B, MAXV, p, lv, next_prefix(false, 0, 0.f, lv.fwd, lok, true, 0.f));
+        if (inf) {  // the fix-up of the light vertex (bdpt.go:188-199)
+          BVert l0 = get_vert(B, MAXV, p);
+          l0.fwd = infinite_density(sc, ep, en, ed);
+          put_vert(B, MAXV, p, l0);
+          subpath_prefix(sc, B, MAXV, 1, p, false);
+        }
+        finish_sample<MAXV>(sc, B, p, nc, 1, rng.pos, ids.z, ids.w);
+      }
+    } else {
+      finish_sample<MAXV>(sc, B, p, nc, 0, rng.pos, ids.z, ids.w);
+    }
+  } else {
+    int nl = len;
+    if (get_vpdf(B, MAXV, p).flags & kFlagInfinite) {
+      // the infinite-light fix-ups of generateLightPath (bdpt.go:188-199)
+      float4 e0 = B.lorig[3 * (size_t)p], e1 = B.lorig[3 * (size_t)p + 1], e2 = B.lorig[3 * (size_t)p + 2];
+      float3 ep = f3(e0), en = f3(e1), ed = f3(e2);
+      float apdf = e0.w, lprob = e1.w;
+      if (nl > 1) {
+        BVert fb = get_vert(B, MAXV + 1, p);
+        fb.fwd = apdf * lprob;
+        if (fb.mat >= 0) fb.fwd *= fabsf(dot(ed, fb.n));
+        put_vert(B, MAXV + 1, p, fb);
+      }
+      BVert l0 = get_vert(B, MAXV, p);
+      l0.fwd = infinite_density(sc, ep, en, ed);
+      put_vert(B, MAXV, p, l0);
+      subpath_prefix(sc, B, MAXV, nl, p, false);  // the corrected pdfs change every prefix
+    }
+    finish_sample<MAXV>(sc, B, p, nc, nl, rng.pos, ids.z, ids.w);
+  }
+  return false;
+}
+
+// extend_subpath for every subpath of queue `cur`; continuing ones move to
+// queue cur ^ 1.
 template <int MAXV>
 __global__ void __launch_bounds__(128, 4) k_bdpt_extend(DevScene sc, DevPaths PS, ChunkDesc ch, int cur) {
   const DevBdpt& B = PS.bd;
   const BdQueue& Q = B.q[cur];
-  const BdQueue& N = B.q[cur ^ 1];
   const uint32_t n = PS.counters[cur];
   if (blockIdx.x == 0 && threadIdx.x == 0) PS.counters[4] = 0;  // the next traversal's ray fetch counter
   for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
     uint32_t i = base + threadIdx.x;
-    bool live = i < n;
     bool cont = false;
-    float4 no = make_float4(0.f, 0.f, 0.f, 0.f), nd = no, nb = no, nl4 = no;
-    uint4 nids = make_uint4(0, 0, 0, 0);
-    uint2 nst = make_uint2(0, 0);
-    if (live) {
-      float4 o4 = Q.o[i], d4 = Q.d[i], b4 = Q.beta[i], l4 = Q.last[i], h4 = B.hit[i];
-      uint4 ids = Q.ids[i];
-      uint2 st2 = Q.st[i];
-      const uint32_t p = ids.x;
-      Rng rng;
-      rng.init(ch.seed, ids.z, ids.w, ids.y);
-      const uint32_t bits = st2.x;
-      bool camera = bits & kStCamera;
-      int len = (int)(bits & 0xFF), b = (int)((bits >> 8) & 0xFF);
-      int nc = (int)st2.y;
-      const int vb = camera ? 0 : MAXV;  // vertex base of the subpath
-      const int max_bounces = camera ? sc.max_depth : sc.max_depth - 1;
-      float3 o = f3(o4), d = f3(d4), beta = f3(b4);
-      float pdf_fwd = d4.w, acc = b4.w;
-      bool ok_before = bits & kStOkBefore, ok_last = bits & kStOkLast;
-      bool surf_last = bits & kStSurfLast, inf_last = bits & kStInfLast;
-      float3 last_n = f3(l4);
-      float last_fwd = l4.w;
-      bool ended = true;
-      uint32_t prim = __float_as_uint(h4.y);
-      float rev_last = 0.f;  // the reverse pdf of the last vertex (0 unless the new vertex scatters)
-      BVert v;
-      bool has_v = false, v_ok = false;
-      if (prim == kNoHit) {
-        if (camera) {  // createBackgroundVertex (bdpt.go:585-601)
-          float3 bg = background(sc, d);
-          v.p = o + d * 1000.f;
-          v.n = -d;
-          v.wi = -d;
-          v.fwd = pdf_fwd;
-          v.rev = 0.f;
-          v.beta = beta;
-          v.Le = bg;
-          v.uv = make_float2(0.f, 0.f);
-          v.mat = -1;
-          v.light = -1;
-          v.prim = kNoHit;
-          v.flags = kFlagInfinite | (is_zero(bg) ? 0 : kFlagLight);
-          has_v = true;
-        }
-      } else {
-        Hit h{h4.x, prim, h4.z, h4.w};
-        Surface s;
-        surface_at(sc, o, d, h, s);
-        DevMaterial m = load_material(sc, s.mat);
-        v.p = s.p;
-        v.n = s.n;
-        v.wi = -d;
-        v.beta = beta;
-        v.Le = emitted(m, s.front, d);
-        v.mat = s.mat;
-        v.uv = s.uv;
-        v.light = -1;
-        v.prim = prim;
-        v.flags = (s.front ? kFlagFront : 0) | (is_zero(v.Le) ? 0 : kFlagLight);
-        v.rev = 0.f;
-        v.fwd = to_area_at(o, v.p, v.n, v.mat >= 0, false, pdf_fwd);
-        has_v = true;
-        Scatter scn;
-        if (scatter(sc, m, d, s, rng, scn)) {
-          float npdf = scn.pdf;
-          if (scn.pdf <= 0.f) v.flags |= kFlagSpecular;
-          float ct = fabsf(dot(scn.dir, s.n));
-          float3 nbeta = scn.pdf <= 0.f ? beta * scn.att : beta * scn.att * (ct / scn.pdf);
-          bool rdelta;
-          float pdf_rev = mat_pdf(sc, m, scn.dir, -d, s.n, rdelta);
-          if (rdelta) {
-            v.flags |= kFlagSpecular;
-            pdf_rev = 0.f;
-            npdf = 0.f;
-          }
-          rev_last = to_area_at(v.p, o, last_n, surf_last, inf_last, pdf_rev);
-          if (b + 1 < max_bounces && len + 1 < MAXV) {
-            ended = false;
-            no = make_float4(s.p.x, s.p.y, s.p.z, __uint_as_float(prim));
-            nd = make_float4(scn.dir.x, scn.dir.y, scn.dir.z, npdf);
-            beta = nbeta;
-          }
-        }
-      }
-      // the last vertex is final now: its reverse pdf and MIS prefix
-      float pre_last = next_prefix(camera, len - 1, rev_last, last_fwd, ok_last, ok_before, acc);
-      patch_vert(B, vb + len - 1, p, rev_last, pre_last);
-      if (has_v) {
-        v_ok = vertex_ok(sc, v, camera);
-        // a vertex that ends its subpath is stored with its final prefix
-        float pre_v = ended ? next_prefix(camera, len, 0.f, v.fwd, v_ok, ok_last, pre_last) : 0.f;
-        put_vert(B, vb + len, p, v, pre_v);
-        len++;
-      }
-      if (!ended) {
-        nb = make_float4(beta.x, beta.y, beta.z, pre_last);
-        nl4 = make_float4(v.n.x, v.n.y, v.n.z, v.fwd);
-        nids = make_uint4(p, rng.pos, ids.z, ids.w);
-        nst = make_uint2((uint32_t)len | ((uint32_t)(b + 1) << 8) | (camera ? kStCamera : 0u) |
-                             (ok_last ? kStOkBefore : 0u) | (v_ok ? kStOkLast : 0u) | (v.mat >= 0 ? kStSurfLast : 0u),
-                         (uint32_t)nc);
-        cont = true;
-      } else if (camera) {
-        nc = len;
-        if (sc.n_lights > 0) {
-          // generateLightPath (bdpt.go:139-202), in the same sampler stream
-          int li = pick_light(sc, rng.next());
-          DevLight L = sc.lights[li];
-          float2 sp = rng.next2();
-          float2 sd = rng.next2();
-          float3 ep, en, ed, Le;
-          float apdf, dpdf;
-          sample_emission(sc, L, sp, sd, ep, en, ed, Le, apdf, dpdf);
-          float ct = fabsf(dot(ed, en));
-          BVert lv;
-          lv.p = ep;
-          lv.n = en;
-          lv.wi = f3(0.f, 0.f, 0.f);
-          lv.uv = make_float2(0.f, 0.f);
-          lv.light = li;
-          lv.mat = -1;
-          lv.prim = L.kind == kLightQuad     ? sc.quad_base + (uint32_t)L.prim
-                    : L.kind == kLightSphere ? (L.prim >= 0 ? sc.sphere_base + (uint32_t)L.prim : kNoHit)
-                    : (L.kind == kLightDisc || L.kind == kLightDiscSpot) ? sc.quadric_base + (uint32_t)L.prim
-                                                                         : kNoHit;
-          lv.fwd = apdf * L.prob;
-          lv.rev = 0.f;
-          bool inf = L.kind == kLightUniformInfinite || L.kind == kLightGradientInfinite;
-          lv.flags = kFlagLight | (inf ? kFlagInfinite : 0);
-          lv.beta = Le;
-          lv.Le = Le;
-          bool lok = vertex_ok(sc, lv, false);
-          bool lsurf = light_is_area(sc, li);
-          if (inf) {
-            B.lorig[3 * (size_t)p] = make_float4(ep.x, ep.y, ep.z, apdf);
-            B.lorig[3 * (size_t)p + 1] = make_float4(en.x, en.y, en.z, L.prob);
-            B.lorig[3 * (size_t)p + 2] = make_float4(ed.x, ed.y, ed.z, 0.f);
-          }
-          if (0 < sc.max_depth - 1 && 1 < MAXV) {
-            put_vert(B, MAXV, p, lv, 0.f);
-            float3 lb = Le * (ct / (L.prob * apdf * dpdf));
-            no = make_float4(ep.x, ep.y, ep.z, __uint_as_float(lv.prim));
-            nd = make_float4(ed.x, ed.y, ed.z, dpdf);
-            nb = make_float4(lb.x, lb.y, lb.z, 0.f);
-            nl4 = make_float4(en.x, en.y, en.z, lv.fwd);
-            nids = make_uint4(p, rng.pos, ids.z, ids.w);
-            nst = make_uint2(1u | kStOkBefore | (lok ? kStOkLast : 0u) | (lsurf ? kStSurfLast : 0u) |
-                                 (inf ? kStInfLast : 0u),
-                             (uint32_t)nc);
-            cont = true;
-          } else {  // a light subpath of the light vertex alone
-            put_vert(B, MAXV, p, lv, next_prefix(false, 0, 0.f, lv.fwd, lok, true, 0.f));
-            if (inf) {  // the fix-up of the light vertex (bdpt.go:188-199)
-              BVert l0 = get_vert(B, MAXV, p);
-              l0.fwd = infinite_density(sc, ep, en, ed);
-              put_vert(B, MAXV, p, l0);
-              subpath_prefix(sc, B, MAXV, 1, p, false);
-            }
-            finish_sample<MAXV>(sc, B, p, nc, 1, rng.pos, ids.z, ids.w);
-          }
-        } else {
-          finish_sample<MAXV>(sc, B, p, nc, 0, rng.pos, ids.z, ids.w);
-        }
-      } else {
-        int nl = len;
-        if (get_vpdf(B, MAXV, p).flags & kFlagInfinite) {
-          // the infinite-light fix-ups of generateLightPath (bdpt.go:188-199)
-          float4 e0 = B.lorig[3 * (size_t)p], e1 = B.lorig[3 * (size_t)p + 1], e2 = B.lorig[3 * (size_t)p + 2];
-          float3 ep = f3(e0), en = f3(e1), ed = f3(e2);
-          float apdf = e0.w, lprob = e1.w;
-          if (nl > 1) {
-            BVert fb = get_vert(B, MAXV + 1, p);
-            fb.fwd = apdf * lprob;
-            if (fb.mat >= 0) fb.fwd *= fabsf(dot(ed, fb.n));
-            put_vert(B, MAXV + 1, p, fb);
-          }
-          BVert l0 = get_vert(B, MAXV, p);
-          l0.fwd = infinite_density(sc, ep, en, ed);
-          put_vert(B, MAXV, p, l0);
-          subpath_prefix(sc, B, MAXV, nl, p, false);  // the corrected pdfs change every prefix
-        }
-        finish_sample<MAXV>(sc, B, p, nc, nl, rng.pos, ids.z, ids.w);
-      }
+    BdState S;
+    if (i < n) {
+      S = BdState{Q.o[i], Q.d[i], Q.beta[i], Q.last[i], Q.ids[i], Q.st[i]};
+      cont = extend_subpath<MAXV>(sc, B, ch.seed, S, B.hit[i]);
     }
     // continuing subpaths to consecutive slots of the next queue (one atomic per warp)
-    uint32_t slot = warp_append(&PS.counters[cur ^ 1], live && cont);
-    if (live && cont) {
-      N.o[slot] = no;
-      N.d[slot] = nd;
-      N.beta[slot] = nb;
-      N.last[slot] = nl4;
-      N.ids[slot] = nids;
-      N.st[slot] = nst;
+    uint32_t slot = warp_append(&PS.counters[cur ^ 1], cont);
+    if (cont) put_state(B.q[cur ^ 1], slot, S);
+  }
+}
+
+// Both subpaths of every sample in one launch, for small chunks: a lane takes
+// a sample from its camera ray to the end of its light subpath, with the state
+// between bounces in registers.  The wavefront's 2 x max_depth pairs of
+// launches each take a ray's or a shading step's chain of latencies, 8 and 22
+// us, on any number of samples (49,000 samples of the spot scene: 490 -> 400
+// us a pass, 361 us with k_bdpt_strategies_all).  The vertices are those of
+// the wavefront, bit for bit (the roundings on which the compiler's
+// contraction differs between the two are spelled out).
+template <int MAXV, bool kOneNode>
+__global__ void __launch_bounds__(kSubpathsBlock, kSubpathsBlocksPerSm)
+    k_bdpt_subpaths(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> geo) {
+  const DevBdpt& B = PS.bd;
+  const uint32_t n = ch.npix * ch.layers;
+  const int lane = threadIdx.x & 31;
+  const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t chunk = min(32u, (n + nw - 1) / nw);
+  int* err = reinterpret_cast<int*>(PS.counters + 3);
+  uint64_t at = (uint64_t)w * chunk;
+  uint32_t cur = (uint32_t)min((uint64_t)n, at), end = (uint32_t)min((uint64_t)n, at + chunk);
+  bool more = cur < end, alive = false;
+  BdState S;
+  S.o = S.d = S.beta = S.last = make_float4(0.f, 0.f, 0.f, 0.f);
+  S.ids = make_uint4(0, 0, 0, 0);
+  S.st = make_uint2(0, 0);
+  TravEntry stack[kOneNode ? 1 : kTraceStack];
+  for (;;) {
+    unsigned idle = __ballot_sync(0xffffffffu, !alive);
+    if (more && idle) {
+      if (cur == end) {
+        at += (uint64_t)nw * chunk;
+        cur = (uint32_t)min((uint64_t)n, at);
+        end = (uint32_t)min((uint64_t)n, at + chunk);
+      }
+      if (cur == end) more = false;
+      uint32_t take = min((uint32_t)__popc(idle), end - cur);
+      uint32_t rank = (uint32_t)__popc(idle & ((1u << lane) - 1u));
+      if (!alive && rank < take) {
+        S = camera_start(sc, film, B, ch, cur + rank);
+        alive = true;
+      }
+      cur += take;
+      if (take) idle = 0;
     }
+    if (idle == 0xffffffffu && !more) break;
+    Hit hit{-1.f, kNoHit, 0.f, 0.f};
+    if constexpr (kOneNode) {
+      trace_one_node<false>(geo, alive, false, f3(S.o), f3(S.d), 0.001f, kInfF, __float_as_uint(S.o.w), hit);
+    } else {
+      Trav s;
+      bool busy = alive;
+      if (busy) trav_init(s, f3(S.o), f3(S.d), 0.001f, kInfF, __float_as_uint(S.o.w), sc.root, stack);
+      for (;;) {
+        const bool testing = busy && s.testing();
+        const unsigned busy_mask = __ballot_sync(0xffffffffu, busy), test_mask = __ballot_sync(0xffffffffu, testing);
+        if (!busy_mask) break;
+        if (trav_test_now(test_mask, busy_mask)) {
+          if (testing) trav_prim<false>(sc, s, false, stack, nullptr);
+        } else if (busy && !testing && s.node >= 0) {
+          trav_visit<false>(sc, s, stack, nullptr);
+        }
+        if (busy && s.done()) {
+          if (s.hit == kOverflowHit) {
+            atomicOr(err, kErrStackOverflow);
+            s.hit = kNoHit;
+          }
+          hit = s.result();
+          busy = false;
+        }
+      }
+    }
+    if (alive)
+      alive = extend_subpath<MAXV>(sc, B, ch.seed, S,
+                                   make_float4(hit.t, __uint_as_float(hit.prim), hit.u, hit.v));
   }
 }
 
@@ -1217,8 +1325,8 @@ __global__ void __launch_bounds__(1024) k_bdpt_prefix(DevPaths PS) {
 // measured fastest on the Cornell-boxes frame (558 ms vs 624 ms at 96
 // registers and 5 blocks).
 template <int MAXV, int CLS, bool kOneNode>
-__global__ void __launch_bounds__(128, 8) 
-    k_bdpt_strategies(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> geo) {
+__device__ __forceinline__ void run_strategies(const DevScene& sc, const DevFilm& film, const DevPaths& PS,
+                                               const ChunkDesc& ch, const Geom<kOneNode>& geo) {
   constexpr int K = (MAXV + 1) * MAXV;
   const DevBdpt& B = PS.bd;
   const uint32_t n = ch.npix * ch.layers;
@@ -1245,6 +1353,26 @@ __global__ void __launch_bounds__(128, 8)
   }
 }
 
+template <int MAXV, int CLS, bool kOneNode>
+__global__ void __launch_bounds__(128, 8)
+    k_bdpt_strategies(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> geo) {
+  run_strategies<MAXV, CLS, kOneNode>(sc, film, PS, ch, geo);
+}
+
+// The four classes in one launch (blockIdx.y), for small chunks, whose launches
+// each take the time of one item (22-25 us; together 28).
+template <int MAXV, bool kOneNode>
+__global__ void __launch_bounds__(128, 8)
+    k_bdpt_strategies_all(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch,
+                          const __grid_constant__ Geom<kOneNode> geo) {
+  switch (blockIdx.y) {
+    case 0: run_strategies<MAXV, 3, kOneNode>(sc, film, PS, ch, geo); break;
+    case 1: run_strategies<MAXV, 1, kOneNode>(sc, film, PS, ch, geo); break;
+    case 2: run_strategies<MAXV, 2, kOneNode>(sc, film, PS, ch, geo); break;
+    default: run_strategies<MAXV, 0, kOneNode>(sc, film, PS, ch, geo); break;
+  }
+}
+
 template <int MAXV>
 __global__ void k_bdpt_sum(DevPaths PS, ChunkDesc ch) {
   const DevBdpt& B = PS.bd;
@@ -1255,10 +1383,18 @@ __global__ void k_bdpt_sum(DevPaths PS, ChunkDesc ch) {
     int nc = (int)(m.x & 0xFF), nl = (int)(m.x >> 8);
     float3 total = f3(0.f, 0.f, 0.f);
     for (int s = 0; s <= nl; s++)
-      for (int t = 1; t <= nc; t++) {
-        if (!listed_strategy(s, t, nc, nl, mk)) continue;  // contributes nothing: not evaluated
-        float4 c = B.contrib[(size_t)(s * MAXV + t - 1) * n + i];
-        total += f3(c);
+      for (int t0 = 1; t0 <= nc; t0 += 4) {
+        // four reads on their way at once, added in the reference's order
+        float4 c[4];
+        bool has[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+          has[k] = t0 + k <= nc && listed_strategy(s, t0 + k, nc, nl, mk);  // else contributes nothing: not evaluated
+          if (has[k]) c[k] = B.contrib[(size_t)(s * MAXV + t0 + k - 1) * n + i];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (has[k]) total += f3(c[k]);
       }
     PS.Lout[i] = make_float4(total.x, total.y, total.z, 0.f);
   }
@@ -1275,22 +1411,31 @@ void launch_bdpt_maxv(const DevScene& sc, const DevFilm& film, const DevPaths& P
   const int g2 = std::max(1, sms * 16);
   const int g3 = launch_grid(n, 256, 0);
   const int gl = std::min(launch_grid(n, 1024, 0), std::max(1, sms * 2));
-  k_bdpt_camgen<MAXV><<<g3, 256, 0, st>>>(sc, film, P, ch);
-  int cur = 0;
-  // at most max_depth camera bounces, then max_depth - 1 light bounces
-  for (int it = 0; it < 2 * sc.max_depth; it++) {
-    BdptSource src{P.bd.q[cur].o, P.bd.q[cur].d, P.bd.hit, P.counters + cur, sc.root,
-                   reinterpret_cast<int*>(P.counters + 3)};
-    k_bdpt_trace<kOneNode><<<gt, 128, 0, st>>>(sc, src, P.counters, cur, geo);
-    k_bdpt_extend<MAXV><<<gs, 128, 0, st>>>(sc, P, ch, cur);
-    cur ^= 1;
+  const bool small = n <= (uint32_t)sms * kSmallBdptPerSm && sc.max_depth > 0;
+  if (small) {
+    k_bdpt_subpaths<MAXV, kOneNode><<<sms * kSubpathsBlocksPerSm, kSubpathsBlock, 0, st>>>(sc, film, P, ch, geo);
+  } else {
+    k_bdpt_camgen<MAXV><<<g3, 256, 0, st>>>(sc, film, P, ch);
+    int cur = 0;
+    // at most max_depth camera bounces, then max_depth - 1 light bounces
+    for (int it = 0; it < 2 * sc.max_depth; it++) {
+      BdptSource src{P.bd.q[cur].o, P.bd.q[cur].d, P.bd.hit, P.counters + cur, sc.root,
+                     reinterpret_cast<int*>(P.counters + 3)};
+      k_bdpt_trace<kOneNode><<<gt, 128, 0, st>>>(sc, src, P.counters, cur, geo);
+      k_bdpt_extend<MAXV><<<gs, 128, 0, st>>>(sc, P, ch, cur);
+      cur ^= 1;
+    }
   }
   k_bdpt_list<MAXV><<<gl, 1024, 0, st>>>(P, ch);
   k_bdpt_prefix<MAXV><<<1, 1024, 0, st>>>(P);
-  k_bdpt_strategies<MAXV, 0, false><<<g2, 128, 0, st>>>(sc, film, P, ch, NoGeom{});
-  k_bdpt_strategies<MAXV, 1, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
-  k_bdpt_strategies<MAXV, 2, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
-  k_bdpt_strategies<MAXV, 3, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+  if (small) {
+    k_bdpt_strategies_all<MAXV, kOneNode><<<dim3(sms * 4, 4), 128, 0, st>>>(sc, film, P, ch, geo);
+  } else {
+    k_bdpt_strategies<MAXV, 0, false><<<g2, 128, 0, st>>>(sc, film, P, ch, NoGeom{});
+    k_bdpt_strategies<MAXV, 1, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+    k_bdpt_strategies<MAXV, 2, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+    k_bdpt_strategies<MAXV, 3, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+  }
   k_bdpt_sum<MAXV><<<g3, 256, 0, st>>>(P, ch);
 }
 

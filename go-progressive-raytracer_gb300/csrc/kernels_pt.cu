@@ -91,7 +91,7 @@ __global__ void k_pt_raygen(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch)
     float2 lens = rng.next2();
     float2 jit = rng.next2();
     float3 o, d;
-    camera_ray(sc.cam, x, y, lens, jit, o, d);
+    camera_ray(sc.cam, x, y, lens, jit, o, d, true);
     const PathBuf& Q = P.q[0];
     store32(Q.ray + 2 * (size_t)p, make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit)),
             make_float4(d.x, d.y, d.z, __int_as_float(sc.root)));
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
         float2 lens = rng.next2();
         float2 jit = rng.next2();
         float3 o, d;
-        camera_ray(sc.cam, x, y, lens, jit, o, d);
+        camera_ray(sc.cam, x, y, lens, jit, o, d, true);
         o4 = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
         d4 = make_float4(d.x, d.y, d.z, __int_as_float(sc.root));
         ids = make_uint4(pix, sample, rng.pos, 0u);

@@ -63,7 +63,7 @@ __device__ __forceinline__ void shade_step(const DevScene& sc, float4 o4, float4
     } else {
       Hit h{h4.x, prim, h4.z, h4.w};
       Surface s;
-      surface_at(sc, f3(o4), d, h, s);
+      surface_at(sc, f3(o4), d, h, s, true);
       DevMaterial m = load_material(sc, s.mat);
       L += W * emitted(m, s.front, d);  // getEmittedLight (:108-113)
       Scatter sc_;

@@ -90,7 +90,7 @@ __global__ void k_srv_raygen(DevPaths P, const StepHdr* hdr, const uint32_t* pat
     float2 lens = rng.next2();
     float2 jit = rng.next2();
     float3 o, d;
-    camera_ray(it.cam, x, y, lens, jit, o, d);
+    camera_ray(it.cam, x, y, lens, jit, o, d, true);
     const PathBuf& Q = P.q[0];
     store32(Q.ray + 2 * (size_t)p, make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit)),
             make_float4(d.x, d.y, d.z, __int_as_float(it.root)));
