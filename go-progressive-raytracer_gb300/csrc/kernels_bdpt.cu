@@ -522,6 +522,56 @@ __device__ __forceinline__ BVert fetch_vert(const SubpathRef& C, const SubpathRe
   return id >= kLightV ? Lp[id - kLightV] : C[id];
 }
 
+// The walk of calculateMISWeight (bdpt_mis.go:61-178) given the reverse pdfs
+// it recomputes next to the connection: cam1, cam2 of camera vertices t-1 and
+// t-2, lit1, lit2 of light vertices s-1 and s-2 (has_*: recomputed at all).
+template <int CLS>
+__device__ __forceinline__ float mis_walk(const DevScene& sc, const SubpathRef& C, const SubpathRef& Lp,
+                                          float sampled_fwd, int s, int t, float cam1, float cam2, float lit1,
+                                          float lit2, bool has_c1, bool has_c2, bool has_l1, bool has_l2) {
+  // the walk of bdpt_mis.go:61-178 in prefix form: the two steps next to
+  // the connection on each side (with the recomputed reverse pdfs and the
+  // connection's own connectibility), then the subpath's stored prefix
+  float sum = 0.f;
+  if (t >= 2) {  // camera vertices t-1 .. 1
+    VPdf v1 = C.pdfs(t - 1), v2 = C.pdfs(t - 2);
+    float r1 = remap0(has_c1 ? cam1 : v1.rev) / remap0(v1.fwd);
+    bool c1 = (has_c1 || !(v1.flags & kFlagSpecular)) && !(v2.flags & kFlagSpecular);
+    float inner = 0.f;
+    if (t >= 3) {
+      VPdf v3 = C.pdfs(t - 3);
+      float r2 = remap0(has_c2 ? cam2 : v2.rev) / remap0(v2.fwd);
+      bool c2 = !(v2.flags & kFlagSpecular) && !(v3.flags & kFlagSpecular);
+      inner = r2 * (v3.pre + (c2 ? 1.f : 0.f));
+    }
+    sum += r1 * (inner + (c1 ? 1.f : 0.f));
+  }
+  if (s >= 1) {  // light vertices s-1 .. 0
+    VPdf u1 = Lp.pdfs(s - 1);
+    float fw1 = (CLS == 2 && has_l1) ? sampled_fwd : u1.fwd;
+    float q1 = remap0(has_l1 ? lit1 : u1.rev) / remap0(fw1);
+    bool d1 = !(u1.flags & kFlagSpecular) && !is_delta_light(sc, u1);
+    float inner = 0.f;
+    if (s >= 2) {
+      VPdf u2 = Lp.pdfs(s - 2);
+      bool ok2 = !(u2.flags & kFlagSpecular) && !is_delta_light(sc, u2);
+      d1 = d1 && ok2;
+      float q2 = remap0(has_l2 ? lit2 : u2.rev) / remap0(u2.fwd);
+      bool d2 = ok2;
+      float b3 = 0.f;
+      if (s >= 3) {
+        VPdf u3 = Lp.pdfs(s - 3);
+        d2 = d2 && !(u3.flags & kFlagSpecular) && !is_delta_light(sc, u3);
+        b3 = u3.pre;
+      }
+      inner = q2 * (b3 + (d2 ? 1.f : 0.f));
+    }
+    if (has_l1) d1 = true;
+    sum += q1 * (inner + (d1 ? 1.f : 0.f));
+  }
+  return 1.f / (1.f + sum);
+}
+
 template <int CLS>
 __device__ __forceinline__ float mis_weight(const DevScene& sc, const SubpathRef& C, const SubpathRef& Lp,
                                          const BVert* sampled, int s, int t) {
@@ -551,11 +601,6 @@ __device__ __forceinline__ float mis_weight(const DevScene& sc, const SubpathRef
     cam1 = add(kSampledV, kNoV, c1);
     cam2 = add(c1, kSampledV, c2);
     lit1 = add(c1, c2, kSampledV);
-  } else {
-    cam1 = add(l1, l2, c1);
-    cam2 = add(c1, l1, c2);
-    lit1 = add(c1, c2, l1);
-    lit2 = add(l1, c1, l2);
   }
   float rv[4];
   for (int q = 0; q < nq; q++) {
@@ -570,47 +615,9 @@ __device__ __forceinline__ float mis_weight(const DevScene& sc, const SubpathRef
       rv[q] = vertex_pdf(sc, cur, hp ? &prev : nullptr, next);
     }
   }
-  // the walk of bdpt_mis.go:61-178 in prefix form: the two steps next to
-  // the connection on each side (with the recomputed reverse pdfs and the
-  // connection's own connectibility), then the subpath's stored prefix
-  float sum = 0.f;
-  if (t >= 2) {  // camera vertices t-1 .. 1
-    VPdf v1 = C.pdfs(t - 1), v2 = C.pdfs(t - 2);
-    float r1 = remap0(cam1 >= 0 ? rv[cam1] : v1.rev) / remap0(v1.fwd);
-    bool c1 = (cam1 >= 0 || !(v1.flags & kFlagSpecular)) && !(v2.flags & kFlagSpecular);
-    float inner = 0.f;
-    if (t >= 3) {
-      VPdf v3 = C.pdfs(t - 3);
-      float r2 = remap0(cam2 >= 0 ? rv[cam2] : v2.rev) / remap0(v2.fwd);
-      bool c2 = !(v2.flags & kFlagSpecular) && !(v3.flags & kFlagSpecular);
-      inner = r2 * (v3.pre + (c2 ? 1.f : 0.f));
-    }
-    sum += r1 * (inner + (c1 ? 1.f : 0.f));
-  }
-  if (s >= 1) {  // light vertices s-1 .. 0
-    VPdf u1 = Lp.pdfs(s - 1);
-    float fw1 = (CLS == 2 && lit1 >= 0) ? sampled->fwd : u1.fwd;
-    float q1 = remap0(lit1 >= 0 ? rv[lit1] : u1.rev) / remap0(fw1);
-    bool d1 = !(u1.flags & kFlagSpecular) && !is_delta_light(sc, u1);
-    float inner = 0.f;
-    if (s >= 2) {
-      VPdf u2 = Lp.pdfs(s - 2);
-      bool ok2 = !(u2.flags & kFlagSpecular) && !is_delta_light(sc, u2);
-      d1 = d1 && ok2;
-      float q2 = remap0(lit2 >= 0 ? rv[lit2] : u2.rev) / remap0(u2.fwd);
-      bool d2 = ok2;
-      float b3 = 0.f;
-      if (s >= 3) {
-        VPdf u3 = Lp.pdfs(s - 3);
-        d2 = d2 && !(u3.flags & kFlagSpecular) && !is_delta_light(sc, u3);
-        b3 = u3.pre;
-      }
-      inner = q2 * (b3 + (d2 ? 1.f : 0.f));
-    }
-    if (lit1 >= 0) d1 = true;
-    sum += q1 * (inner + (d1 ? 1.f : 0.f));
-  }
-  return 1.f / (1.f + sum);
+  return mis_walk<CLS>(sc, C, Lp, sampled ? sampled->fwd : 0.f, s, t, cam1 >= 0 ? rv[cam1] : 0.f,
+                       cam2 >= 0 ? rv[cam2] : 0.f, lit1 >= 0 ? rv[lit1] : 0.f, lit2 >= 0 ? rv[lit2] : 0.f, cam1 >= 0,
+                       cam2 >= 0, lit1 >= 0, lit2 >= 0);
 }
 
 // Uniform numbers the strategies before (s, t) draw, in the reference's
@@ -685,7 +692,7 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
     has = true;
     splat = true;
     Lc = c;
-  } else if (CLS == 2) {
+  } else {
     // evaluateDirectLightingStrategy (bdpt.go:334-394)
     BVert cv = C[t - 1];
     if (cv.is(kFlagSpecular) || cv.mat < 0) return zero;
@@ -719,28 +726,6 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
     sampled.beta = lb;
     sampled.Le = ls.emission;
     has = true;
-    Lc = c;
-  } else {
-    // evaluateConnectionStrategy (bdpt.go:502-561)
-    BVert lv = Lp[s - 1];
-    BVert cv = C[t - 1];
-    if (lv.is(kFlagSpecular) || cv.is(kFlagSpecular)) return zero;
-    float3 dd = lv.p - cv.p;
-    float dist = length(dd);
-    if (dist < 0.001f) return zero;
-    dd = dd * (1.f / dist);
-    float cc = dot(dd, cv.n), cl = dot(-dd, lv.n);
-    if (cc <= 0.f || cl <= 0.f) return zero;
-    float g = (cc * cl) / (dist * dist);
-    float3 cb = vertex_brdf(sc, cv, dd, true);
-    float3 lb = vertex_brdf(sc, lv, -dd, false);
-    float3 c = lv.beta * lb * cb * cv.beta * g;
-    if (is_zero(c)) return zero;
-    test = true;
-    ro = cv.p;
-    rd = dd;
-    rt = dist - 0.001f;
-    rskip = cv.prim;
     Lc = c;
   }
   if (test && occluded<kOneNode>(sc, geo, ro, rd, rt, rskip, err)) return zero;
@@ -1316,14 +1301,36 @@ __global__ void __launch_bounds__(1024) k_bdpt_prefix(DevPaths PS) {
   }
 }
 
+// The entry e = w * K + k of item g of class-prefix P (E entries, P[e] <= g <
+// P[e + 1]) for the warp's 32 consecutive items from `base`: 32 probes a
+// round for the first item's, and a search of their own for the lanes whose
+// items lie past its end.  (A binary search per lane took 13 dependent loads.)
+__device__ __forceinline__ uint32_t item_entry(const uint32_t* P, uint32_t E, uint32_t base, uint32_t g, int lane) {
+  uint32_t lo = 0, len = E;
+  while (len > 1) {
+    const uint32_t step = (len + 31) >> 5, at = lane * step;
+    const bool le = at < len && __ldg(P + lo + at) <= base;
+    const uint32_t c = (uint32_t)__popc(__ballot_sync(0xffffffffu, le)) - 1u;  // P[lo] <= base
+    lo += c * step;
+    len = min(step, len - c * step);
+  }
+  if (__ldg(P + lo + 1) > g) return lo;
+  uint32_t hi = E;
+  while (hi - lo > 1) {
+    uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(P + mid) <= g) lo = mid;
+    else hi = mid;
+  }
+  return lo;
+}
+
 // One thread per listed (strategy, sample) item of class CLS, in (window,
 // strategy) order: a warp evaluates one (s, t) for 32 samples of one window
 // that have it (uniform control flow, neighbouring warps on the same code),
 // and every strategy of a window of samples runs before the next window, so
 // the vertex reads of the window's later strategies hit L2.  The work is
-// latency-bound; 8 blocks per SM (at most 64 registers, a few spilled)
-// measured fastest on the Cornell-boxes frame (558 ms vs 624 ms at 96
-// registers and 5 blocks).
+// latency-bound: 8 blocks per SM and at most 64 registers, a few spilled.
+// Whole warps run it, for classes 0, 1 and 2.
 template <int MAXV, int CLS, bool kOneNode>
 __device__ __forceinline__ void run_strategies(const DevScene& sc, const DevFilm& film, const DevPaths& PS,
                                                const ChunkDesc& ch, const Geom<kOneNode>& geo) {
@@ -1333,30 +1340,195 @@ __device__ __forceinline__ void run_strategies(const DevScene& sc, const DevFilm
   const uint32_t E = B.nw * K;
   const uint32_t* P = B.sprefix + (size_t)CLS * (E + 1);
   const uint32_t total = __ldg(P + E);
+  const int lane = threadIdx.x & 31;
   int* err = reinterpret_cast<int*>(PS.counters + 3);
-  for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = E;  // P[lo] <= g < P[hi]
-    while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (__ldg(P + mid) <= g) lo = mid;
-      else hi = mid;
+  for (uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += gridDim.x * blockDim.x) {
+    const uint32_t g = min(base + lane, total - 1);
+    const uint32_t lo = item_entry(P, E, base, g, lane);
+    if (base + lane < total) {
+      const uint32_t w = lo / K;
+      const int k = (int)(lo - w * K);
+      const uint32_t i = B.slist[(size_t)k * B.ns + w * kBdWindow + (g - __ldg(P + lo))];
+      const int s = k / MAXV, t = k % MAXV + 1;
+      uint4 m = B.meta[i];
+      Rng rs;
+      rs.init(ch.seed, m.z, m.w, m.y + draws_before(s, t, B.masks[i]));
+      float3 c = eval_strategy<CLS, kOneNode>(sc, geo, film, B, i, s, t, rs, err);
+      B.contrib[(size_t)k * n + i] = make_float4(c.x, c.y, c.z, 0.f);
     }
-    const uint32_t w = lo / K;
-    const int k = (int)(lo - w * K);
-    const uint32_t i = B.slist[(size_t)k * B.ns + w * kBdWindow + (g - __ldg(P + lo))];
-    const int s = k / MAXV, t = k % MAXV + 1;
-    uint4 m = B.meta[i];
-    Rng rs;
-    rs.init(ch.seed, m.z, m.w, m.y + draws_before(s, t, B.masks[i]));
-    float3 c = eval_strategy<CLS, kOneNode>(sc, geo, film, B, i, s, t, rs, err);
-    B.contrib[(size_t)k * n + i] = make_float4(c.x, c.y, c.z, 0.f);
+    __syncwarp();
+  }
+}
+
+// The segment that joins light vertex pl to camera vertex pc.
+struct Connection {
+  float3 d;  // from pc to pl, unit length
+  float dist;
+};
+__device__ __forceinline__ Connection connect(float3 pl, float3 pc) {
+  Connection c;
+  c.d = pl - pc;
+  c.dist = sqrtf(dot_xy(c.d, c.d));
+  c.d = c.d * (1.f / c.dist);
+  return c;
+}
+
+// The connection strategy (evaluateConnectionStrategy, bdpt.go:502-561) of
+// light vertex s - 1 and camera vertex t - 1 of sample i, neither of them
+// specular, in three steps.  First: whether the vertices face each other.
+__device__ __forceinline__ bool connection_faces(const DevBdpt& B, uint32_t i, int s, int t) {
+  const size_t kl = (size_t)(B.maxv + s - 1) * B.ns + i, kc = (size_t)(t - 1) * B.ns + i;
+  const float3 nl = f3(B.v[1][kl]), nc = f3(B.v[1][kc]);
+  const Connection c = connect(f3(B.v[0][kl]), f3(B.v[0][kc]));
+  return !(c.dist < 0.001f) && !(dot_xy(c.d, nc) <= 0.f) && !(dot_yx(-c.d, nl) <= 0.f);
+}
+
+// Second: whether they see each other.
+template <bool kOneNode>
+__device__ __forceinline__ bool connection_visible(const DevScene& sc, const Geom<kOneNode>& geo, const DevBdpt& B,
+                                                   uint32_t i, int s, int t, int* err) {
+  const size_t kl = (size_t)(B.maxv + s - 1) * B.ns + i, kc = (size_t)(t - 1) * B.ns + i;
+  const float3 pc = f3(B.v[0][kc]);
+  const Connection c = connect(f3(B.v[0][kl]), pc);
+  return !occluded<kOneNode>(sc, geo, pc, c.d, c.dist - 0.001f, __float_as_uint(B.v[4][kc].y), err);
+}
+
+// Third: the weighted contribution.  The four reverse pdfs of the MIS weight
+// (bdpt_mis.go:61-105, 140-178) are two at each end: from the own subpath
+// towards the other end's vertex, and back.
+__device__ __forceinline__ float3 connection_value(const DevScene& sc, const DevBdpt& B, uint32_t i, int s, int t) {
+  const SubpathRef C{&B, i, 0}, Lp{&B, i, B.maxv};
+  float3 bl = f3(0.f, 0.f, 0.f), bc = bl, wl = bl, wc = bl;  // BRDFs and throughputs at the two ends
+  float cc = 0.f, cl = 0.f, dist = 0.f;
+  float cam1 = 0.f, cam2 = 0.f, lit1 = 0.f, lit2 = 0.f;
+#pragma unroll 1
+  for (int q = 0; q < 2; q++) {  // the light end, the camera end
+    const int kx = q ? t - 1 : B.maxv + s - 1, ko = q ? B.maxv + s - 1 : t - 1;
+    const BVert x = get_vert(B, kx, i), o = get_vert(B, ko, i), own = get_vert(B, kx - 1, i);
+    const Connection c = connect(q ? o.p : x.p, q ? x.p : o.p);
+    const float3 f = vertex_brdf(sc, x, q ? c.d : -c.d, q == 1);
+    float to_o, to_own;  // the pdfs of x towards o (coming from own) and towards own (coming from o)
+    if (x.is(kFlagLight)) {
+      to_o = to_own = 0.f;
+#pragma unroll 1
+      for (int r = 0; r < 2; r++) {
+        float v = vertex_light_pdf(sc, x, r ? own : o);
+        if (r) to_own = v;
+        else to_o = v;
+      }
+    } else {
+      to_o = to_own = 0.f;
+      float3 wo = o.p - x.p, wn = own.p - x.p;
+      if (x.mat >= 0 && dot(wo, wo) != 0.f && dot(wn, wn) != 0.f) {
+        wo = normalize(wo);
+        wn = normalize(wn);
+        const DevMaterial m = load_material(sc, x.mat);
+        bool d1, d2;
+        float p1 = mat_pdf(sc, m, wn, wo, x.n, d1), p2 = mat_pdf(sc, m, wo, wn, x.n, d2);
+        if (!d1) to_o = to_area(sc, x, o, p1);
+        if (!d2) to_own = to_area(sc, x, own, p2);
+      }
+    }
+    dist = c.dist;
+    if (q) {
+      bc = f;
+      wc = x.beta;
+      cc = dot_xy(c.d, x.n);
+      lit1 = to_o;
+      cam2 = to_own;
+    } else {
+      bl = f;
+      wl = x.beta;
+      cl = dot_yx(-c.d, x.n);
+      cam1 = to_o;
+      lit2 = to_own;
+    }
+  }
+  const float g = (cc * cl) / (dist * dist);
+  const float3 v = wl * bl * bc * wc * g;
+  if (is_zero(v)) return v;
+  return v * mis_walk<3>(sc, C, Lp, 0.f, s, t, cam1, cam2, lit1, lit2, true, true, true, true);
+}
+
+// The connections, by whole warps.  Of the pairs 74 % face each other and
+// 54 % see each other (Cornell boxes): the items that pass a step are
+// collected per warp until 32 of them take the next, so that every step runs
+// on full warps (25 of 32 lanes active instead of 19; 28.7 -> 24.5 ms of the
+// Cornell-boxes frame of 512 x 512 x 64 samples).  Then bound by the latency
+// of the vertex reads: 6 blocks per SM and 80 registers are faster than 8 and
+// 64 (81.4 / 83.0 ms of the frame) or 10 (85.6), and a grid that is resident
+// at once than two waves of it, which read each window of vertices twice
+// (83.0 / 86.3).
+constexpr int kConnectBlocks = 6;
+template <int MAXV, bool kOneNode>
+__device__ __forceinline__ void run_connections(const DevScene& sc, const DevPaths& PS, const ChunkDesc& ch,
+                                                const Geom<kOneNode>& geo) {
+  constexpr int K = (MAXV + 1) * MAXV;
+  __shared__ uint2 facing[4][64], seen[4][64];  // {sample, strategy}; fewer than 32 are left before 32 are added
+  const DevBdpt& B = PS.bd;
+  const uint32_t n = ch.npix * ch.layers;
+  const uint32_t E = B.nw * K;
+  const uint32_t* P = B.sprefix + (size_t)3 * (E + 1);
+  const uint32_t total = __ldg(P + E);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  int* err = reinterpret_cast<int*>(PS.counters + 3);
+  uint32_t base = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
+  int nf = 0, ns = 0;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (;;) {
+    const bool more = base < total;
+    if (ns >= 32 || (ns > 0 && !more && nf == 0)) {
+      const int take = min(ns, 32);
+      ns -= take;
+      if (lane < take) {
+        const uint2 it = seen[wp][ns + lane];
+        const int s = (int)it.y / MAXV, t = (int)it.y % MAXV + 1;
+        const float3 c = connection_value(sc, B, it.x, s, t);
+        B.contrib[(size_t)it.y * n + it.x] = make_float4(c.x, c.y, c.z, 0.f);
+      }
+      __syncwarp();
+    } else if (nf >= 32 || (nf > 0 && !more)) {
+      const int take = min(nf, 32);
+      nf -= take;
+      bool pass = false;
+      uint2 it = make_uint2(0u, 0u);
+      if (lane < take) {
+        it = facing[wp][nf + lane];
+        pass = connection_visible<kOneNode>(sc, geo, B, it.x, (int)it.y / MAXV, (int)it.y % MAXV + 1, err);
+        if (!pass) B.contrib[(size_t)it.y * n + it.x] = zero;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, pass);
+      if (pass) seen[wp][ns + __popc(m & below)] = it;
+      ns += __popc(m);
+      __syncwarp();
+    } else if (more) {
+      const uint32_t g = min(base + lane, total - 1);
+      const uint32_t lo = item_entry(P, E, base, g, lane);
+      const uint32_t w = lo / K;
+      uint2 it = make_uint2(0u, lo - w * K);
+      bool pass = false;
+      if (base + lane < total) {
+        it.x = B.slist[(size_t)it.y * B.ns + w * kBdWindow + (g - __ldg(P + lo))];
+        pass = connection_faces(B, it.x, (int)it.y / MAXV, (int)it.y % MAXV + 1);
+        if (!pass) B.contrib[(size_t)it.y * n + it.x] = zero;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, pass);
+      if (pass) facing[wp][nf + __popc(m & below)] = it;
+      nf += __popc(m);
+      base += gridDim.x * blockDim.x;
+      __syncwarp();
+    } else {
+      break;
+    }
   }
 }
 
 template <int MAXV, int CLS, bool kOneNode>
-__global__ void __launch_bounds__(128, 8)
+__global__ void __launch_bounds__(128, CLS == 3 ? kConnectBlocks : 8)
     k_bdpt_strategies(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> geo) {
-  run_strategies<MAXV, CLS, kOneNode>(sc, film, PS, ch, geo);
+  if constexpr (CLS == 3) run_connections<MAXV, kOneNode>(sc, PS, ch, geo);
+  else run_strategies<MAXV, CLS, kOneNode>(sc, film, PS, ch, geo);
 }
 
 // The four classes in one launch (blockIdx.y), for small chunks, whose launches
@@ -1366,7 +1538,7 @@ __global__ void __launch_bounds__(128, 8)
     k_bdpt_strategies_all(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch,
                           const __grid_constant__ Geom<kOneNode> geo) {
   switch (blockIdx.y) {
-    case 0: run_strategies<MAXV, 3, kOneNode>(sc, film, PS, ch, geo); break;
+    case 0: run_connections<MAXV, kOneNode>(sc, PS, ch, geo); break;
     case 1: run_strategies<MAXV, 1, kOneNode>(sc, film, PS, ch, geo); break;
     case 2: run_strategies<MAXV, 2, kOneNode>(sc, film, PS, ch, geo); break;
     default: run_strategies<MAXV, 0, kOneNode>(sc, film, PS, ch, geo); break;
@@ -1434,7 +1606,7 @@ void launch_bdpt_maxv(const DevScene& sc, const DevFilm& film, const DevPaths& P
     k_bdpt_strategies<MAXV, 0, false><<<g2, 128, 0, st>>>(sc, film, P, ch, NoGeom{});
     k_bdpt_strategies<MAXV, 1, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
     k_bdpt_strategies<MAXV, 2, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
-    k_bdpt_strategies<MAXV, 3, kOneNode><<<g2, 128, 0, st>>>(sc, film, P, ch, geo);
+    k_bdpt_strategies<MAXV, 3, kOneNode><<<sms * kConnectBlocks, 128, 0, st>>>(sc, film, P, ch, geo);
   }
   k_bdpt_sum<MAXV><<<g3, 256, 0, st>>>(P, ch);
 }

@@ -40,7 +40,7 @@ def test_small_chunks_equal_the_wavefronts(ctx, name):
         return f
 
     _, lum, lum2, count = film(0)
-    for chunk in (WARPS - 1, 32 * WARPS + 1, SMALL, SMALL + 1):
+    for chunk in (997, WARPS - 1, 32 * WARPS + 1, SMALL, SMALL + 1):
         _, l, l2, c = film(chunk)
         assert np.array_equal(c, count)
         assert np.array_equal(l, lum), chunk
