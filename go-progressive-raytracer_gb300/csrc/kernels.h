@@ -46,8 +46,8 @@ struct PathBuf {
 // last vertex's normal and forward pdf, the sample (index in the chunk,
 // sampler position, pixel, sample number) and the state bits (length,
 // bounces, camera / light, connectibility of the last two vertices, whether
-// the last vertex is on a surface or at infinity; the camera subpath's
-// length for a light subpath).
+// the last vertex is on a surface or at infinity, the strategies so far that
+// draw samples; the camera subpath's length for a light subpath).
 struct BdQueue {
   float4* o;
   float4* d;
@@ -59,7 +59,7 @@ struct BdQueue {
 
 struct DevBdpt {
   float4* v[5];
-  float4* pdf;    // per vertex: fwd, flags | (light + 1) << 8 (int bits), rev, the subpath's MIS prefix
+  float2* pdf;    // per vertex: reverse pdf, the subpath's MIS prefix through the vertex before it
   BdQueue q[2];   // the subpath wavefront's two queues
   float4* hit;    // closest hit of each slot of the current queue
   float4* lorig;  // per sample, 3 float4: the light subpath's origin (infinite lights: pdf fix-ups)
@@ -80,7 +80,7 @@ struct DevBdpt {
 };
 
 // Samples per window of the BDPT strategy lists: the vertices of a window
-// (2 * maxv records of 96 B per sample: 31 MB at maxv = 10) stay in L2 while
+// (2 * maxv records of 88 B per sample: 29 MB at maxv = 10) stay in L2 while
 // all of its strategies run.  A multiple of the list kernel's 1,024-sample
 // block.
 constexpr uint32_t kBdWindow = 16384;
@@ -111,7 +111,7 @@ struct DevPaths {
 // of the BDPT working set of `ns` samples.
 inline int bdpt_maxv(int max_depth) { return max_depth <= 9 ? 10 : 18; }
 inline size_t bdpt_bytes(uint32_t ns, int maxv) {
-  return (size_t)ns * (6 * 2 * maxv * 16 + 16 + 8 + (size_t)(maxv + 1) * maxv * 16 + 16 + 2 * 88 + 16 + 48) +
+  return (size_t)ns * (2 * maxv * 88 + 16 + 8 + (size_t)(maxv + 1) * maxv * 16 + 16 + 2 * 88 + 16 + 48) +
          (size_t)5 * (bdpt_windows(ns) * (maxv + 1) * maxv + 1) * 4 + 26 * 256;
 }
 

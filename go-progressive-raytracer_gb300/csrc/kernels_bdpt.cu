@@ -344,94 +344,73 @@ __device__ __forceinline__ bool occluded(const DevScene& sc, const Geom<kOneNode
 // ---------------------------------------------------------------- vertex store
 // Subpath vertices live in global memory as 5 float4 fields indexed
 // [vertex * ns + sample], so the 32 lanes of a warp (32 consecutive samples)
-// read one field of one vertex in a single coalesced access.  The first two
-// fields hold what a pdf request of the MIS weight reads of a vertex
-// (position, normal, material, flags, light), so those requests load two
-// fields; the forward and reverse pdfs live in the pdf record.
-__device__ __forceinline__ void put_vert(const DevBdpt& B, int v, uint32_t i, const BVert& x, float pre = 0.f) {
+// read one field of one vertex in a single coalesced access: position and
+// material | flags, normal and forward pdf, throughput and incoming direction
+// (x), incoming direction (y, z), primitive and light, emission.  The first
+// two are what a pdf request of the MIS weight reads of a vertex, the first
+// four what a strategy reads of the vertex it ends at; the emission is read at
+// a camera path's last vertex only.  What is known one bounce later (the
+// reverse pdf and the MIS prefix) is the vertex's `pdf` record.
+__device__ __forceinline__ void put_vert(const DevBdpt& B, int v, uint32_t i, const BVert& x) {
   size_t k = (size_t)v * B.ns + i;
   B.v[0][k] = make_float4(x.p.x, x.p.y, x.p.z, __int_as_float((x.mat + 1) | (x.flags << 24)));
-  B.v[1][k] = make_float4(x.n.x, x.n.y, x.n.z, __int_as_float(x.light));
+  B.v[1][k] = make_float4(x.n.x, x.n.y, x.n.z, x.fwd);
   B.v[2][k] = make_float4(x.beta.x, x.beta.y, x.beta.z, x.wi.x);
-  B.v[3][k] = make_float4(x.Le.x, x.Le.y, x.Le.z, x.wi.y);
-  B.v[4][k] = make_float4(x.wi.z, __uint_as_float(x.prim), 0.f, 0.f);
-  B.pdf[k] = make_float4(x.fwd, __int_as_float(x.flags | ((x.light + 1) << 8)), x.rev, pre);
+  B.v[3][k] = make_float4(x.wi.y, x.wi.z, __uint_as_float(x.prim), __int_as_float(x.light));
+  B.v[4][k] = make_float4(x.Le.x, x.Le.y, x.Le.z, 0.f);
   if (B.uv) B.uv[k] = x.mat >= 0 ? x.uv : make_float2(0.f, 0.f);
 }
 
 __device__ __forceinline__ BVert get_vert(const DevBdpt& B, int v, uint32_t i) {
   size_t k = (size_t)v * B.ns + i;
-  float4 a = B.v[0][k], b = B.v[1][k], c = B.v[2][k], d = B.v[3][k], e = B.v[4][k], q = B.pdf[k];
+  float4 a = B.v[0][k], b = B.v[1][k], c = B.v[2][k], d = B.v[3][k], e = B.v[4][k];
   BVert x;
   x.p = f3(a);
   int mf = __float_as_int(a.w);
   x.mat = (mf & 0xFFFFFF) - 1;
   x.flags = (mf >> 24) & 0xFF;
   x.n = f3(b);
-  x.light = __float_as_int(b.w);
-  x.fwd = q.x;
-  x.rev = q.z;  // patched after the next bounce
+  x.fwd = b.w;
+  x.rev = 0.f;
   x.beta = f3(c);
-  x.Le = f3(d);
-  x.wi = make_float3(c.w, d.w, e.x);
-  x.prim = __float_as_uint(e.y);
+  x.wi = make_float3(c.w, d.x, d.y);
+  x.prim = __float_as_uint(d.z);
+  x.light = __float_as_int(d.w);
+  x.Le = f3(e);
   x.uv = B.uv ? B.uv[k] : make_float2(0.f, 0.f);
   return x;
 }
 
-// The pdfs and flags of a stored vertex and its subpath's MIS prefix (one
-// 16-byte record): all the MIS weight reads away from the connection.
-struct VPdf {
-  float fwd, rev;
-  int flags, light;
-  float pre;
-};
-__device__ __forceinline__ VPdf get_vpdf(const DevBdpt& B, int v, uint32_t i) {
-  float4 a = B.pdf[(size_t)v * B.ns + i];
-  VPdf r;
-  r.fwd = a.x;
-  r.rev = a.z;
-  int m = __float_as_int(a.y);
-  r.flags = m & 0xFF;
-  r.light = (m >> 8) - 1;
-  r.pre = a.w;
-  return r;
-}
-// a vertex on a point light (LightTypePoint, bdpt_mis.go:130-137)
-__device__ __forceinline__ bool is_delta_light(const DevScene& sc, const VPdf& v) {
-  return (v.flags & kFlagLight) && v.light >= 0 && sc.lights[v.light].kind == kLightPointSpot;
-}
-
 __device__ __forceinline__ float remap0(float f) { return f != 0.f ? f : 1.f; }
 
-// The MIS prefix of a finished subpath, written into each vertex's pdf
-// record.  calculateMISWeight (bdpt_mis.go:13-181) walks each subpath from
-// the connection outwards, multiplying ratios r_i = remap0(rev_i) /
-// remap0(fwd_i) and adding the running product at every connectible vertex;
-// away from the two vertices next to the connection those ratios and flags
-// do not depend on the strategy, so the sum over vertices 0..k is kept as
-//   A_k = r_k * (A_{k-1} + c_k)
+// The MIS prefix of a subpath, in each vertex's pdf record.
+// calculateMISWeight (bdpt_mis.go:13-181) walks each subpath from the
+// connection outwards, multiplying ratios r_i = remap0(rev_i) / remap0(fwd_i)
+// and adding the running product at every connectible vertex; away from the
+// two vertices next to the connection those ratios and flags do not depend on
+// the strategy, so with the sum over vertices 0..k
+//   A_k = r_k * q_k,   q_k = A_{k-1} + c_k
 // (camera subpath: from vertex 1, c_k = neither vertex k nor k-1 specular;
-// light subpath: from vertex 0, c_k also excludes delta lights), and each
-// strategy evaluates only its two connection-side steps on top of it.
-__device__ __forceinline__ void subpath_prefix(const DevScene& sc, const DevBdpt& B, int base, int len, uint32_t i,
-                                               bool camera) {
+// light subpath: from vertex 0, c_k also excludes delta lights) each strategy
+// evaluates only its two connection-side steps, on top of q of the vertex
+// before the connection's.
+__device__ __forceinline__ float prefix_q(int k, bool ok, bool ok_before, float acc) {
+  return acc + (ok && (k == 0 || ok_before) ? 1.f : 0.f);
+}
+
+// The q of a finished light subpath again (its forward pdfs have changed).
+__device__ __forceinline__ void light_prefix(const DevScene& sc, const DevBdpt& B, int base, int len, uint32_t i) {
   float acc = 0.f;
   bool prev_ok = true;  // the previous vertex is neither specular nor a delta light
   for (int k = 0; k < len; k++) {
     size_t at = (size_t)(base + k) * B.ns + i;
-    float4 a = B.pdf[at];
-    int m = __float_as_int(a.y);
-    int flags = m & 0xFF, light = (m >> 8) - 1;
-    bool ok = !(flags & kFlagSpecular);
-    if (!camera) ok = ok && !((flags & kFlagLight) && light >= 0 && sc.lights[light].kind == kLightPointSpot);
-    if (camera && k == 0) {
-      acc = 0.f;  // the camera vertex takes no part in the walk
-    } else {
-      bool conn = ok && (k == 0 || prev_ok);
-      acc = (remap0(a.z) / remap0(a.x)) * (acc + (conn ? 1.f : 0.f));
-    }
-    B.pdf[at].w = acc;
+    const int flags = __float_as_int(B.v[0][at].w) >> 24 & 0xFF, light = __float_as_int(B.v[3][at].w);
+    const float fwd = B.v[1][at].w, rev = B.pdf[at].x;
+    const bool ok = !(flags & kFlagSpecular) &&
+                    !((flags & kFlagLight) && light >= 0 && sc.lights[light].kind == kLightPointSpot);
+    const float q = prefix_q(k, ok, prev_ok, acc);
+    B.pdf[at].y = q;
+    acc = (remap0(rev) / remap0(fwd)) * q;
     prev_ok = ok;
   }
 }
@@ -442,7 +421,10 @@ struct SubpathRef {
   uint32_t i;
   int base;
   __device__ BVert operator[](int k) const { return get_vert(*B, base + k, i); }
-  __device__ VPdf pdfs(int k) const { return get_vpdf(*B, base + k, i); }
+  __device__ size_t at(int k) const { return (size_t)(base + k) * B->ns + i; }
+  __device__ float fwd(int k) const { return B->v[1][at(k)].w; }
+  __device__ float q(int k) const { return B->pdf[at(k)].y; }
+  __device__ bool specular(int k) const { return __float_as_int(B->v[0][at(k)].w) >> 24 & kFlagSpecular; }
 };
 
 // ---------------------------------------------------------------- subpath wavefront
@@ -453,13 +435,20 @@ struct SubpathRef {
 // other queue.  A sample's light subpath starts, in the same sampler stream,
 // in the step that ends its camera subpath, so both kinds share the queue.
 // Each vertex is stored when it is created; its reverse pdf (set by the
-// scatter at the next vertex, bdpt.go:273-285) and its MIS prefix
-// (subpath_prefix) are patched one bounce later with one 8-byte store.
+// scatter at the next vertex, bdpt.go:273-285) and its MIS prefix are stored
+// one bounce later.
 
-// State bits of a queue slot (BdQueue::st.x): length, bounces, kind, and
-// properties of the last two vertices; st.y holds the camera subpath length.
-constexpr uint32_t kStCamera = 1u << 16, kStOkBefore = 1u << 17, kStOkLast = 1u << 18, kStSurfLast = 1u << 19,
-                   kStInfLast = 1u << 20;
+// A queue slot's state (BdQueue::st).  x: the subpath's length (5 bits),
+// bounces (5), the bits below, and from kStLightMask the light vertices whose
+// light tracing draws samples; y: the camera subpath's length (5), whether the
+// light is infinite, and from kStCamMask the camera vertices whose direct
+// lighting draws samples.  Bit s - 2 (t - 2) is strategy s (t): at most 17
+// bits for 18 vertices.  Kept along with the subpath, the masks need no second
+// pass over its vertices (of up to 2 x max_depth loads one after another, in
+// the lane that ends the sample while its warp waits).
+constexpr uint32_t kStCamera = 1u << 10, kStOkBefore = 1u << 11, kStOkLast = 1u << 12, kStSurfLast = 1u << 13,
+                   kStInfLast = 1u << 14, kStInfinite = 1u << 5;
+constexpr int kStLightMask = 15, kStCamMask = 6;
 
 // The subpath vertex is neither specular nor (light subpaths) a delta light:
 // it can take part in a connection (bdpt_mis.go:61-178).
@@ -481,35 +470,18 @@ __device__ __forceinline__ float to_area_at(float3 from, float3 p, float3 n, boo
   return pdf * inv;
 }
 
-// The MIS prefix of vertex k of a subpath from the prefix `acc` through
-// vertex k - 1 (subpath_prefix's recurrence; the camera vertex has none).
-__device__ __forceinline__ float next_prefix(bool camera, int k, float rev, float fwd, bool ok, bool ok_before,
-                                             float acc) {
-  if (camera && k == 0) return 0.f;
-  bool conn = ok && (k == 0 || ok_before);
-  return (remap0(rev) / remap0(fwd)) * (acc + (conn ? 1.f : 0.f));
-}
-
 // The reverse pdf and MIS prefix of a stored vertex, once final.
-__device__ __forceinline__ void patch_vert(const DevBdpt& B, int v, uint32_t i, float rev, float pre) {
-  *reinterpret_cast<float2*>(&B.pdf[(size_t)v * B.ns + i].z) = make_float2(rev, pre);
+__device__ __forceinline__ void put_pdf(const DevBdpt& B, int v, uint32_t i, float rev, float q) {
+  B.pdf[(size_t)v * B.ns + i] = make_float2(rev, q);
 }
 
-// The strategies that draw uniform numbers (draws_before) and the sample's
-// record for the strategy kernels, once both subpaths are stored.
-template <int MAXV>
-__device__ __forceinline__ void finish_sample(const DevScene& sc, const DevBdpt& B, uint32_t p, int nc, int nl,
-                                              uint32_t pos, uint32_t pix, uint32_t sample) {
-  uint32_t lm = 0, cm = 0;
-  for (int s = 2; s <= nl; s++)
-    if (!(get_vpdf(B, MAXV + s - 1, p).flags & kFlagSpecular)) lm |= 1u << s;
-  if (sc.n_lights > 0)
-    for (int t = 2; t <= nc; t++) {
-      BVert v = get_vert(B, t - 1, p);
-      if (!v.is(kFlagSpecular) && v.mat >= 0) cm |= 1u << t;
-    }
+// The sample's record for the strategy kernels, once both subpaths are
+// stored: lengths, and the strategies that draw uniform numbers
+// (draws_before) from the state's masks.
+__device__ __forceinline__ void finish_sample(const DevBdpt& B, uint32_t p, int nc, int nl, uint32_t pos, uint32_t pix,
+                                              uint32_t sample, uint32_t light_mask, uint32_t cam_mask) {
   B.meta[p] = make_uint4((uint32_t)nc | ((uint32_t)nl << 8), pos, pix, sample);
-  B.masks[p] = make_uint2(lm, cm);
+  B.masks[p] = make_uint2(light_mask << 2, cam_mask << 2);
 }
 
 // calculateMISWeight (bdpt_mis.go:13-181) over the stored subpaths
@@ -522,52 +494,22 @@ __device__ __forceinline__ BVert fetch_vert(const SubpathRef& C, const SubpathRe
   return id >= kLightV ? Lp[id - kLightV] : C[id];
 }
 
-// The walk of calculateMISWeight (bdpt_mis.go:61-178) given the reverse pdfs
-// it recomputes next to the connection: cam1, cam2 of camera vertices t-1 and
-// t-2, lit1, lit2 of light vertices s-1 and s-2 (has_*: recomputed at all).
+// The walk of calculateMISWeight (bdpt_mis.go:61-178) in prefix form, given
+// the reverse pdfs it recomputes next to the connection: cam1, cam2 of camera
+// vertices t - 1 and t - 2, lit1, lit2 of light vertices s - 1 and s - 2.
 template <int CLS>
-__device__ __forceinline__ float mis_walk(const DevScene& sc, const SubpathRef& C, const SubpathRef& Lp,
-                                          float sampled_fwd, int s, int t, float cam1, float cam2, float lit1,
-                                          float lit2, bool has_c1, bool has_c2, bool has_l1, bool has_l2) {
-  // the walk of bdpt_mis.go:61-178 in prefix form: the two steps next to
-  // the connection on each side (with the recomputed reverse pdfs and the
-  // connection's own connectibility), then the subpath's stored prefix
+__device__ __forceinline__ float mis_walk(const SubpathRef& C, const SubpathRef& Lp, float sampled_fwd, int s, int t,
+                                          float cam1, float cam2, float lit1, float lit2) {
   float sum = 0.f;
   if (t >= 2) {  // camera vertices t-1 .. 1
-    VPdf v1 = C.pdfs(t - 1), v2 = C.pdfs(t - 2);
-    float r1 = remap0(has_c1 ? cam1 : v1.rev) / remap0(v1.fwd);
-    bool c1 = (has_c1 || !(v1.flags & kFlagSpecular)) && !(v2.flags & kFlagSpecular);
-    float inner = 0.f;
-    if (t >= 3) {
-      VPdf v3 = C.pdfs(t - 3);
-      float r2 = remap0(has_c2 ? cam2 : v2.rev) / remap0(v2.fwd);
-      bool c2 = !(v2.flags & kFlagSpecular) && !(v3.flags & kFlagSpecular);
-      inner = r2 * (v3.pre + (c2 ? 1.f : 0.f));
-    }
-    sum += r1 * (inner + (c1 ? 1.f : 0.f));
+    const float r1 = remap0(cam1) / remap0(C.fwd(t - 1));
+    const float inner = t >= 3 ? remap0(cam2) / remap0(C.fwd(t - 2)) * C.q(t - 2) : 0.f;
+    sum += r1 * (inner + (C.specular(t - 2) ? 0.f : 1.f));
   }
   if (s >= 1) {  // light vertices s-1 .. 0
-    VPdf u1 = Lp.pdfs(s - 1);
-    float fw1 = (CLS == 2 && has_l1) ? sampled_fwd : u1.fwd;
-    float q1 = remap0(has_l1 ? lit1 : u1.rev) / remap0(fw1);
-    bool d1 = !(u1.flags & kFlagSpecular) && !is_delta_light(sc, u1);
-    float inner = 0.f;
-    if (s >= 2) {
-      VPdf u2 = Lp.pdfs(s - 2);
-      bool ok2 = !(u2.flags & kFlagSpecular) && !is_delta_light(sc, u2);
-      d1 = d1 && ok2;
-      float q2 = remap0(has_l2 ? lit2 : u2.rev) / remap0(u2.fwd);
-      bool d2 = ok2;
-      float b3 = 0.f;
-      if (s >= 3) {
-        VPdf u3 = Lp.pdfs(s - 3);
-        d2 = d2 && !(u3.flags & kFlagSpecular) && !is_delta_light(sc, u3);
-        b3 = u3.pre;
-      }
-      inner = q2 * (b3 + (d2 ? 1.f : 0.f));
-    }
-    if (has_l1) d1 = true;
-    sum += q1 * (inner + (d1 ? 1.f : 0.f));
+    const float q1 = remap0(lit1) / remap0(CLS == 2 ? sampled_fwd : Lp.fwd(s - 1));
+    const float inner = s >= 2 ? remap0(lit2) / remap0(Lp.fwd(s - 2)) * Lp.q(s - 2) : 0.f;
+    sum += q1 * (inner + 1.f);
   }
   return 1.f / (1.f + sum);
 }
@@ -615,9 +557,8 @@ __device__ __forceinline__ float mis_weight(const DevScene& sc, const SubpathRef
       rv[q] = vertex_pdf(sc, cur, hp ? &prev : nullptr, next);
     }
   }
-  return mis_walk<CLS>(sc, C, Lp, sampled ? sampled->fwd : 0.f, s, t, cam1 >= 0 ? rv[cam1] : 0.f,
-                       cam2 >= 0 ? rv[cam2] : 0.f, lit1 >= 0 ? rv[lit1] : 0.f, lit2 >= 0 ? rv[lit2] : 0.f, cam1 >= 0,
-                       cam2 >= 0, lit1 >= 0, lit2 >= 0);
+  return mis_walk<CLS>(C, Lp, sampled ? sampled->fwd : 0.f, s, t, cam1 >= 0 ? rv[cam1] : 0.f,
+                       cam2 >= 0 ? rv[cam2] : 0.f, lit1 >= 0 ? rv[lit1] : 0.f, lit2 >= 0 ? rv[lit2] : 0.f);
 }
 
 // Uniform numbers the strategies before (s, t) draw, in the reference's
@@ -792,7 +733,7 @@ __device__ __forceinline__ BdState camera_start(const DevScene& sc, const DevFil
   c.light = -1;
   c.prim = kNoHit;
   c.flags = kFlagCamera;
-  put_vert(B, 0, p, c, 0.f);
+  put_vert(B, 0, p, c);
   BdState S;
   S.o = make_float4(o.x, o.y, o.z, __uint_as_float(kNoHit));
   S.d = make_float4(d.x, d.y, d.z, camera_dir_pdf(sc.cam, o, d));
@@ -881,8 +822,8 @@ __device__ __forceinline__ bool extend_subpath(const DevScene& sc, const DevBdpt
   rng.init(seed, ids.z, ids.w, ids.y);
   const uint32_t bits = st2.x;
   bool camera = bits & kStCamera;
-  int len = (int)(bits & 0xFF), b = (int)((bits >> 8) & 0xFF);
-  int nc = (int)st2.y;
+  int len = (int)(bits & 31u), b = (int)(bits >> 5 & 31u);
+  uint32_t light_mask = bits >> kStLightMask, cam_mask = st2.y >> kStCamMask;
   const int vb = camera ? 0 : MAXV;  // vertex base of the subpath
   const int max_bounces = camera ? sc.max_depth : sc.max_depth - 1;
   float3 o = f3(o4), d = f3(d4), beta = f3(b4);
@@ -954,25 +895,29 @@ __device__ __forceinline__ bool extend_subpath(const DevScene& sc, const DevBdpt
     }
   }
   // the last vertex is final now: its reverse pdf and MIS prefix
-  float pre_last = next_prefix(camera, len - 1, rev_last, last_fwd, ok_last, ok_before, acc);
-  patch_vert(B, vb + len - 1, p, rev_last, pre_last);
+  const float q_last = prefix_q(len - 1, ok_last, ok_before, acc);
+  const float pre_last = camera && len == 1 ? 0.f : (remap0(rev_last) / remap0(last_fwd)) * q_last;
+  put_pdf(B, vb + len - 1, p, rev_last, q_last);
   if (has_v) {
     v_ok = vertex_ok(sc, v, camera);
-    // a vertex that ends its subpath is stored with its final prefix
-    float pre_v = ended ? next_prefix(camera, len, 0.f, v.fwd, v_ok, ok_last, pre_last) : 0.f;
-    put_vert(B, vb + len, p, v, pre_v);
+    put_vert(B, vb + len, p, v);
+    if (ended) put_pdf(B, vb + len, p, 0.f, prefix_q(len, v_ok, ok_last, pre_last));  // no bounce follows
+    const bool specular = v.is(kFlagSpecular);
+    if (camera) cam_mask |= !specular && v.mat >= 0 && sc.n_lights > 0 ? 1u << (len - 1) : 0u;
+    else light_mask |= specular ? 0u : 1u << (len - 1);
     len++;
   }
   if (!ended) {
     S.beta = make_float4(beta.x, beta.y, beta.z, pre_last);
     S.last = make_float4(v.n.x, v.n.y, v.n.z, v.fwd);
     S.ids = make_uint4(p, rng.pos, ids.z, ids.w);
-    S.st = make_uint2((uint32_t)len | ((uint32_t)(b + 1) << 8) | (camera ? kStCamera : 0u) |
-                         (ok_last ? kStOkBefore : 0u) | (v_ok ? kStOkLast : 0u) | (v.mat >= 0 ? kStSurfLast : 0u),
-                     (uint32_t)nc);
+    S.st = make_uint2((uint32_t)len | ((uint32_t)(b + 1) << 5) | (camera ? kStCamera : 0u) |
+                         (ok_last ? kStOkBefore : 0u) | (v_ok ? kStOkLast : 0u) | (v.mat >= 0 ? kStSurfLast : 0u) |
+                         light_mask << kStLightMask,
+                     (st2.y & 63u) | cam_mask << kStCamMask);
     return true;
   } else if (camera) {
-    nc = len;
+    const int nc = len;
     if (sc.n_lights > 0) {
       // generateLightPath (bdpt.go:139-202), in the same sampler stream
       int li = pick_light(sc, rng.next());
@@ -1008,7 +953,7 @@ __device__ __forceinline__ bool extend_subpath(const DevScene& sc, const DevBdpt
         B.lorig[3 * (size_t)p + 2] = make_float4(ed.x, ed.y, ed.z, 0.f);
       }
       if (0 < sc.max_depth - 1 && 1 < MAXV) {
-        put_vert(B, MAXV, p, lv, 0.f);
+        put_vert(B, MAXV, p, lv);
         float3 lb = Le * (ct / (L.prob * apdf * dpdf));
         S.o = make_float4(ep.x, ep.y, ep.z, __uint_as_float(lv.prim));
         S.d = make_float4(ed.x, ed.y, ed.z, dpdf);
@@ -1017,40 +962,35 @@ __device__ __forceinline__ bool extend_subpath(const DevScene& sc, const DevBdpt
         S.ids = make_uint4(p, rng.pos, ids.z, ids.w);
         S.st = make_uint2(1u | kStOkBefore | (lok ? kStOkLast : 0u) | (lsurf ? kStSurfLast : 0u) |
                              (inf ? kStInfLast : 0u),
-                         (uint32_t)nc);
+                         (uint32_t)nc | (inf ? kStInfinite : 0u) | cam_mask << kStCamMask);
         return true;
       } else {  // a light subpath of the light vertex alone
-        put_vert(B, MAXV, p, lv, next_prefix(false, 0, 0.f, lv.fwd, lok, true, 0.f));
-        if (inf) {  // the fix-up of the light vertex (bdpt.go:188-199)
-          BVert l0 = get_vert(B, MAXV, p);
-          l0.fwd = infinite_density(sc, ep, en, ed);
-          put_vert(B, MAXV, p, l0);
-          subpath_prefix(sc, B, MAXV, 1, p, false);
-        }
-        finish_sample<MAXV>(sc, B, p, nc, 1, rng.pos, ids.z, ids.w);
+        if (inf) lv.fwd = infinite_density(sc, ep, en, ed);  // the fix-up of the light vertex (bdpt.go:188-199)
+        put_vert(B, MAXV, p, lv);
+        put_pdf(B, MAXV, p, 0.f, prefix_q(0, lok, true, 0.f));
+        finish_sample(B, p, nc, 1, rng.pos, ids.z, ids.w, 0u, cam_mask);
       }
     } else {
-      finish_sample<MAXV>(sc, B, p, nc, 0, rng.pos, ids.z, ids.w);
+      finish_sample(B, p, nc, 0, rng.pos, ids.z, ids.w, 0u, cam_mask);
     }
   } else {
     int nl = len;
-    if (get_vpdf(B, MAXV, p).flags & kFlagInfinite) {
+    if (st2.y & kStInfinite) {
       // the infinite-light fix-ups of generateLightPath (bdpt.go:188-199)
       float4 e0 = B.lorig[3 * (size_t)p], e1 = B.lorig[3 * (size_t)p + 1], e2 = B.lorig[3 * (size_t)p + 2];
       float3 ep = f3(e0), en = f3(e1), ed = f3(e2);
       float apdf = e0.w, lprob = e1.w;
       if (nl > 1) {
-        BVert fb = get_vert(B, MAXV + 1, p);
-        fb.fwd = apdf * lprob;
-        if (fb.mat >= 0) fb.fwd *= fabsf(dot(ed, fb.n));
-        put_vert(B, MAXV + 1, p, fb);
+        const size_t at = (size_t)(MAXV + 1) * B.ns + p;
+        const float4 n4 = B.v[1][at];
+        float fwd = apdf * lprob;
+        if ((__float_as_int(B.v[0][at].w) & 0xFFFFFF) > 0) fwd *= fabsf(dot(ed, f3(n4)));  // a surface
+        B.v[1][at].w = fwd;
       }
-      BVert l0 = get_vert(B, MAXV, p);
-      l0.fwd = infinite_density(sc, ep, en, ed);
-      put_vert(B, MAXV, p, l0);
-      subpath_prefix(sc, B, MAXV, nl, p, false);  // the corrected pdfs change every prefix
+      B.v[1][(size_t)MAXV * B.ns + p].w = infinite_density(sc, ep, en, ed);
+      light_prefix(sc, B, MAXV, nl, p);  // the corrected pdfs change every prefix
     }
-    finish_sample<MAXV>(sc, B, p, nc, nl, rng.pos, ids.z, ids.w);
+    finish_sample(B, p, (int)(st2.y & 31u), nl, rng.pos, ids.z, ids.w, light_mask, cam_mask);
   }
   return false;
 }
@@ -1390,7 +1330,7 @@ __device__ __forceinline__ bool connection_visible(const DevScene& sc, const Geo
   const size_t kl = (size_t)(B.maxv + s - 1) * B.ns + i, kc = (size_t)(t - 1) * B.ns + i;
   const float3 pc = f3(B.v[0][kc]);
   const Connection c = connect(f3(B.v[0][kl]), pc);
-  return !occluded<kOneNode>(sc, geo, pc, c.d, c.dist - 0.001f, __float_as_uint(B.v[4][kc].y), err);
+  return !occluded<kOneNode>(sc, geo, pc, c.d, c.dist - 0.001f, __float_as_uint(B.v[3][kc].z), err);
 }
 
 // Third: the weighted contribution.  The four reverse pdfs of the MIS weight
@@ -1447,7 +1387,7 @@ __device__ __forceinline__ float3 connection_value(const DevScene& sc, const Dev
   const float g = (cc * cl) / (dist * dist);
   const float3 v = wl * bl * bc * wc * g;
   if (is_zero(v)) return v;
-  return v * mis_walk<3>(sc, C, Lp, 0.f, s, t, cam1, cam2, lit1, lit2, true, true, true, true);
+  return v * mis_walk<3>(C, Lp, 0.f, s, t, cam1, cam2, lit1, lit2);
 }
 
 // The connections, by whole warps.  Of the pairs 74 % face each other and
