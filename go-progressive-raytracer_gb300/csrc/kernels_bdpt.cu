@@ -692,12 +692,13 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
 
 // Samples of a chunk per SM at most whose subpaths run in one launch and whose
 // strategies share one: above it the wavefront is as fast (1 sample per pixel,
-// depth 8, wavefront / one launch each in us: Cornell boxes 644 / 471 at
-// 65,536 samples, 993 / 970 at 147,456; spot scene 525 / 499 at 93,440, 692 /
-// 983 at 210,432; sphere scene 470 / 328 at 65,536, 564 / 617 at 147,456;
-// 20,480 triangles 877 / 505 at 65,536, 1343 / 1382 at 262,144).
-constexpr uint32_t kSmallBdptPerSm = 640;
-constexpr int kSubpathsBlock = 64, kSubpathsBlocksPerSm = 8;
+// depth 8, wavefront / one launch each in us: Cornell boxes 570 / 418 at
+// 65,536 samples, 865 / 835 at 147,456, 1324 / 1475 at 262,144; spot scene
+// 628 / 507 at 210,432, 851 / 830 at 374,272; sphere scene 535 / 372 at
+// 147,456, 1106 / 1085 at 589,824; 20,480 triangles 1015 / 801 at 147,456,
+// 1281 / 1253 at 262,144).
+constexpr uint32_t kSmallBdptPerSm = 1024;
+constexpr int kSubpathsBlock = 512, kSubpathsBlocksPerSm = 1;
 
 // A subpath between bounces (one slot of BdQueue).
 struct BdState {
@@ -1021,10 +1022,13 @@ __global__ void __launch_bounds__(128, 4) k_bdpt_extend(DevScene sc, DevPaths PS
 // a sample from its camera ray to the end of its light subpath, with the state
 // between bounces in registers.  The wavefront's 2 x max_depth pairs of
 // launches each take a ray's or a shading step's chain of latencies, 8 and 22
-// us, on any number of samples (49,000 samples of the spot scene: 490 -> 400
-// us a pass, 361 us with k_bdpt_strategies_all).  The vertices are those of
-// the wavefront, bit for bit (the roundings on which the compiler's
-// contraction differs between the two are spelled out).
+// us, on any number of samples (34,000 samples of the spot scene: 480 us a
+// frame, 371 so).  What is left is bound by fetching instructions, so the
+// warps of a block trace together and extend together and share them (two
+// barriers a bounce; the same frame, after other changes: 64-thread blocks
+// without the barriers 341 us, with them 336, 128 299, 256 277, 512 247).
+// The vertices are those of the wavefront, bit for bit (the roundings on which
+// the compiler's contraction differs between the two are spelled out).
 template <int MAXV, bool kOneNode>
 __global__ void __launch_bounds__(kSubpathsBlock, kSubpathsBlocksPerSm)
     k_bdpt_subpaths(DevScene sc, DevFilm film, DevPaths PS, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> geo) {
@@ -1060,7 +1064,7 @@ __global__ void __launch_bounds__(kSubpathsBlock, kSubpathsBlocksPerSm)
       cur += take;
       if (take) idle = 0;
     }
-    if (idle == 0xffffffffu && !more) break;
+    if (!__syncthreads_or(idle != 0xffffffffu || more)) break;
     Hit hit{-1.f, kNoHit, 0.f, 0.f};
     if constexpr (kOneNode) {
       trace_one_node<false>(geo, alive, false, f3(S.o), f3(S.d), 0.001f, kInfF, __float_as_uint(S.o.w), hit);
@@ -1087,6 +1091,7 @@ __global__ void __launch_bounds__(kSubpathsBlock, kSubpathsBlocksPerSm)
         }
       }
     }
+    __syncthreads();
     if (alive)
       alive = extend_subpath<MAXV>(sc, B, ch.seed, S,
                                    make_float4(hit.t, __uint_as_float(hit.prim), hit.u, hit.v));

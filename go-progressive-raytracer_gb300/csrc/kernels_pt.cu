@@ -395,31 +395,43 @@ void launch_pt_shadow(const DevScene& sc, const DevPaths& P, int cur, int block,
 // pass through memory.  The wavefront's 3-4 launches per bounce cost 30-45 us
 // each on any number of paths (a launch, and one ray's chain of dependent
 // loads on an almost empty chip), and a scene of depth 50 pays that 50 times;
-// here the chain of a path's bounces is all that is left.  It loses on large
-// wavefronts, where lanes of a warp part ways and 16 warps per SM hide less
-// than the traversal kernels' 32.
+// here the chain of a path's bounces is all that is left.
+// What bounds that chain is fetching instructions: a bounce runs 2,600 of
+// them, more than the caches near the scheduler hold, and warps at different
+// places of the code evict each other's (6.5-9 of 11 cycles per instruction
+// waited for one).  So the warps of a block trace together and shade together
+// (two barriers a bounce) and share what they fetch: default scene, 90,000
+// paths of depth 50, 16 rounds, 64-thread blocks without the barriers 9.96 ms,
+// blocks of 128 with them 8.94, 256 7.86, 512 7.23; more barriers, inside the
+// shading step, gained 1 %.  Trees, whose traversals differ more in length,
+// keep to 256 (sphere scene 128 x 128: 188 us without, 178 at 256, 183 at 512).
+// It loses on large wavefronts, where lanes of a warp part ways and 16 warps
+// per SM hide less than the traversal kernels' 32.
 // Results are those of the wavefront, bit for bit: the same tests in the same
 // order, the shading with its roundings spelled out, and the radiance added
 // up as the kernels of the wavefront add it (each unoccluded shadow ray, and
 // what the path itself gathered when it ends).
-// 8 blocks of 2 warps per SM at 128 registers (10: 3-10 % slower up to one
-// path per lane; 1-warp blocks the same); a finished lane takes the warp's
-// next path at once (waiting for 8 or 16 idle lanes: 2 and 14 % slower at
-// 160,000 paths).
-constexpr int kPathsBlock = 64, kPathsBlocksPerSm = 8;
+// 512 threads per SM at 128 registers; a finished lane takes the warp's next
+// path at once (waiting for 8 or 16 idle lanes: 2 and 14 % slower at 160,000
+// paths).
+constexpr int kPathsThreads = 512;  // per SM
+constexpr int paths_block(bool one_node) { return one_node ? 512 : 256; }
 
 // Paths of a wavefront at most that k_pt_paths renders: where both forms took
 // the same time on GB300 (1 sample per pixel, depth 8; wavefront / whole paths
-// in us).  One-node scenes, bound by issue: Cornell box 346 / 248 at 147,456
-// paths, 413 / 394 at 262,144; textured shapes 352 / 184 and 382 / 350 at
-// 331,776; quadrics 323 / 310 and 351 / 461 at 262,144.  Trees, whose
-// wavefront waits longer: sphere scene 582 / 491 at 262,144, 770 / 939 at
-// 589,824; sphere grid 437 / 293 at 147,456, 540 / 558 at 331,776; 20,480
-// triangles 1340 / 825 at 262,144, 1748 / 1522 at 589,824.
-uint32_t pt_paths_max(const DevScene& sc, int sms) { return (uint32_t)sms * (one_node(sc) ? 1024u : 2048u); }
+// in us).  Scenes with an infinite light, whose paths leave at different
+// depths: sphere scene 607 / 506 at 360,000 paths, 719 / 672 at 589,824, 832 /
+// 898 at 810,000; 20,480 triangles 1597 / 1522 and 1795 / 1926; quadrics
+// 406 / 403 and 455 / 552; sphere grid 560 / 423 at 455,400, 644 / 542 at
+// 679,800; textured shapes 352 / 193 at 331,776, 519 / 488 at 1,101,800.
+// Closed scenes, where all lanes stay busy: Cornell box 294 / 280 at 176,400,
+// 313 / 309 at 211,600, 410 / 462 at 360,000 (with spheres 379 / 344 there).
+uint32_t pt_paths_max(const DevScene& sc, int sms) {
+  return (uint32_t)sms * (sc.has_infinite ? 4096u : one_node(sc) ? 1536u : 2048u);
+}
 
 template <bool kOneNode>
-__global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
+__global__ void __launch_bounds__(paths_block(kOneNode), kPathsThreads / paths_block(kOneNode))
     k_pt_paths(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> g) {
   const uint32_t n = ch.npix * ch.layers;
   const int lane = threadIdx.x & 31;
@@ -473,7 +485,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
       cur += take;
       if (take) idle = 0;
     }
-    if (idle == 0xffffffffu && !more) break;
+    if (!__syncthreads_or(idle != 0xffffffffu || more)) break;
     // the shadow ray of the last step, then the path's ray
     Hit hit{-1.f, kNoHit, 0.f, 0.f};
     if constexpr (kOneNode) {
@@ -524,6 +536,7 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
         }
       }
     }
+    __syncthreads();
     if (shadow && !alive) P.Lout[path] = make_float4(Lo.x, Lo.y, Lo.z, 0.f);
     shadow = false;
     if (alive) {
@@ -552,9 +565,11 @@ __global__ void __launch_bounds__(kPathsBlock, kPathsBlocksPerSm)
 
 void launch_pt_paths(const DevScene& sc, const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int sms,
                      cudaStream_t st) {
-  const int grid = sms * kPathsBlocksPerSm;
-  if (one_node(sc)) k_pt_paths<true><<<grid, kPathsBlock, 0, st>>>(sc, film, P, ch, *sc.one);
-  else k_pt_paths<false><<<grid, kPathsBlock, 0, st>>>(sc, film, P, ch, NoGeom{});
+  auto run = [&](auto kernel, int block, auto geo) {
+    kernel<<<sms * (kPathsThreads / block), block, 0, st>>>(sc, film, P, ch, geo);
+  };
+  if (one_node(sc)) run(k_pt_paths<true>, paths_block(true), *sc.one);
+  else run(k_pt_paths<false>, paths_block(false), NoGeom{});
 }
 
 // ----------------------------------------------------------------- accumulate

@@ -8,18 +8,18 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 SMS = 152
-WARPS = SMS * 8 * 2
-SMALL = SMS * 640
+WARPS = SMS * 16
+SMALL = SMS * 1024
 
 
 def _scene(name):
     from gprt import scenes
     from gprt.scene import CameraConfig
-    s = {"boxes": lambda: scenes.cornell_boxes_bdpt(320),
-         "spot": lambda: scenes.spot_scene(270),
-         "spheres": lambda: scenes.default_style_scene(5, 321, 310),
-         "textures": lambda: scenes.texture_test_scene(CameraConfig(width=424)),
-         "mesh": lambda: scenes.icosphere_scene(level=3, width=320)}[name]()
+    s = {"boxes": lambda: scenes.cornell_boxes_bdpt(400),
+         "spot": lambda: scenes.spot_scene(340),
+         "spheres": lambda: scenes.default_style_scene(5, 401, 390),
+         "textures": lambda: scenes.texture_test_scene(CameraConfig(width=540)),
+         "mesh": lambda: scenes.icosphere_scene(level=3, width=400)}[name]()
     s.sampling.max_depth = 6
     s.sampling.adaptive_min_samples = 1.0
     return s

@@ -8,7 +8,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 SMS = 152
-WARPS = SMS * 8 * 2
+WARPS = SMS * 16
 
 
 def _film(g, spp, flags=0, chunk=0):
@@ -60,8 +60,8 @@ def test_films_equal_the_wavefronts(ctx, name, roulette):
 @pytest.mark.parametrize("name", ["cornell", "spheres"])
 def test_chunk_edges(ctx, name):
     from gprt import scenes
-    scene = scenes.cornell_baseline(400) if name == "cornell" else scenes.default_style_scene(5, 600, 530)
-    most = SMS * (1024 if name == "cornell" else 2048)
+    scene = scenes.cornell_baseline(490) if name == "cornell" else scenes.default_style_scene(5, 800, 790)
+    most = SMS * (1536 if name == "cornell" else 4096)
     _same(ctx, scene, (1,), [32 * WARPS - 1, 32 * WARPS + 1, most, most + 1])
 
 
