@@ -62,7 +62,7 @@ def test_chunk_edges(ctx, name):
     from gprt import scenes
     scene = scenes.cornell_baseline(490) if name == "cornell" else scenes.default_style_scene(5, 800, 790)
     most = SMS * (1536 if name == "cornell" else 4096)
-    _same(ctx, scene, (1,), [32 * WARPS - 1, 32 * WARPS + 1, most, most + 1])
+    _same(ctx, scene, (1,), [SMS * 256, SMS * 256 + 1, 32 * WARPS - 1, 32 * WARPS + 1, most, most + 1])
 
 
 @pytest.mark.parametrize("depth", [0, 1])
