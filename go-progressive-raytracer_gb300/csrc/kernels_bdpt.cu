@@ -1098,31 +1098,26 @@ __global__ void __launch_bounds__(kSubpathsBlock, kSubpathsBlocksPerSm)
   }
 }
 
-// Strategy k = s * MAXV + (t - 1) of a sample is evaluated when s <= nl and
-// t <= nc, except (1,1) (bdpt.go:300-301) and s = 0 with t != nc (the
-// path-tracing strategy contributes only at the full camera path).
-__device__ __forceinline__ bool has_strategy(int s, int t, int nc, int nl) {
-  return s <= nl && t <= nc && !(s == 1 && t == 1) && !(s == 0 && t != nc);
-}
-
-// A strategy the sample has whose contribution can be non-zero: listed for
-// the strategy kernels and summed.  The others return zero before drawing
-// any number, so leaving them out changes neither a sampler position
-// (draws_before) nor a sum: light tracing with a specular light vertex
-// (mask bit s clear), direct lighting at a specular or material-less camera
-// vertex or without lights (bit t clear), and a connection with either
+// The strategies (s, t) of a sample with s light vertices (s <= nl), as bits t:
+// strategy k = s * MAXV + (t - 1) is evaluated when s <= nl and t <= nc, except
+// (1,1) (bdpt.go:300-301) and s = 0 with t != nc (the path-tracing strategy
+// contributes only at the full camera path).  Of these, the ones left out here
+// return zero before drawing any number, so that changes neither a sampler
+// position (draws_before) nor a sum: light tracing with a specular light
+// vertex (mask bit s clear), direct lighting at a specular or material-less
+// camera vertex or without lights (bit t clear), and a connection with either
 // (bdpt.go:398-561).
-__device__ __forceinline__ bool listed_strategy(int s, int t, int nc, int nl, uint2 m) {
-  if (!has_strategy(s, t, nc, nl)) return false;
-  if (s == 0) return true;
-  bool ls = (m.x >> s) & 1u, ct = (m.y >> t) & 1u;
-  return t == 1 ? ls : s == 1 ? ct : ls && ct;
+__device__ __forceinline__ uint32_t strategy_row(int s, int nc, uint2 m) {
+  if (s == 0) return 1u << nc;
+  if (s == 1) return m.y;
+  return (m.x >> s) & 1u ? m.y | 2u : 0u;
 }
 
 // Lists, per strategy, the samples that have it, so that the strategy kernel
 // gives each warp 32 real (s, t, sample) items.  A block of 1,024 samples
 // counts each strategy's items in shared memory (one shared atomic per warp
-// and strategy), reserves its range of every list with one global atomic per
+// and row of strategies, lane t for strategy (s, t): 228 -> 137 us per 2^20
+// samples against one per strategy, whose answer lane 0 waited for), reserves its range of every list with one global atomic per
 // strategy, then writes the items: per-warp global atomics on the
 // (MAXV + 1) x MAXV list counters serialised in L2 (16.7 ms of a 200 ms
 // Cornell-boxes frame).  The order within a list does not matter: every
@@ -1149,26 +1144,34 @@ __global__ void __launch_bounds__(1024) k_bdpt_list(DevPaths PS, ChunkDesc ch) {
       nl = (int)(m >> 8);
       mk = B.masks[i];
     }
-    // a warp visits only the strategies its longest subpaths reach (both
-    // loops over the same range: wofs is written and read for those only)
-    const int wnc = __reduce_max_sync(0xFFFFFFFFu, nc), wnl = __reduce_max_sync(0xFFFFFFFFu, nl);
-    for (int s = 0; s <= wnl; s++)
-      for (int t = 1; t <= wnc; t++) {
-        const int k = s * MAXV + t - 1;
-        unsigned mask = __ballot_sync(0xFFFFFFFFu, listed_strategy(s, t, nc, nl, mk));
-        if (mask && lane == 0) wofs[wp][k] = (uint16_t)atomicAdd(&cnt[k], (uint32_t)__popc(mask));
+    // a warp visits only the strategies that some lane of it has, the same in
+    // both loops, so wofs is written and read for those only
+    const int wnl = __reduce_max_sync(0xFFFFFFFFu, nl);
+    for (int s = 0; s <= wnl; s++) {
+      const uint32_t mine = s <= nl ? strategy_row(s, nc, mk) : 0u;
+      const uint32_t all = __reduce_or_sync(0xFFFFFFFFu, mine);
+      uint32_t c = 0;  // lane t: the row's count of strategy t
+      for (uint32_t left = all; left; left &= left - 1u) {
+        const int t = __ffs(left) - 1;
+        const unsigned mask = __ballot_sync(0xFFFFFFFFu, (mine >> t) & 1u);
+        if (lane == t) c = __popc(mask);
       }
+      if (c) wofs[wp][s * MAXV + lane - 1] = (uint16_t)atomicAdd(&cnt[s * MAXV + lane - 1], c);
+    }
     __syncthreads();
     for (int k = threadIdx.x; k < K; k += blockDim.x)
       base[k] = cnt[k] ? w * kBdWindow + atomicAdd(B.scount + w * K + k, cnt[k]) : 0u;
     __syncthreads();
-    for (int s = 0; s <= wnl; s++)
-      for (int t = 1; t <= wnc; t++) {
-        const int k = s * MAXV + t - 1;
-        bool has = listed_strategy(s, t, nc, nl, mk);
-        unsigned mask = __ballot_sync(0xFFFFFFFFu, has);
+    for (int s = 0; s <= wnl; s++) {
+      const uint32_t mine = s <= nl ? strategy_row(s, nc, mk) : 0u;
+      const uint32_t all = __reduce_or_sync(0xFFFFFFFFu, mine);
+      for (uint32_t left = all; left; left &= left - 1u) {
+        const int t = __ffs(left) - 1, k = s * MAXV + t - 1;
+        const bool has = (mine >> t) & 1u;
+        const unsigned mask = __ballot_sync(0xFFFFFFFFu, has);
         if (has) B.slist[(size_t)k * B.ns + base[k] + wofs[wp][k] + __popc(mask & below)] = i;
       }
+    }
     __syncthreads();  // cnt, base and wofs are rewritten for the next range
   }
 }
@@ -1499,20 +1502,20 @@ __global__ void k_bdpt_sum(DevPaths PS, ChunkDesc ch) {
     const uint2 mk = B.masks[i];
     int nc = (int)(m.x & 0xFF), nl = (int)(m.x >> 8);
     float3 total = f3(0.f, 0.f, 0.f);
-    for (int s = 0; s <= nl; s++)
+    for (int s = 0; s <= nl; s++) {
+      const uint32_t row = strategy_row(s, nc, mk);  // the others contribute nothing: not evaluated
       for (int t0 = 1; t0 <= nc; t0 += 4) {
-        // four reads on their way at once, added in the reference's order
+        // four reads on their way at once, each of one strategy (the warp's are
+        // neighbours), added in the reference's order
         float4 c[4];
-        bool has[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-          has[k] = t0 + k <= nc && listed_strategy(s, t0 + k, nc, nl, mk);  // else contributes nothing: not evaluated
-          if (has[k]) c[k] = B.contrib[(size_t)(s * MAXV + t0 + k - 1) * n + i];
-        }
 #pragma unroll
         for (int k = 0; k < 4; k++)
-          if (has[k]) total += f3(c[k]);
+          if (row >> (t0 + k) & 1u) c[k] = B.contrib[(size_t)(s * MAXV + t0 + k - 1) * n + i];
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+          if (row >> (t0 + k) & 1u) total += f3(c[k]);
       }
+    }
     PS.Lout[i] = make_float4(total.x, total.y, total.z, 0.f);
   }
 }
