@@ -484,16 +484,6 @@ __device__ __forceinline__ void finish_sample(const DevBdpt& B, uint32_t p, int 
   B.masks[p] = make_uint2(light_mask << 2, cam_mask << 2);
 }
 
-// calculateMISWeight (bdpt_mis.go:13-181) over the stored subpaths
-// A vertex named by a pdf request: camera subpath vertex k (k >= 0), light
-// subpath vertex k (kLightV + k), the strategy's sampled vertex, or none.
-constexpr int kNoV = -1, kSampledV = -2, kLightV = 1024;
-
-__device__ __forceinline__ BVert fetch_vert(const SubpathRef& C, const SubpathRef& Lp, const BVert* sampled, int id) {
-  if (id == kSampledV) return *sampled;
-  return id >= kLightV ? Lp[id - kLightV] : C[id];
-}
-
 // The walk of calculateMISWeight (bdpt_mis.go:61-178) in prefix form, given
 // the reverse pdfs it recomputes next to the connection: cam1, cam2 of camera
 // vertices t - 1 and t - 2, lit1, lit2 of light vertices s - 1 and s - 2.
@@ -514,51 +504,54 @@ __device__ __forceinline__ float mis_walk(const SubpathRef& C, const SubpathRef&
   return 1.f / (1.f + sum);
 }
 
+// The two reverse pdfs at the end x of a connection to vertex o, whose subpath
+// comes from `own` (calculateVertexPdf, bdpt_mis.go:186-236): of x towards o
+// coming from own, and towards own coming from o.
+__device__ __forceinline__ void end_pdfs(const DevScene& sc, const BVert& x, const BVert& o, const BVert& own,
+                                         float& to_o, float& to_own) {
+  to_o = to_own = 0.f;
+  if (x.is(kFlagLight)) {
+#pragma unroll 1
+    for (int r = 0; r < 2; r++) {
+      float v = vertex_light_pdf(sc, x, r ? own : o);
+      if (r) to_own = v;
+      else to_o = v;
+    }
+    return;
+  }
+  float3 wo = o.p - x.p, wn = own.p - x.p;
+  if (x.mat >= 0 && dot(wo, wo) != 0.f && dot(wn, wn) != 0.f) {
+    wo = normalize(wo);
+    wn = normalize(wn);
+    const DevMaterial m = load_material(sc, x.mat);
+    bool d1, d2;
+    float p1 = mat_pdf(sc, m, wn, wo, x.n, d1), p2 = mat_pdf(sc, m, wo, wn, x.n, d2);
+    if (!d1) to_o = to_area(sc, x, o, p1);
+    if (!d2) to_own = to_area(sc, x, own, p2);
+  }
+}
+
+// calculateMISWeight (bdpt_mis.go:13-181) of a strategy of class 0, 1 or 2
+// whose stored vertex next to the connection is x: the reverse pdfs the walk
+// recomputes there (:61-105 camera side, :140-178 light side), each
+// calculateVertexPdf, or for s = 0 at t - 1 calculateLightOriginPdf.
 template <int CLS>
 __device__ __forceinline__ float mis_weight(const DevScene& sc, const SubpathRef& C, const SubpathRef& Lp,
-                                         const BVert* sampled, int s, int t) {
-  if (s + t == 2) return 1.f;
-  // The reverse pdfs the walk recomputes next to the connection
-  // (bdpt_mis.go:61-105 camera side, :140-178 light side): at most two per
-  // side, each calculateVertexPdf(cur, prev, next), or for s = 0 at t-1
-  // calculateLightOriginPdf(cur, next).  They are named by vertex ids and
-  // evaluated in one loop, so the pdf code is inlined once.
-  int rq[4][3];
-  int nq = 0;
-  int cam1 = -1, cam2 = -1, lit1 = -1, lit2 = -1;  // request of rev at t-1, t-2, s-1, s-2
-  const int c1 = t - 1, c2 = t - 2, l1 = kLightV + s - 1, l2 = kLightV + s - 2;
-  auto add = [&](int cur, int prev, int next) {
-    rq[nq][0] = cur;
-    rq[nq][1] = prev;
-    rq[nq][2] = next;
-    return nq++;
-  };
+                                            const BVert& x, const BVert& sampled, int s, int t) {
+  if (s + t <= 2) return 1.f;
+  float cam1 = 0.f, cam2 = 0.f, lit1 = 0.f, lit2 = 0.f;
   if (CLS == 0) {
-    if (t > 1) cam1 = add(c1, kNoV, c2);  // the light origin pdf
-    if (t > 2) cam2 = add(c1, kNoV, c2);
+    const BVert own = C[t - 2];
+    cam1 = light_origin_pdf(sc, x, own);
+    cam2 = vertex_pdf(sc, x, nullptr, own);
   } else if (CLS == 1) {
-    lit1 = add(kSampledV, kNoV, l1);
-    lit2 = add(l1, kSampledV, l2);
-  } else if (CLS == 2) {
-    cam1 = add(kSampledV, kNoV, c1);
-    cam2 = add(c1, kSampledV, c2);
-    lit1 = add(c1, c2, kSampledV);
+    lit1 = vertex_pdf(sc, sampled, nullptr, x);
+    lit2 = vertex_pdf(sc, x, &sampled, Lp[s - 2]);
+  } else {
+    cam1 = vertex_light_pdf(sc, sampled, x);
+    end_pdfs(sc, x, sampled, C[t - 2], lit1, cam2);
   }
-  float rv[4];
-  for (int q = 0; q < nq; q++) {
-    BVert cur = fetch_vert(C, Lp, sampled, rq[q][0]);
-    BVert next = fetch_vert(C, Lp, sampled, rq[q][2]);
-    if (CLS == 0 && q == cam1) {
-      rv[q] = light_origin_pdf(sc, cur, next);
-    } else {
-      BVert prev;
-      bool hp = rq[q][1] != kNoV;
-      if (hp) prev = fetch_vert(C, Lp, sampled, rq[q][1]);
-      rv[q] = vertex_pdf(sc, cur, hp ? &prev : nullptr, next);
-    }
-  }
-  return mis_walk<CLS>(C, Lp, sampled ? sampled->fwd : 0.f, s, t, cam1 >= 0 ? rv[cam1] : 0.f,
-                       cam2 >= 0 ? rv[cam2] : 0.f, lit1 >= 0 ? rv[lit1] : 0.f, lit2 >= 0 ? rv[lit2] : 0.f);
+  return mis_walk<CLS>(C, Lp, CLS == 2 ? sampled.fwd : 0.f, s, t, cam1, cam2, lit1, lit2);
 }
 
 // Uniform numbers the strategies before (s, t) draw, in the reference's
@@ -583,7 +576,7 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
   SubpathRef C{&B, i, 0}, Lp{&B, i, B.maxv};
   float3 Lc = zero;
   BVert sampled;
-  bool has = false, splat = false;
+  bool splat = false;
   int spx = 0, spy = 0;
   bool test = false;
   float3 ro = zero, rd = f3(0.f, 0.f, 1.f);
@@ -630,7 +623,6 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
     sampled.light = -1;
     sampled.prim = kNoHit;
     sampled.flags = kFlagCamera;
-    has = true;
     splat = true;
     Lc = c;
   } else {
@@ -666,7 +658,6 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
     sampled.flags = kFlagLight | (inf ? kFlagInfinite : 0);
     sampled.beta = lb;
     sampled.Le = ls.emission;
-    has = true;
     Lc = c;
   }
   if (test && occluded<kOneNode>(sc, geo, ro, rd, rt, rskip, err)) return zero;
@@ -678,7 +669,7 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
     sampled.rev = total_light_pdf(sc, sampled.p, sampled.n, normalize(Lp[s - 1].p - sampled.p));
   }
   if (is_zero(Lc) && !splat) return zero;
-  float w = mis_weight<CLS>(sc, C, Lp, has ? &sampled : nullptr, s, t);
+  const float w = mis_weight<CLS>(sc, C, Lp, CLS == 1 ? Lp[s - 1] : C[t - 1], sampled, s, t);
   if (splat) {
     float3 c = Lc * w;
     float4* dst = film.splat + (size_t)spy * film.width + spx;
@@ -1355,28 +1346,8 @@ __device__ __forceinline__ float3 connection_value(const DevScene& sc, const Dev
     const BVert x = get_vert(B, kx, i), o = get_vert(B, ko, i), own = get_vert(B, kx - 1, i);
     const Connection c = connect(q ? o.p : x.p, q ? x.p : o.p);
     const float3 f = vertex_brdf(sc, x, q ? c.d : -c.d, q == 1);
-    float to_o, to_own;  // the pdfs of x towards o (coming from own) and towards own (coming from o)
-    if (x.is(kFlagLight)) {
-      to_o = to_own = 0.f;
-#pragma unroll 1
-      for (int r = 0; r < 2; r++) {
-        float v = vertex_light_pdf(sc, x, r ? own : o);
-        if (r) to_own = v;
-        else to_o = v;
-      }
-    } else {
-      to_o = to_own = 0.f;
-      float3 wo = o.p - x.p, wn = own.p - x.p;
-      if (x.mat >= 0 && dot(wo, wo) != 0.f && dot(wn, wn) != 0.f) {
-        wo = normalize(wo);
-        wn = normalize(wn);
-        const DevMaterial m = load_material(sc, x.mat);
-        bool d1, d2;
-        float p1 = mat_pdf(sc, m, wn, wo, x.n, d1), p2 = mat_pdf(sc, m, wo, wn, x.n, d2);
-        if (!d1) to_o = to_area(sc, x, o, p1);
-        if (!d2) to_own = to_area(sc, x, own, p2);
-      }
-    }
+    float to_o, to_own;
+    end_pdfs(sc, x, o, own, to_o, to_own);
     dist = c.dist;
     if (q) {
       bc = f;
