@@ -207,15 +207,13 @@ def l2_fraction(achieved, torch):
             "l2_peak_how": "torch bf16 copy over 2 x 40 MB (L2-resident), 64 copies per CUDA graph, best of 5"}
 
 
-# Path-state bytes of one shading step (the SoA queues of the wavefront):
-# a shaded path reads ray origin, direction, hit, weight, roulette
-# throughput, radiance and ids (7 x 16 B), except at bounce 0 (one shaded
-# path per sample), where weight, throughput and radiance are implied
-# (4 x 16 B); a
-# continuing path writes all but the hit to the next queue (6 x 16 B); a
+# Path-state bytes of one shading step (the queues of the wavefront): a shaded
+# path reads its ray (32 B), its weight and ids (32 B) and its hit (16 B); a
+# continuing path writes ray, weight and ids to the next queue (64 B); a
 # finished path writes its radiance (16 B); a shadow ray writes origin,
-# direction, contribution (3 x 16 B) and its BVH root (4 B).
-SHADE_READ_B, SHADE_BOUNCE0_B, SHADE_CONT_B, SHADE_DONE_B, SHADE_SHADOW_B = 112, 64, 96, 16, 52
+# direction, contribution (3 x 16 B) and its BVH root (4 B).  The roulette
+# throughput (16 B each way, in scenes with Russian roulette) is not counted.
+SHADE_READ_B, SHADE_BOUNCE0_B, SHADE_CONT_B, SHADE_DONE_B, SHADE_SHADOW_B = 80, 80, 64, 16, 52
 
 
 def shade_roofline(cnt, kc, kc_batches, samples, peak, peak_kind, timing_source):
@@ -989,7 +987,7 @@ def run_gprt(args):
                 "warmup": args.warmup, "ms_per_step": ms / args.steps, "higher_is_better": True, "scaling": "weak",
                 "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded scenes, no dataset)",
                 "config": {"workload": WORKLOAD, "jobs": NJOBS, "samples_per_step": samples_per_step,
-                           "l2": "flushed (512 MB write before every timed step); path state 4.6 GB > L2",
+                           "l2": "flushed (512 MB write before every timed step); path state 4.1 GB > L2",
                            "parallelism": "replicas" if world > 1 else "single GPU",
                            "autotuned": {"step_paths": tune["chunk_paths"], "block_size": tune["block_size"],
                                          "simple_extend": bool(tune["flags"] & capi.JOB_SIMPLE_EXTEND),

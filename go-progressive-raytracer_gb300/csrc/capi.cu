@@ -621,8 +621,8 @@ int gprt_job_create(gprt_scene* s, const gprt_job_desc* desc, gprt_job** out) {
   uint32_t npix = s->host.sampling.width * s->host.sampling.height;
   if (d.chunk_paths == 0) {
     uint64_t want = (uint64_t)npix * std::max(1u, d.max_samples_per_pixel);
-    // path tracing: up to 2^24 paths per wavefront (about 4.6 GB of path
-    // state); BDPT: 2^20 samples per chunk (3.5 GB of vertices and strategy
+    // path tracing: up to 2^24 paths per wavefront (about 4.1 GB of path
+    // state); BDPT: 2^20 samples per chunk (3.4 GB of vertices and strategy
     // contributions at depth <= 9, 8.4 GB up to depth 17)
     d.chunk_paths = (uint32_t)std::min<uint64_t>(want, d.integrator == GPRT_INTEGRATOR_BDPT ? (1u << 20) : (1u << 24));
   }
@@ -886,7 +886,7 @@ namespace {
 
 constexpr size_t kNoAllocPaths = GPRT_NOALLOC_MAX_PATHS;
 // the path state of kNoAllocPaths paths (two compacted queues of ray, weight,
-// throughput, radiance and sampler ids; hits; origin radiance; shadow rays)
+// sampler ids and throughput; hits; origin radiance; shadow rays; slot order)
 constexpr size_t kNoAllocBytes = path_region_bytes((uint32_t)kNoAllocPaths, false);
 
 __device__ __align__(256) static unsigned char g_noalloc_scratch[kNoAllocBytes];

@@ -26,7 +26,9 @@
 //                      samples, the samples that have it;
 //   k_bdpt_prefix      each strategy class's prefix sums of the list counts
 //                      in (window, strategy) order;
-//   k_bdpt_strategies  one thread per listed (strategy, sample) item, in
+//   k_bdpt_strategies  (small chunks: k_bdpt_strategies_all, one launch for the
+//                      four classes; connections by run_connections, in three
+//                      steps) one thread per listed (strategy, sample) item, in
 //                      (window, strategy) order, so every strategy of a
 //                      window runs while its vertices are in L2; the
 //                      items of a strategy in consecutive threads: each warp

@@ -420,7 +420,7 @@ int gprt_autotune(gprt_scene* scene, const gprt_job_desc* base, uint32_t spp, gp
  * takes) and writes the per-pixel mean radiance, 3 floats per pixel
  * (PixelStats.GetColor), into the caller's DEVICE buffer `rgb_out`.  The
  * path state lives in one statically sized device array inside the library
- * (GPRT_NOALLOC_MAX_PATHS paths, about 34 MB, held by every GPU that loads
+ * (GPRT_NOALLOC_MAX_PATHS paths, about 32 MB, held by every GPU that loads
  * the library until the process exits); requests with
  * width * height * spp > GPRT_NOALLOC_MAX_PATHS return GPRT_E_INVALID.  It
  * calls no cudaMalloc or cudaFree.  The first call through a context looks
