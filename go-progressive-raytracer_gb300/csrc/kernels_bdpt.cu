@@ -1015,7 +1015,7 @@ __global__ void __launch_bounds__(128, 4) k_bdpt_extend(DevScene sc, DevPaths PS
 // a sample from its camera ray to the end of its light subpath, with the state
 // between bounces in registers.  The wavefront's 2 x max_depth pairs of
 // launches each take a ray's or a shading step's chain of latencies, 8 and 22
-// us, on any number of samples (34,000 samples of the spot scene: 480 us a
+// us, on any number of samples (49,000 samples of the spot scene: 480 us a
 // frame, 371 so).  What is left is bound by fetching instructions, so the
 // warps of a block trace together and extend together and share them (two
 // barriers a bounce; the same frame, after other changes: 64-thread blocks

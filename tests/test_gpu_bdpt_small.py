@@ -12,7 +12,7 @@ WARPS = SMS * 16
 SMALL = SMS * 1024
 
 
-def _scene(name):
+def _scene(name, depth):
     from gprt import scenes
     from gprt.scene import CameraConfig
     s = {"boxes": lambda: scenes.cornell_boxes_bdpt(400),
@@ -20,15 +20,16 @@ def _scene(name):
          "spheres": lambda: scenes.default_style_scene(5, 401, 390),
          "textures": lambda: scenes.texture_test_scene(CameraConfig(width=540)),
          "mesh": lambda: scenes.icosphere_scene(level=3, width=400)}[name]()
-    s.sampling.max_depth = 6
+    s.sampling.max_depth = depth
     s.sampling.adaptive_min_samples = 1.0
     return s
 
 
-@pytest.mark.parametrize("name", ["boxes", "spot", "spheres", "textures", "mesh"])
-def test_small_chunks_equal_the_wavefronts(ctx, name):
+@pytest.mark.parametrize("name,depth", [("boxes", 6), ("spot", 6), ("spheres", 6), ("textures", 6), ("mesh", 6),
+                                        ("boxes", 1), ("spheres", 1), ("boxes", 17), ("spheres", 12)])
+def test_small_chunks_equal_the_wavefronts(ctx, name, depth):
     import gprt
-    g = gprt.GpuScene(ctx, _scene(name))
+    g = gprt.GpuScene(ctx, _scene(name, depth))
     assert g.width * g.height > SMALL  # one chunk of all pixels takes the wavefront
 
     def film(chunk):
