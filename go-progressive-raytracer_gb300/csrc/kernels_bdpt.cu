@@ -1504,7 +1504,7 @@ void launch_bdpt_maxv(const DevScene& sc, const DevFilm& film, const DevPaths& P
   const int g2 = std::max(1, sms * 16);
   const int g3 = launch_grid(n, 256, 0);
   const int gl = std::min(launch_grid(n, 1024, 0), std::max(1, sms * 2));
-  const bool small = n <= (uint32_t)sms * kSmallBdptPerSm && sc.max_depth > 0;
+  const bool small = n <= (uint32_t)sms * kSmallBdptPerSm;
   if (small) {
     k_bdpt_subpaths<MAXV, kOneNode><<<sms * kSubpathsBlocksPerSm, kSubpathsBlock, 0, st>>>(sc, film, P, ch, geo);
   } else {
@@ -1540,6 +1540,13 @@ void launch_bdpt_maxv(const DevScene& sc, const DevFilm& film, const DevPaths& P
 void launch_bdpt(const DevScene& sc, const DevFilm& film, const DevPaths& P, const ChunkDesc& ch, int block,
                  cudaStream_t st) {
   (void)block;
+  if (sc.max_depth <= 0) {
+    // No ray leaves the camera: the one strategy with a camera subpath of its
+    // single vertex sees no emission.  The kernels below take at least one
+    // bounce to have written each sample's record (meta, masks).
+    cudaMemsetAsync(P.Lout, 0, (size_t)ch.npix * ch.layers * sizeof(float4), st);
+    return;
+  }
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
