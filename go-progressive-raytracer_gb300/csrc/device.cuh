@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "deal.h"
 #include "layout.h"
 
 namespace gprt {
@@ -900,9 +901,9 @@ __device__ __forceinline__ bool trace(const DevScene& sc, const Geom<kOneNode>& 
 template <bool kAnyHit, bool kCount, class Source>
 __device__ __forceinline__ void trace_batch_one_node(const OneNode& g, Source& src, TraceStats* st, uint32_t* traced) {
   const uint32_t n = src.count();
-  for (uint32_t base = blockIdx.x * blockDim.x; base < n; base += gridDim.x * blockDim.x) {
-    const uint32_t i = base + threadIdx.x;
-    const bool live = i < n;
+  deal_blocks(n, blockIdx.x * blockDim.x, gridDim.x * blockDim.x, [&](uint64_t base) {
+    const bool live = base + threadIdx.x < n;
+    const uint32_t i = (uint32_t)base + threadIdx.x;
     float3 o = f3(0.f, 0.f, 0.f), d = f3(0.f, 0.f, 1.f);
     float tmin = 0.f, tmax = 0.f;
     uint32_t skip = kNoHit;
@@ -914,7 +915,7 @@ __device__ __forceinline__ void trace_batch_one_node(const OneNode& g, Source& s
       src.store(i, h);
       if (kCount) (*traced)++;
     }
-  }
+  });
 }
 
 // The step of a warp whose lanes `busy` are on a ray and `testing` wait for a
@@ -942,6 +943,7 @@ __device__ __forceinline__ bool trav_test_now(unsigned testing, unsigned busy) {
 // load(i, o, d, tmin, tmax, skip, root) and store(i, hit); store() sees the
 // marker hit of a ray that overflowed its stack and reports it.
 constexpr uint32_t kFetchChunk = 64;
+constexpr uint32_t kNoRay = 0xffffffffu;  // no ray in a batch has this number
 constexpr int kRefillIdle = 16;
 // 128-thread blocks per SM of the traversal kernels: 64 registers, 40 bytes
 // spilled; 7 blocks (72 registers) and 6 (80) measured 2 % and 6 % slower on
@@ -955,16 +957,16 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   const uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t chunk = min(kFetchChunk, (n + nw - 1) / nw);
+  const uint32_t chunk = deal_chunk(n, nw, kFetchChunk);
   // the warp's current chunk [cur, end), warp-uniform
-  uint32_t cur = min((uint64_t)n, (uint64_t)w * chunk), end = min((uint64_t)n, (uint64_t)cur + chunk);
+  uint32_t cur = deal_at(n, (uint64_t)w * chunk), end = deal_at(n, (uint64_t)cur + chunk);
   bool more = cur < end;  // the warp may still draw rays
   uint32_t next = w;      // without `work`: the chunk it holds
   Trav s;
   TravEntry stack[kTraceStack];
-  int ray = -1;
+  uint32_t ray = kNoRay;
   for (;;) {
-    const bool idle = ray < 0, testing = !idle && s.testing();
+    const bool idle = ray == kNoRay, testing = !idle && s.testing();
     const unsigned idle_mask = __ballot_sync(0xffffffffu, idle), test_mask = __ballot_sync(0xffffffffu, testing);
     if (more && __popc(idle_mask) >= kRefillIdle) {
       if (cur == end) {
@@ -977,8 +979,8 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
           next += nw;
           at = (uint64_t)next * chunk;
         }
-        cur = (uint32_t)min((uint64_t)n, at);
-        end = (uint32_t)min((uint64_t)n, at + chunk);
+        cur = deal_at(n, at);
+        end = deal_at(n, at + chunk);
       }
       if (cur == end) {
         more = false;
@@ -993,7 +995,7 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
           uint32_t mine = cur + rank;
           src.load(mine, o, d, tmin, tmax, skip, root);
           trav_init(s, o, d, tmin, tmax, skip, root, stack);
-          ray = (int)mine;
+          ray = mine;
           if (kCount) (*traced)++;
         }
         cur += take;
@@ -1007,8 +1009,8 @@ __device__ __forceinline__ void trace_persistent(const DevScene& sc, Source& src
       trav_visit<kCount>(sc, s, stack, st);
     }
     if (!idle && s.done()) {
-      src.store((uint32_t)ray, s.result());
-      ray = -1;
+      src.store(ray, s.result());
+      ray = kNoRay;
     }
   }
 }

@@ -20,7 +20,7 @@
 namespace gprt {
 
 int launch_grid(uint32_t n, int block, int max_blocks) {
-  uint32_t g = (n + block - 1) / block;
+  uint32_t g = n / (uint32_t)block + (n % (uint32_t)block != 0);
   if (g < 1) g = 1;
   if (max_blocks > 0 && g > (uint32_t)max_blocks) g = (uint32_t)max_blocks;
   return (int)g;
@@ -69,7 +69,7 @@ void launch_intersect(const DevScene& sc, const gprt_ray* rays, uint32_t n, bool
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  int grid = launch_grid((n + 31) / 32 * 32, 128, persistent_grid(sms, 128));
+  int grid = launch_grid(n, 128, persistent_grid(sms, 128));
   BatchSource src{rays, hits, n, sc.root, err};
   if (one_node(sc)) (any_hit ? k_intersect<true, true> : k_intersect<false, true>)<<<grid, 128, 0, st>>>(sc, src, *sc.one);
   else (any_hit ? k_intersect<true, false> : k_intersect<false, false>)<<<grid, 128, 0, st>>>(sc, src, NoGeom{});
