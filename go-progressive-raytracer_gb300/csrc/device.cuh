@@ -636,6 +636,53 @@ __device__ __forceinline__ void trav_pop(Trav& s, const TravEntry* stack) {
   s.node = node;
 }
 
+// The first leaf of the node just visited, whose box was tested there.
+__device__ __forceinline__ void trav_first_leaf(const DevScene& sc, Trav& s) {
+  const int i = __ffs(s.leaves) - 1;
+  s.leaves &= s.leaves - 1;
+  const int2 rm = __ldg(reinterpret_cast<const int2*>(sc.nodes + (size_t)s.lnode * 8 + 2 * i + 1) + 1);
+  s.prim = rm.x;
+  s.end = rm.x + (rm.y & kLeafCountMask);
+  s.type = (rm.y >> kLeafTypeShift) & 3;
+}
+
+// A ray that has met something at a distance which is not a number (the ray or
+// the primitive is not one either): no node is known to be near enough then, so
+// the children of `lnode`, whose leaves it has tested, are taken off the stack
+// (they are its top entries), and it tests only the leaves of the nodes below
+// them there, instead of visiting every node that those lead to.  A node is
+// visited in full if a hit in its leaves is at a distance again.
+__device__ __forceinline__ void trav_leaves_only(const DevScene& sc, Trav& s, const TravEntry* stack) {
+  bool left = true;  // the top entry may be a child of lnode
+  while (s.sp > 0 && stack[s.sp - 1].node >= 0) {  // negative: the sentinel of trav_init
+    const int node = stack[s.sp - 1].node, from = left ? s.lnode : node;
+    bool child = false;
+    s.leaves = 0;
+#pragma unroll 1
+    for (int i = 0; i < 4; i++) {
+      const ChildRec c = ldg_child(sc.nodes + (size_t)from * 8 + 2 * i);
+      if (c.ref() == kEmptyChild) break;
+      float tn, tf;
+      child_span(s.inv, s.nood, s.tmin, c, tn, tf);
+      if (c.meta() == 0) child |= c.ref() == node;
+      else if (!(tn > tf)) s.leaves |= 1u << i;
+    }
+    if (left && !child) {
+      left = false;
+      continue;
+    }
+    s.sp--;
+    if (!left && s.leaves) {
+      s.node = s.lnode = node;
+      s.node_t = -kInfF;
+      trav_first_leaf(sc, s);
+      return;
+    }
+  }
+  s.leaves = 0;
+  s.node = -1;
+}
+
 // The ray's next leaf of node `lnode`, or, when none is left, its next node.
 // A leaf whose box starts behind a hit in a leaf before it is left out.
 __device__ __forceinline__ void trav_next_leaf(const DevScene& sc, Trav& s, const TravEntry* stack) {
@@ -651,7 +698,10 @@ __device__ __forceinline__ void trav_next_leaf(const DevScene& sc, Trav& s, cons
     s.type = (c.meta() >> kLeafTypeShift) & 3;
     return;
   }
-  if (s.node == kPopNext || s.node_t > s.best) trav_pop(s, stack);
+  if (s.node == kPopNext || !(s.node_t <= s.best)) {
+    if (s.best == s.best) trav_pop(s, stack);
+    else trav_leaves_only(sc, s, stack);
+  }
 }
 
 // The ray (o, d) against the record R (read through `ld`) of a primitive of
@@ -703,16 +753,6 @@ __device__ __forceinline__ bool hit_prim(const DevScene& sc, int type, int p, fl
   }
   gid = sc.quadric_base + (uint32_t)p;
   return hit_record(kPrimQuadric, sc.quadrics + (size_t)p * 5, ld, o, d, tmin, best, skip, gid, t, u, v);
-}
-
-// The first leaf of the node just visited, whose box was tested there.
-__device__ __forceinline__ void trav_first_leaf(const DevScene& sc, Trav& s) {
-  const int i = __ffs(s.leaves) - 1;
-  s.leaves &= s.leaves - 1;
-  const int2 rm = __ldg(reinterpret_cast<const int2*>(sc.nodes + (size_t)s.lnode * 8 + 2 * i + 1) + 1);
-  s.prim = rm.x;
-  s.end = rm.x + (rm.y & kLeafCountMask);
-  s.type = (rm.y >> kLeafTypeShift) & 3;
 }
 
 // Tests the ray against primitive `prim` of its leaf and moves on: to the
