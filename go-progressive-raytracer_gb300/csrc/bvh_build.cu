@@ -450,7 +450,7 @@ int device_build_bvh(gprt_ctx* ctx, HostScene& h, DevScene& d, std::vector<void*
   }
   for (size_t i = 0; i < h.lights.size() && i < bp.light_prim.size(); i++)
     if (bp.light_prim[i] >= 0) h.lights[i].prim = (int)fi[bp.light_prim[i]];
-  h.bvh_depth = levels;
+  h.bvh_depth = levels - 1;
   d.nodes = nodes;
   d.tris = tris;
   d.tri_normals = normals;

@@ -442,6 +442,17 @@ int gprt_scene_create(gprt_ctx* ctx, const gprt_scene_desc* desc, gprt_scene** o
     if (h.custom_normals && h.n_tris)
       CK(ctx, cudaMemcpyAsync(const_cast<float4*>(d.tri_normals), h.tri_normals.data(), h.tri_normals.size() * 16,
                               cudaMemcpyHostToDevice, ctx->stream));
+    const size_t node_bytes = h.nodes.size() * sizeof(float4);
+    if (fit_stack(h)) {
+      s->buffers.erase(std::find(s->buffers.begin(), s->buffers.end(), (void*)d.nodes));
+      cudaFree((void*)d.nodes);
+      s->bytes -= node_bytes;
+      rc = upload(ctx, s->buffers, h.nodes, &d.nodes, &s->bytes);
+      if (rc) {
+        free_all(s->buffers);
+        return rc;
+      }
+    }
     // the tree is checked on the host copy before any kernel walks it
     auto tc = std::chrono::steady_clock::now();
     std::string bad = validate_layout(h);
@@ -452,6 +463,7 @@ int gprt_scene_create(gprt_ctx* ctx, const gprt_scene_desc* desc, gprt_scene** o
       return fail(ctx, GPRT_E_DEVICE, "device BVH build produced an invalid tree: " + bad);
     }
   } else {
+    fit_stack(h);
     rc = upload_geometry(ctx, s.get());
     if (rc) {
       free_all(s->buffers);

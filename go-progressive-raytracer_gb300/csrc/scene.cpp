@@ -1113,6 +1113,93 @@ void apply_mesh_options(const gprt_scene_desc* d, HostScene& h) {
   });
 }
 
+namespace {
+NodeChild child_at(const std::vector<float4>& nodes, size_t node, int i) {
+  NodeChild c;
+  std::memcpy(&c, &nodes[node * 8 + 2 * i], sizeof(c));
+  return c;
+}
+}  // namespace
+
+// The traversal pushes all farther children of a node that a ray meets, and
+// tests the node's leaves afterwards: children behind a hit in those leaves
+// take room on the stack until they are popped.  A tree whose rays could
+// overflow the stack (`need`: per node, one entry less than its internal
+// children, along the path where these add up to most) gets the leaves of such
+// nodes separated from their internal children, which move into a node of
+// their own behind them: it is reached after the leaves, so only children
+// still nearer than the hit are pushed.  The primitives are tested in the same
+// order.  Only trees of more than 22 levels can need it (1.3 M triangles have 12
+// and need 32 entries), so it is done here: room made in the visit itself cost
+// other trees up to 4 % (any hit of 300,007 rays on 81,920 triangles 80.2 ->
+// 83.2 us, the frame of 1.3 M triangles 20.6 -> 21.4 ms).
+bool fit_stack(HostScene& h) {
+  const int room = h.test_stack_cap ? kTestStackCap : kTraceStack;
+  const size_t n = h.nodes.size() / 8;
+  if (n < 2 || 3 * (int64_t)h.bvh_depth <= room) return false;
+  std::vector<int> need(n, 0);
+  for (size_t k = n; k-- > 0;) {  // children come after their parents
+    int inner = 0, below = 0;
+    for (int i = 0; i < 4; i++) {
+      const NodeChild c = child_at(h.nodes, k, i);
+      if (c.ref == kEmptyChild || c.meta != 0) continue;
+      inner++;
+      below = std::max(below, need[(size_t)c.ref]);
+    }
+    need[k] = std::max(0, inner - 1) + below;
+  }
+  if (need[0] <= room) return false;
+  const NodeChild empty = {{1e30f, -1e30f}, {1e30f, -1e30f}, {1e30f, -1e30f}, kEmptyChild, 0};
+  std::vector<NodeChild> out(4, empty);
+  std::vector<std::pair<int, int>> todo = {{0, 0}};  // node, its place in `out`
+  auto place = [&](int node) {
+    const int at = (int)(out.size() / 4);
+    out.resize(out.size() + 4, empty);
+    if (node >= 0) todo.push_back({node, at});
+    return at;
+  };
+  bool changed = false;
+  while (!todo.empty()) {
+    const auto [node, at] = todo.back();
+    todo.pop_back();
+    NodeChild leaf[4], inner[4];
+    int nl = 0, ni = 0;
+    for (int i = 0; i < 4; i++) {
+      const NodeChild c = child_at(h.nodes, (size_t)node, i);
+      if (c.ref != kEmptyChild) (c.meta != 0 ? leaf[nl++] : inner[ni++]) = c;
+    }
+    if (nl == 0 || ni < 2) {
+      for (int i = 0; i < 4; i++) {
+        NodeChild c = child_at(h.nodes, (size_t)node, i);
+        if (c.ref != kEmptyChild && c.meta == 0) c.ref = place(c.ref);
+        out[(size_t)at * 4 + i] = c;
+      }
+      continue;
+    }
+    NodeChild rest = inner[0];  // the box around the internal children
+    for (int i = 1; i < ni; i++) {
+      float* lohi[3] = {rest.x, rest.y, rest.z};
+      const float* c[3] = {inner[i].x, inner[i].y, inner[i].z};
+      for (int k = 0; k < 3; k++) {
+        lohi[k][0] = std::min(lohi[k][0], c[k][0]);
+        lohi[k][1] = std::max(lohi[k][1], c[k][1]);
+      }
+    }
+    rest.ref = place(-1);
+    for (int i = 0; i < nl; i++) out[(size_t)at * 4 + i] = leaf[i];
+    out[(size_t)at * 4 + nl] = rest;
+    for (int i = 0; i < ni; i++) {
+      inner[i].ref = place(inner[i].ref);
+      out[(size_t)rest.ref * 4 + i] = inner[i];
+    }
+    changed = true;
+  }
+  if (!changed) return false;
+  h.nodes.resize(out.size() * 2);
+  std::memcpy(h.nodes.data(), out.data(), out.size() * sizeof(NodeChild));
+  return true;
+}
+
 std::string validate_layout(const HostScene& s) {
   size_t nn = s.nodes.size() / 8;
   if (nn == 0) return (s.n_tris + s.n_quads + s.n_spheres + s.n_quadrics) ? "primitives without a BVH" : "";
@@ -1126,11 +1213,7 @@ std::string validate_layout(const HostScene& s) {
   for (size_t k = 0; k < nn; k++) nseen[k].store(0, std::memory_order_relaxed);
   std::mutex mu;
   std::string first_err;
-  auto child_of = [&](size_t n, int i) {
-    NodeChild c;
-    std::memcpy(&c, &s.nodes[n * 8 + 2 * i], sizeof(c));
-    return c;
-  };
+  auto child_of = [&](size_t n, int i) { return child_at(s.nodes, n, i); };
   parallel_for(nn, [&](size_t b0, size_t b1) {
     auto bad = [&](const char* m) {
       std::lock_guard<std::mutex> g(mu);

@@ -37,7 +37,7 @@ struct HostScene {
   double world_radius = 0;
   DevCamera cam{};
   gprt_sampling_desc sampling{};
-  int bvh_depth = 0;
+  int bvh_depth = 0;  // of the deepest node, the root's being 0
   double build_ms = 0, flatten_ms = 0, bvh_ms = 0, check_ms = 0;
   bool device_bvh = false;  // the BVH and primitive arrays are built on the GPU from `pending`
   bool test_stack_cap = false;  // GPRT_BUILD_TEST_STACK_CAP: rays get kTestStackCap stack entries
@@ -55,6 +55,11 @@ bool build_scene(const gprt_scene_desc* desc, HostScene& out, std::string& err, 
 // final triangle id through the primitive maps (either builder): patches
 // tri_normals and fills tri_uvs.
 void apply_mesh_options(const gprt_scene_desc* desc, HostScene& h);
+
+// Makes the tree fit traversal stacks of the size that its rays get
+// (kTraceStack, or kTestStackCap with test_stack_cap) as far as the order of
+// the traversal allows; returns whether it changed the nodes.
+bool fit_stack(HostScene& h);
 
 // Checks the layout invariants of a built scene; returns "" when valid.
 std::string validate_layout(const HostScene& s);
