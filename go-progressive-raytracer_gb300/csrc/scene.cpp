@@ -1392,20 +1392,25 @@ void count_traversal(const HostScene& s, const gprt_ray* rays, uint32_t n, bool 
       inv[k] = 1.0f / dd;
       ood[k] = o[k] * inv[k];
     }
-    std::vector<int> stack;
+    std::vector<std::pair<int, float>> stack;  // node, distance at which the ray enters its box
     int node = 0;
     float best = ray.tmax;
     bool done = false;
+    auto pop = [&]() {  // the nearest entry that is not behind the hit
+      node = -1;
+      while (!stack.empty() && node < 0) {
+        if (!(stack.back().second > best)) node = stack.back().first;
+        stack.pop_back();
+      }
+    };
     while (node >= 0 && !done) {
       nodes++;
-      int ich[4];
-      float itn[4];
-      int nint = 0;
-      for (int i = 0; i < 4 && !done; i++) {
-        NodeChild c;
-        std::memcpy(&c, &s.nodes[(size_t)node * 8 + 2 * i], sizeof(c));
-        const int ch = c.ref, mt = c.meta;
-        if (ch == kEmptyChild) break;
+      int ich[4], leaf[4];
+      float itn[4], ltn[4];
+      int nint = 0, nleaf = 0;
+      for (int i = 0; i < 4; i++) {
+        const NodeChild c = child_at(s.nodes, (size_t)node, i);
+        if (c.ref == kEmptyChild) break;
         boxes++;
         float t0[3], t1[3];
         for (int k = 0; k < 3; k++) {
@@ -1418,17 +1423,25 @@ void count_traversal(const HostScene& s, const gprt_ray* rays, uint32_t n, bool 
         float tn = std::max(std::max(t0[0], t0[1]), std::max(t0[2], ray.tmin));
         float tf = std::min(std::min(t1[0], t1[1]), std::min(t1[2], best));
         if (tn > tf) continue;
-        if (mt == 0) {
-          int k = nint++;
-          while (k > 0 && itn[k - 1] > tn) {
-            itn[k] = itn[k - 1];
-            ich[k] = ich[k - 1];
-            k--;
-          }
-          itn[k] = tn;
-          ich[k] = ch;
+        if (c.meta != 0) {
+          ltn[nleaf] = tn;
+          leaf[nleaf++] = i;
           continue;
         }
+        int k = nint++;
+        while (k > 0 && itn[k - 1] > tn) {
+          itn[k] = itn[k - 1];
+          ich[k] = ich[k - 1];
+          k--;
+        }
+        itn[k] = tn;
+        ich[k] = c.ref;
+      }
+      for (int k = nint - 1; k >= 1; k--) stack.push_back({ich[k], itn[k]});
+      for (int l = 0; l < nleaf && !done; l++) {
+        if (ltn[l] > best) continue;
+        const NodeChild c = child_at(s.nodes, (size_t)node, leaf[l]);
+        const int ch = c.ref, mt = c.meta;
         int cnt = mt & kLeafCountMask, type = (mt >> kLeafTypeShift) & 3;
         for (int k = 0; k < cnt; k++) {
           prims++;
@@ -1483,22 +1496,8 @@ void count_traversal(const HostScene& s, const gprt_ray* rays, uint32_t n, bool 
         }
       }
       if (done) break;
-      int keep = 0;
-      for (int k = 0; k < nint; k++)
-        if (itn[k] <= best) {
-          itn[keep] = itn[k];
-          ich[keep] = ich[k];
-          keep++;
-        }
-      if (keep > 0) {
-        for (int k = keep - 1; k >= 1; k--) stack.push_back(ich[k]);
-        node = ich[0];
-      } else if (!stack.empty()) {
-        node = stack.back();
-        stack.pop_back();
-      } else {
-        node = -1;
-      }
+      if (nint > 0 && itn[0] <= best) node = ich[0];
+      else pop();
     }
   }
 }
