@@ -580,7 +580,8 @@ int gprt_intersect_host(gprt_scene* s, const gprt_ray* rays, uint32_t n, uint32_
     std::memcpy(r, rays, in);
     launch_intersect(s->dev, r, n, flags == GPRT_ANY, h, err, ctx->stream);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    const cudaError_t w = cudaStreamSynchronize(ctx->stream);  // also after an error: the staging is the next call's
+    if (e == cudaSuccess) e = w;
     if (e == cudaSuccess) std::memcpy(hits, h, out);
   } else {
     unsigned char* d = stage_device(ctx, in + out, own);
@@ -593,7 +594,8 @@ int gprt_intersect_host(gprt_scene* s, const gprt_ray* rays, uint32_t n, uint32_
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(hits, h, out, cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    const cudaError_t w = cudaStreamSynchronize(ctx->stream);
+    if (e == cudaSuccess) e = w;
     free_all(own);
   }
   if (e != cudaSuccess) return cuda_fail(ctx, e, "intersect_host");
