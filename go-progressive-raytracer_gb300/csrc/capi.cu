@@ -321,11 +321,6 @@ int upload_rest(gprt_ctx* ctx, gprt_scene* s) {
     free_all(s->buffers);
     return rc;
   }
-  if (dev_alloc(ctx, s->buffers, &s->d_err, 1)) {
-    free_all(s->buffers);
-    return GPRT_E_OOM;
-  }
-  cudaMemsetAsync(s->d_err, 0, sizeof(int), ctx->stream);
   if (h.nodes.size() / 8 >= (size_t)kMaxNodes) {
     free_all(s->buffers);
     return fail(ctx, GPRT_E_INVALID, "the scene's BVH has more than 2^30 nodes");
@@ -555,7 +550,7 @@ int gprt_intersect(gprt_scene* s, const gprt_ray* rays, uint32_t n, uint32_t fla
   std::lock_guard<std::recursive_mutex> lk(ctx->mu);
   cudaSetDevice(ctx->device);
   cudaStream_t st = stream ? static_cast<cudaStream_t>(stream) : ctx->stream;
-  launch_intersect(s->dev, rays, n, flags == GPRT_ANY, hits, s->d_err, st);
+  launch_intersect(s->dev, rays, n, flags == GPRT_ANY, hits, nullptr, st);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "intersect launch");
   return GPRT_OK;

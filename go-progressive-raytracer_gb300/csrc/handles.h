@@ -58,7 +58,6 @@ struct gprt_scene {
   OneNode one{};  // what dev.one points to
   std::vector<void*> buffers;
   size_t bytes = 0;
-  int* d_err = nullptr;
   std::set<gprt_job*> jobs;
   uint64_t serial = 0;  // unique per scene created in this process
 };

@@ -33,7 +33,7 @@ struct BatchSource {
   uint32_t n;
   __device__ uint32_t count() const { return n; }
   int root;
-  int* err;
+  int* err;  // null: the hit records alone tell
   __device__ void load(uint32_t i, float3& o, float3& d, float& tmin, float& tmax, uint32_t& skip, int& rt) const {
     rt = root;
     const float4* r = reinterpret_cast<const float4*>(rays + i);
@@ -46,7 +46,7 @@ struct BatchSource {
   }
   __device__ void store(uint32_t i, const Hit& h) const {
     bool over = h.prim == kOverflowHit;
-    if (over) atomicOr(err, kErrStackOverflow);
+    if (over && err) atomicOr(err, kErrStackOverflow);
     bool any = h.prim != kNoHit && !over;
     reinterpret_cast<float4*>(hits)[i] =
         make_float4(any ? h.t : -1.f, __uint_as_float(any || over ? h.prim : kNoHit), any ? h.u : 0.f,
