@@ -26,7 +26,13 @@ __device__ __forceinline__ float3& operator+=(float3& a, float3 b) { a = a + b; 
 __device__ __forceinline__ float3& operator*=(float3& a, float3 b) { a = a * b; return a; }
 __device__ __forceinline__ float3& operator*=(float3& a, float s) { a = a * s; return a; }
 __device__ __forceinline__ float dot(float3 a, float3 b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-// dot with its roundings spelled out (as normalize_xy and normalize_yx)
+// The path tracer and BDPT each have their shading in two kernels (the
+// wavefront's and the one that takes small chunks whole), which have to render
+// the same films.  The compiler contracts products and sums into multiply-adds
+// kernel by kernel, and in most places alike; where the two did not agree the
+// order is spelled out, as the wavefront's kernel of that integrator rounds:
+// _xy rounds y y first, _yx x x (dot_yx_z also z z).  That the rest agrees is a
+// property of the build, held by the tests that compare the films bit for bit.
 __device__ __forceinline__ float dot_xy(float3 a, float3 b) {
   return __fmaf_rn(a.z, b.z, __fmaf_rn(a.x, b.x, __fmul_rn(a.y, b.y)));
 }
@@ -45,9 +51,7 @@ __device__ __forceinline__ float3 normalize(float3 a) {
   float l = length(a);
   return l == 0.f ? f3(0.f, 0.f, 0.f) : f3(a.x / l, a.y / l, a.z / l);
 }
-// normalize with the rounding of the squared length spelled out: z z + (x x +
-// y y) with y y rounded first, or (normalize_yx) x x rounded first.  Kernels
-// that inline the shading code differently then give the same directions.
+// normalize with the rounding of the squared length spelled out, as dot_xy.
 __device__ __forceinline__ float3 normalize_by(float3 a, float l2) {
   float l = sqrtf(l2);
   return l == 0.f ? f3(0.f, 0.f, 0.f) : f3(a.x / l, a.y / l, a.z / l);
@@ -60,7 +64,7 @@ __device__ __forceinline__ float3 normalize_yx(float3 a) {
 }
 // core.Vec3.Luminance (pkg/core/vec3.go:134-136)
 __device__ __forceinline__ float luminance(float3 c) { return 0.2126f * c.x + 0.7152f * c.y + 0.0722f * c.z; }
-// with its roundings spelled out (as normalize_xy)
+// with its roundings spelled out (as dot_xy)
 __device__ __forceinline__ float luminance_xy(float3 c) {
   return __fmaf_rn(0.0722f, c.z, __fmaf_rn(0.2126f, c.x, __fmul_rn(0.7152f, c.y)));
 }
@@ -498,10 +502,11 @@ struct TraceStats {
 // each checked against the hit so far when its turn comes: the primitives are
 // tested in the order, and culled by the comparisons, of a loop that
 // intersects each leaf as it meets it, so ties between equal distances fall
-// the same way.  Measured on GB300, before -> after: 2^24 rays on 1.3 M
-// triangles (closest hit) 23.0 -> 10.1 ms, 300,007 rays (any hit) on 81,920
-// triangles 268 -> 167 us, the 1024^2 x 16 frame of the 1.3 M triangles
-// 28.7 -> 21.0 ms.
+// the same way.  (The stack holds children that such a hit hides until they are
+// popped: fit_stack in scene.cpp.)  Measured on GB300 against that loop, back
+// to back: 2^24 rays on 1.3 M triangles (closest hit) 16.9 -> 9.2 ms, 300,007
+// rays (any hit) on 81,920 triangles 130 -> 81 us, the 1024^2 x 16 frame of the
+// 1.3 M triangles 28.6 -> 20.6 ms.
 
 // State of one ray's traversal; `skip` is the primitive the ray leaves from:
 // a ray cannot re-enter the plane of the triangle or quad it starts on, and
@@ -879,13 +884,13 @@ using Geom = typename GeomOf<kOneNode>::type;
 // type and the record's address are the same for all lanes; a lane whose ray
 // misses the leaf's box (or without a ray: !live) sits it out.  The tests and
 // their order are those of trav_visit / trav_prim, whose step per primitive
-// costs more here than the lanes it fills (Cornell box, 18 quads, 400^2 x 64:
-// 10.7 ms a frame stepped, 7.8 ms in this loop).  The records come from the
-// launch's constant bank: as 128-bit global loads they kept the load pipe at
-// 65-71 % (every one returns 512 bytes a warp, though all lanes read the same
-// 16); now it is at 2-6 % and issue bounds the loop (IPC 2.6-2.9).  Cornell
-// box 7.83 -> 7.58 ms, Cornell boxes BDPT 512^2 x 64 90.8 -> 85.9 ms,
-// textured shapes 517x290 x 3 605 -> 559 us.
+// costs more here than the lanes it fills.  The records come from the launch's
+// constant bank: a 128-bit global load returns 512 bytes a warp, though all
+// lanes read the same 16, and those loads kept the load pipe at 65-71 %; now
+// issue bounds the loop.  Against the steps on global records: Cornell box (18
+// quads) 400^2 x 64 10.26 -> 7.19 ms, Cornell boxes BDPT 512^2 x 64 86.0 -> 70.5
+// ms, textured shapes 517 x 290 x 3 527 -> 345 us (of the 3 ms of the Cornell
+// box the constant bank gave 0.25).
 template <bool kCount>
 __device__ __forceinline__ bool trace_one_node(const OneNode& g, bool live, bool any_hit, float3 o, float3 d, float tmin,
                                                float tmax, uint32_t skip, Hit& hit, TraceStats* st = nullptr) {
@@ -960,19 +965,19 @@ __device__ __forceinline__ void trace_batch_one_node(const OneNode& g, Source& s
 
 // The step of a warp whose lanes `busy` are on a ray and `testing` wait for a
 // primitive test: a test costs about a third of a node visit, so it is taken
-// once more than a third of the lanes wait for it (1/2, 1/4, 1/6 and 2/3:
-// 21.3, 21.1, 21.5 and 22.5 against 21.0 ms for the frame of 1.3 M triangles;
-// 64.3, 64.5, 64.9 and 65.3 against 64.3 ms for 32 sphere scenes).
+// once more than a third of the lanes wait for it (1/2 and 1/4: 21.0 and 20.8
+// against 20.6 ms for the frame of 1.3 M triangles; 68.0 and 68.4 against 67.9
+// ms for 32 sphere scenes).
 __device__ __forceinline__ bool trav_test_now(unsigned testing, unsigned busy) {
   return 3 * __popc(testing) > __popc(busy);
 }
 
 // Persistent traversal of a batch of rays: every warp loops until its work
-// is exhausted, one step per iteration (trav_test_now), and lanes whose ray finished take new rays
-// once at least 16 lanes are idle (8, 12 and 20 measured within 2 %: 69.9,
-// 68.6 and 68.5 against 68.3 ms on the sphere batch, 22.7, 22.8 and 23.1
-// against 22.8 ms on 1.3 M triangles), so warps stay full instead of waiting
-// for their slowest ray.  Rays are dealt in chunks of up to 64.  Warp w of W
+// is exhausted, one step per iteration (trav_test_now), and lanes whose ray
+// finished take new rays once at least 16 lanes are idle (8 and 24: 69.6 and
+// 69.6 against 67.9 ms on the sphere batch, 20.4 and 22.0 against 20.6 ms on
+// 1.3 M triangles), so warps stay full instead of waiting for their slowest
+// ray.  Rays are dealt in chunks of up to 64 (deal.h).  Warp w of W
 // starts on chunk w; with `work` != null the chunks after the first W come
 // from that counter (zeroed by the previous kernel on the same stream),
 // otherwise warp w goes on with chunks w + W, w + 2 W, ... (calls on
@@ -985,9 +990,10 @@ __device__ __forceinline__ bool trav_test_now(unsigned testing, unsigned busy) {
 constexpr uint32_t kFetchChunk = 64;
 constexpr uint32_t kNoRay = 0xffffffffu;  // no ray in a batch has this number
 constexpr int kRefillIdle = 16;
-// 128-thread blocks per SM of the traversal kernels: 64 registers, 40 bytes
-// spilled; 7 blocks (72 registers) and 6 (80) measured 2 % and 6 % slower on
-// the sphere batch, 0 and 5 % on the 1.3 M triangles.
+// 128-thread blocks per SM of the traversal kernels: 64 registers, up to 54
+// bytes spilled; 7 blocks (72 registers) and 6 (80) measured 2 and 8 % slower
+// on the sphere batch and on the frame of 1.3 M triangles (its raw batch of
+// 2^24 rays 4 % faster and 2 % slower).
 constexpr int kTravBlocks = 8;
 
 template <bool kAnyHit, bool kCount, class Source>

@@ -17,11 +17,11 @@
 using namespace gprt;
 
 // Up to kHostStage bytes a copy each way costs more than the kernel's own
-// access to host memory: a call with 1,000 rays 49 -> 20 us (41 -> 18 us with
-// one ray, the launch and the wait), the RGBA image of 128^2 pixels 26 -> 20 us;
-// at 192 KB (a 128^2 float image) both ways take 30 us.  Above it the buffer
-// that is not allocated and freed by every call counts: 10^6 rays 830 -> 594 us,
-// the float image of 400^2 pixels 170 -> 63 us.
+// access to host memory: a call with 1,000 rays 39 -> 26 us, a preview pass of
+// 128^2 pixels with its RGBA image 128 -> 125 us; at 192 KB (a 128^2 float
+// image) both ways take the same.  Above it the buffer that is not allocated
+// and freed by every call counts: 10^6 rays 830 -> 594 us, the float image of
+// 400^2 pixels 170 -> 63 us.
 constexpr size_t kHostStage = 96 << 10, kDevStage = 64 << 20;
 
 // Ownership: a context owns its scenes and a scene owns its jobs, so

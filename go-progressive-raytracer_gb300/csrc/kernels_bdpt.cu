@@ -685,11 +685,11 @@ __device__ __forceinline__ float3 eval_strategy(const DevScene& sc, const Geom<k
 
 // Samples of a chunk per SM at most whose subpaths run in one launch and whose
 // strategies share one: above it the wavefront is as fast (1 sample per pixel,
-// depth 8, wavefront / one launch each in us: Cornell boxes 570 / 418 at
-// 65,536 samples, 865 / 835 at 147,456, 1324 / 1475 at 262,144; spot scene
-// 628 / 507 at 210,432, 851 / 830 at 374,272; sphere scene 535 / 372 at
-// 147,456, 1106 / 1085 at 589,824; 20,480 triangles 1015 / 801 at 147,456,
-// 1281 / 1253 at 262,144).
+// depth 8, wavefront / one launch each in us: Cornell boxes 564 / 414 at
+// 65,536 samples, 868 / 819 at 147,456, 1321 / 1423 at 262,144; spot scene
+// 633 / 515 at 210,432, 866 / 839 at 374,272; sphere scene 500 / 334 at
+// 147,456, 992 / 916 at 589,824; 20,480 triangles 1030 / 817 at 147,456,
+// 1282 / 1293 at 262,144).
 constexpr uint32_t kSmallBdptPerSm = 1024;
 constexpr int kSubpathsBlock = 512, kSubpathsBlocksPerSm = 1;
 
@@ -1015,11 +1015,10 @@ __global__ void __launch_bounds__(128, 4) k_bdpt_extend(DevScene sc, DevPaths PS
 // a sample from its camera ray to the end of its light subpath, with the state
 // between bounces in registers.  The wavefront's 2 x max_depth pairs of
 // launches each take a ray's or a shading step's chain of latencies, 8 and 22
-// us, on any number of samples (49,000 samples of the spot scene: 480 us a
-// frame, 371 so).  What is left is bound by fetching instructions, so the
+// us, on any number of samples (49,000 samples of the spot scene: 448 us a
+// frame, 225 so).  What is left is bound by fetching instructions, so the
 // warps of a block trace together and extend together and share them (two
-// barriers a bounce; the same frame, after other changes: 64-thread blocks
-// without the barriers 341 us, with them 336, 128 299, 256 277, 512 247).
+// barriers a bounce; the same frame in blocks of 128 276 us, 256 255, 512 225).
 // The vertices are those of the wavefront, bit for bit (the roundings on which
 // the compiler's contraction differs between the two are spelled out).
 template <int MAXV, bool kOneNode>
@@ -1375,11 +1374,11 @@ __device__ __forceinline__ float3 connection_value(const DevScene& sc, const Dev
 // 54 % see each other (Cornell boxes): the items that pass a step are
 // collected per warp until 32 of them take the next, so that every step runs
 // on full warps (25 of 32 lanes active instead of 19; 28.7 -> 24.5 ms of the
-// Cornell-boxes frame of 512 x 512 x 64 samples).  Then bound by the latency
-// of the vertex reads: 6 blocks per SM and 80 registers are faster than 8 and
-// 64 (81.4 / 83.0 ms of the frame) or 10 (85.6), and a grid that is resident
-// at once than two waves of it, which read each window of vertices twice
-// (83.0 / 86.3).
+// Cornell-boxes frame of 512 x 512 x 64 samples when it came in).  Then bound
+// by the latency of the vertex reads: 6 blocks per SM and 80 registers are
+// faster than 4 or 8 (70.5 ms the whole frame, 71.8 and 72.7), and a grid that
+// is resident at once than two waves of it, which read each window of vertices
+// twice (3 ms of the frame).
 constexpr int kConnectBlocks = 6;
 template <int MAXV, bool kOneNode>
 __device__ __forceinline__ void run_connections(const DevScene& sc, const DevPaths& PS, const ChunkDesc& ch,

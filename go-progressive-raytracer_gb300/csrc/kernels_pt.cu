@@ -392,23 +392,23 @@ void launch_pt_shadow(const DevScene& sc, const DevPaths& P, int cur, int block,
 // Small wavefronts in one launch: a lane takes a path from its camera ray to
 // its end (trace the shadow ray of the last level and the path's ray, shade,
 // repeat), keeping the state in registers that the queues of the wavefront
-// pass through memory.  The wavefront's 3-4 launches per bounce cost 30-45 us
-// each on any number of paths (a launch, and one ray's chain of dependent
-// loads on an almost empty chip), and a scene of depth 50 pays that 50 times;
-// here the chain of a path's bounces is all that is left.
+// pass through memory.  The wavefront's 3-4 launches cost 30-45 us a bounce on
+// any number of paths (launches, and one ray's chain of dependent loads on an
+// almost empty chip), and a scene of depth 50 pays that 50 times; here the
+// chain of a path's bounces is all that is left: default scene, 90,000 paths of
+// depth 50, 16 rounds 24.2 -> 7.18 ms, sphere scene 128 x 128 373 -> 125 us.
 // What bounds that chain is fetching instructions: a bounce runs 2,600 of
 // them, more than the caches near the scheduler hold, and warps at different
-// places of the code evict each other's (6.5-9 of 11 cycles per instruction
-// waited for one).  So the warps of a block trace together and shade together
-// (two barriers a bounce) and share what they fetch: default scene, 90,000
-// paths of depth 50, 16 rounds, 64-thread blocks without the barriers 9.96 ms,
-// blocks of 128 with them 8.94, 256 7.86, 512 7.23; more barriers, inside the
-// shading step, gained 1 %.  Trees, whose traversals differ more in length,
-// keep to 256 (sphere scene 128 x 128: 188 us without, 178 at 256, 183 at 512).
+// places of the code evict each other's.  So the warps of a block trace together
+// and shade together (two barriers a bounce) and share what they fetch: the
+// default scene as above in blocks of 128 8.81 ms, 256 7.72, 512 7.18 (of 64
+// without the barriers 9.96, before the pairing below).  Trees, whose traversals
+// differ more in length, keep to 256 (128, 256 and 512: sphere scene 128 x 128
+// 132, 125 and 125 us; 20,480 triangles 256 x 256 357, 367 and 389).
 // It loses on large wavefronts, where lanes of a warp part ways and 16 warps
 // per SM hide less than the traversal kernels' 32.
 // Results are those of the wavefront, bit for bit: the same tests in the same
-// order, the shading with its roundings spelled out, and the radiance added
+// order, the shading with the same roundings (dot_xy), and the radiance added
 // up as the kernels of the wavefront add it (each unoccluded shadow ray, and
 // what the path itself gathered when it ends).
 // 512 threads per SM at 128 registers; a finished lane takes the warp's next
@@ -420,12 +420,13 @@ constexpr int paths_block(bool one_node) { return one_node ? 512 : 256; }
 // Paths of a wavefront at most that k_pt_paths renders: where both forms took
 // the same time on GB300 (1 sample per pixel, depth 8; wavefront / whole paths
 // in us).  Scenes with an infinite light, whose paths leave at different
-// depths: sphere scene 607 / 506 at 360,000 paths, 719 / 672 at 589,824, 832 /
-// 898 at 810,000; 20,480 triangles 1597 / 1522 and 1795 / 1926; quadrics
-// 406 / 403 and 455 / 552; sphere grid 560 / 423 at 455,400, 644 / 542 at
-// 679,800; textured shapes 352 / 193 at 331,776, 519 / 488 at 1,101,800.
-// Closed scenes, where all lanes stay busy: Cornell box 294 / 280 at 176,400,
-// 313 / 309 at 211,600, 410 / 462 at 360,000 (with spheres 379 / 344 there).
+// depths: sphere scene 526 / 404 at 360,000 paths, 639 / 572 at 589,824, 740 /
+// 749 at 810,000; 20,480 triangles 1651 / 1516 at 589,824 and 1862 / 1924 at
+// 810,000, 1.3 M triangles 2822 / 2396 and 3137 / 2991; quadrics 409 / 405 at
+// 409,600 and 462 / 466 at 589,824; textured shapes 396 / 256 at 360,000, 533 /
+// 471 at 810,000.  Closed scenes, where all lanes stay busy: Cornell box 334 /
+// 317 at 176,400, 347 / 347 at 211,600, 455 / 509 at 360,000 (with spheres
+// 423 / 391 there).
 uint32_t pt_paths_max(const DevScene& sc, int sms) {
   return (uint32_t)sms * (sc.has_infinite ? 4096u : one_node(sc) ? 1536u : 2048u);
 }
@@ -438,8 +439,8 @@ __device__ __forceinline__ float4 shfl4(float4 v, int src) {
 // kPair: a lane that has both a shadow ray and the path's ray hands the shadow
 // ray to a lane of the warp that has neither, where there is one, and gets its
 // answer back, so that both are on their way at once; without, and for the
-// lanes that find none, one after the other.  (Sphere scene 128 x 128: 177 ->
-// 157 us a pass; 20,480 triangles, 65,536 paths 389 -> 351, 262,144 806 -> 765.)
+// lanes that find none, one after the other.  (Sphere scene 128 x 128: 143 ->
+// 125 us a pass; 20,480 triangles, 65,536 paths 399 -> 367.)
 template <bool kOneNode, bool kPair>
 __global__ void __launch_bounds__(paths_block(kOneNode), kPathsThreads / paths_block(kOneNode))
     k_pt_paths(DevScene sc, DevFilm film, DevPaths P, ChunkDesc ch, const __grid_constant__ Geom<kOneNode> g) {
@@ -611,8 +612,8 @@ void launch_pt_paths(const DevScene& sc, const DevFilm& film, const DevPaths& P,
   };
   // In a one-node scene a ray's loop takes the time of its slowest lane anyway,
   // and pairing pays only while most lanes are idle (Cornell box without / with
-  // it 105 / 91 us at 16,384 paths, 109 / 94 at 36,864, 111 / 117 at 65,536,
-  // 225 / 236 at 147,456; textured shapes 110 / 99 at 9,216, 132 / 133 at 82,944).
+  // it 125 / 112 us at 16,384 paths, 130 / 117 at 36,864, 137 / 141 at 65,536,
+  // 258 / 269 at 147,456; textured shapes 345 / 357 at 449,790).
   const bool few = ch.npix * ch.layers <= (uint32_t)sms * 256u;
   if (!one_node(sc)) run(k_pt_paths<false, true>, paths_block(false), NoGeom{});
   else if (few) run(k_pt_paths<true, true>, paths_block(true), *sc.one);

@@ -32,10 +32,10 @@ struct ShadeOut {
 // soon as it is known, so its state is not held to the end of the step.
 // `goes_on()` is called when the path is known to continue, before next-event
 // estimation: the wavefront reserves the path's place in the next queue there,
-// and the atomic's way to L2 and back passes under it (Cornell box 400^2 x 64
-// 7.57 -> 7.40 ms, 32 sphere scenes 64.1 -> 63.3 ms; without the shading
-// kernel's two atomics its launches are 15-17 % shorter.  Shadow rays at the
-// path's own index need none, but leave holes: Cornell box 8.3 ms).
+// and the atomic's way to L2 and back passes under it (reserved at the end
+// instead: Cornell box 400^2 x 64 7.31 against 7.19 ms, 32 sphere scenes and
+// 1.3 M triangles the same.  Shadow rays at the path's own index would need no
+// atomic, but leave holes in their queue, which cost the Cornell box 10 %).
 template <class Continue, class Shadow>
 __device__ __forceinline__ void shade_step(const DevScene& sc, float4 o4, float4 d4, float4 h4, uint4 ids, float4 w4,
                                            float3 thr, uint64_t seed, int bounce, ShadeOut& out,

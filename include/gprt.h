@@ -267,6 +267,12 @@ typedef struct gprt_job_desc {
   uint64_t seed;
 } gprt_job_desc;
 
+/* Path-traced chunks of few paths (up to 1,536 to 4,096 per SM, by scene)
+ * are rendered by one kernel from camera ray to last bounce, which has no
+ * launches or counters per kernel class: a job with any of the flags below
+ * runs the bounce-by-bounce kernels at every size instead, and renders the
+ * same film.  The times of such a job with few paths are those of these
+ * kernels, not of the job without the flag. */
 #define GPRT_JOB_TIME_KERNELS 1u     /* CUDA-event timing of every kernel launch, per kernel class */
 #define GPRT_JOB_COUNT_TRAVERSAL 2u  /* count BVH node / box / primitive tests (slower kernels) */
 /* Kernel variants (normally chosen by gprt_autotune): the closest-hit and the
@@ -310,7 +316,12 @@ typedef struct gprt_server gprt_server;
 
 /* ---- context ------------------------------------------------------------ */
 int gprt_version(void);
-/* Creates a context on CUDA device `device`. */
+/* Creates a context on CUDA device `device`.  Besides its scenes and jobs a
+ * context keeps, until it is destroyed, 96 KiB of pinned host memory and the
+ * device buffer through which calls with host pointers (gprt_intersect_host,
+ * gprt_job_read_image / _rgba8 / _tile) copy more than that: it grows to the
+ * largest such call's size, at most 64 MiB (a call that needs more allocates
+ * and frees its own).  A fixed device-memory budget counts it. */
 int gprt_ctx_create(int device, gprt_ctx** out);
 int gprt_ctx_destroy(gprt_ctx* ctx);
 /* Message of the last failed call on this context ("" when none). */
