@@ -4,12 +4,14 @@
     python profile_cases.py icosphere [--width 512] [--spp 4] [--count]
     python profile_cases.py bdpt [--width 512] [--spp 4]
     python profile_cases.py cornell [--width 400] [--spp 64]
+    python profile_cases.py paths [--scene spheres|default] [--width 128] [--spp 1]
 
 `batch` renders the first jobs of the heterogeneous default-style batch
 (seed 17; each job at its own spp, or at --spp N) through the batched render
 server; `icosphere` renders the displaced level-8 icosphere (1,310,720
 triangles) through the per-job path; `bdpt` renders the Cornell-boxes scene
-under BDPT through the per-job path.  All keep a few GB on the device at
+under BDPT through the per-job path; `paths` renders small frames, whose paths
+take one launch each.  All keep a few GB on the device at
 most and run each kernel a bounded number of times, so a capture of a few
 launches of one kernel ends by itself.  With --count the same case runs with
 the traversal counters on (and direct launches) and prints the rays, node
@@ -103,24 +105,47 @@ def bdpt(width, spp):
     print(json.dumps({"case": "bdpt", "width": width, "spp": spp}))
 
 
+def paths(scene, width, spp):
+    """Three frames of a sphere scene or of the reference's default scene (adaptive
+    sampling off), small enough for the whole-path kernel."""
+    import gprt
+    from gprt import scenes
+    ctx = gprt.Context(0)
+    s = (scenes.default_style_scene(3, width, width) if scene == "spheres"
+         else scenes.default_scene(gprt.CameraConfig(width=width)))
+    g = gprt.GpuScene(ctx, s.to_desc())
+    r = gprt.ProgressiveRaytracer(g, gprt.ProgressiveConfig(max_samples_per_pixel=3 * spp, max_passes=1, seed=1,
+                                                            chunk_paths=g.width * g.height * spp))
+    for _ in range(3):
+        r.add_samples(spp)
+    r.sync()
+    r.close()
+    g.close()
+    ctx.close()
+    print(json.dumps({"case": "paths", "scene": scene, "width": width, "spp": spp}))
+
+
 def main(argv=None):
     _setup()
     ap = argparse.ArgumentParser()
-    ap.add_argument("case", choices=["batch", "icosphere", "bdpt", "cornell"])
+    ap.add_argument("case", choices=["batch", "icosphere", "bdpt", "cornell", "paths"])
+    ap.add_argument("--scene", choices=["spheres", "default"], default="spheres")
     ap.add_argument("--jobs", type=int, default=24)
     ap.add_argument("--step-paths", type=int, default=1 << 22)
-    ap.add_argument("--width", type=int, default=512)
+    ap.add_argument("--width", type=int, default=0)
     ap.add_argument("--spp", type=int, default=0)
     ap.add_argument("--count", action="store_true")
     a = ap.parse_args(argv)
     if a.case == "batch":
         batch(a.jobs, a.step_paths, a.spp or None, a.count)
     elif a.case == "bdpt":
-        bdpt(a.width, a.spp or 4)
+        bdpt(a.width or 512, a.spp or 4)
     elif a.case == "cornell":
-        cornell(a.width, a.spp or 64)
+        cornell(a.width or 400, a.spp or 64)
+    elif a.case == "paths":
+        paths(a.scene, a.width or 128, a.spp or 1)
     else:
-        icosphere(a.width, a.spp or 4, a.count)
+        icosphere(a.width or 512, a.spp or 4, a.count)
     return 0
 
 
