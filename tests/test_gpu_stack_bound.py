@@ -27,23 +27,27 @@ def _scene(wall=True):
     return s.finalize_size()
 
 
-def _both(ctx, scene):
+def _both(ctx, scene, device_bvh=False):
     import gprt
-    return gprt.GpuScene(ctx, scene.to_desc()), gprt.GpuScene(ctx, scene.to_desc(), test_stack_cap=True)
+    return tuple(gprt.GpuScene(ctx, scene.to_desc(), device_bvh=device_bvh, test_stack_cap=cap) for cap in (False, True))
 
 
+@pytest.mark.parametrize("device_bvh", [False, True])
 @pytest.mark.parametrize("any_hit", [False, True])
-def test_children_behind_a_leaf_hit_take_no_room(ctx, any_hit):
+def test_children_behind_a_leaf_hit_take_no_room(ctx, any_hit, device_bvh):
     import gprt
     from test_gpu_intersect import _camera_rays
     scene = _scene()
-    plain, capped = _both(ctx, scene)
+    plain, capped = _both(ctx, scene, device_bvh)
+    assert capped.info.n_nodes > plain.info.n_nodes  # the root's children moved apart from its leaf
     rays = _camera_rays(scene, 5000, 2)
     want = plain.intersect(rays, any_hit=any_hit)
     assert (want["prim"] != gprt.capi.NO_HIT).all()
     assert np.array_equal(capped.intersect(rays, any_hit=any_hit), want)
     plain.close()
     capped.close()
+    if device_bvh:
+        return  # its tree splits the spheres so that a ray without the wall needs one entry
     plain, capped = _both(ctx, _scene(wall=False))
     with pytest.raises(gprt.capi.GprtError) as e:
         capped.intersect(rays, any_hit=any_hit)
